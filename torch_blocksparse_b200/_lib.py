@@ -1,10 +1,12 @@
-"""ctypes binding of libbsp_b200.so (the C ABI declared in include/bsp.h).
+"""ctypes binding of libbsp_b200.so (the C ABI declared in include/bsp.h), and the loader of the
+torch module _ops.so, through which the public classes call it.
 
 The library is the only compute path of this package: there is no Python or
-CPU fallback.  If the shared object is missing it is compiled on first use
-(needs nvcc); if that fails the import error is raised to the caller.
+CPU fallback.  If a shared object is missing it is compiled on first use
+(needs nvcc / g++); if that fails the import error is raised to the caller.
 """
 import ctypes
+import importlib
 import os
 from ctypes import POINTER, c_char_p, c_float, c_int, c_int32, c_int64, c_void_p
 
@@ -17,6 +19,7 @@ META_HEADER = 8
 ATTN_STATIC_ROWS = 1 << 20
 
 _lib = None
+_ops = None
 
 _I64P = POINTER(c_int64)
 _I32P = POINTER(c_int32)
@@ -88,6 +91,24 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+def ops():
+    """The torch module around the library (csrc/torch/ops.cpp)."""
+    global _ops
+    if _ops is None:
+        if not os.path.exists(_build.OPS_PATH):
+            _build.build()
+        _ops = importlib.import_module('._ops', __package__)
+    return _ops
+
+
+class OpCache(dict):
+    """Native operations of one object, by device.  A copy or a pickle of the owner starts without
+    them (they are rebuilt on first use)."""
+
+    def __reduce_ex__(self, protocol):
+        return (OpCache, ())
 
 
 _EXC = {ERR_INVALID: ValueError, ERR_UNSUPPORTED: NotImplementedError, ERR_CAPACITY: RuntimeError,

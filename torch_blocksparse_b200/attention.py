@@ -22,7 +22,7 @@ import weakref
 import torch
 import torch.nn as nn
 
-from . import tables
+from . import _lib, fused, tables
 from .matmul import MatMul
 from .softmax import Softmax
 
@@ -66,6 +66,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         self.fused = fused
         self.ops = dict()
         self.tiles = dict()
+        self._attn = _lib.OpCache()       # native attention per (heads, length, device index)
         self._causal_cache = dict()
         self.causal_checks = 0            # comparisons of a mask against the causal one made so far
 
@@ -97,6 +98,14 @@ class DeepSpeedSparseSelfAttention(nn.Module):
             self.tiles[key] = tables.build_attn_tiles(layout, self.block) if self.fused else None
         return self.ops[key]
 
+    def _attn_op(self, query):
+        """The fused attention with this module's tables on the device of `query`."""
+        _, H, L, _ = query.shape
+        sdd_nt, _, _ = self.get_ops(H, L)
+        op = fused.Attention(sdd_nt.meta, self.tiles[(H, L)], self.block, query.device)
+        self._attn[(H, L, query.get_device())] = op
+        return op
+
     def _is_causal(self, attn_mask, owner=None):
         """True when a 'mul' attention mask is exactly the lower-triangular (causal) mask: the
         fused kernels then derive it from the indices.  The answer is remembered per tensor
@@ -122,12 +131,11 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         """Forward + backward on the given [bsz, heads, L, head_dim] buffers as one CUDA graph (see
         fused.GraphedStep): `step = module.graphed(q, k, v, do)`, then `step.replay()` per step;
         results in step.o, step.dq, step.dk, step.dv.  No rpe / masks."""
-        from .fused import GraphedStep
         bsz, num_heads, tgt_len, head_dim = query.size()
         sdd_nt, _, _ = self.get_ops(num_heads, tgt_len)
         tiles = self.tiles.get((num_heads, tgt_len))
-        return GraphedStep(sdd_nt.meta, tiles, self.block, float(head_dim) ** -0.5 if scale is None else float(scale),
-                           query, key, value, dout)
+        return fused.GraphedStep(sdd_nt.meta, tiles, self.block, float(head_dim) ** -0.5 if scale is None else float(scale),
+                                 query, key, value, dout)
 
     def transpose_key_for_scores(self, x, L):
         """deepspeedsparseselfattention.py:119-123: a key given as [.., hd, L] is
@@ -139,7 +147,10 @@ class DeepSpeedSparseSelfAttention(nn.Module):
 
     def transpose_mask_for_sparse(self, qtype, x, is_key_padding_mask=False):
         """deepspeedsparseselfattention.py:125-132."""
-        x = x.type(qtype)
+        if x.dtype != qtype:
+            x = x.to(qtype)
+        if x.dim() == 2 and 1 not in x.shape:
+            return x
         if is_key_padding_mask:
             xdim = x.dim()
             for d in range(xdim - 1, 0, -1):
@@ -148,10 +159,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         return x.squeeze()
 
     def forward(self, query, key, value, rpe=None, key_padding_mask=None, attn_mask=None):
-        bsz, num_heads, tgt_len, head_dim = query.size()
-        key = self.transpose_key_for_scores(key, tgt_len)
-        if query.shape != key.shape or key.shape != value.shape:
-            raise NotImplementedError('only self-attention is supported for now')
+        key = _lib.ops().attention_key(query, key, value)       # (a key given as [.., hd, L] is viewed back)
         if key_padding_mask is not None:
             key_padding_mask = self.transpose_mask_for_sparse(query.dtype, key_padding_mask, is_key_padding_mask=True)
             if key_padding_mask.dim() == 1:
@@ -159,7 +167,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         mask_owner = attn_mask
         if attn_mask is not None:
             attn_mask = self.transpose_mask_for_sparse(query.dtype, attn_mask)
-        return self.attend(query, key, value, float(head_dim) ** -0.5, rpe, key_padding_mask, attn_mask,
+        return self.attend(query, key, value, query.size(3) ** -0.5, rpe, key_padding_mask, attn_mask,
                            mask_owner=mask_owner)
 
     def attend(self, query, key, value, scaling, rpe=None, key_padding_mask=None, attn_mask=None, mask_owner=None,
@@ -169,24 +177,21 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         mask tensor when `attn_mask` was derived from it (see _is_causal).  `seq_first_out`: the
         fused kernel writes its result in [L, bsz, heads * head_dim] memory order (returned as the
         [bsz, heads, L, head_dim] view of it)."""
-        bsz, num_heads, tgt_len, head_dim = query.size()
+        _, num_heads, tgt_len, _ = query.shape
         if key_padding_mask is not None and key_padding_mask.dtype != query.dtype:
             key_padding_mask = key_padding_mask.to(query.dtype)
         if attn_mask is not None and attn_mask.dtype != query.dtype:
             if mask_owner is None:
                 mask_owner = attn_mask
             attn_mask = attn_mask.to(query.dtype)
+        if self.fused and fused.fused_supported(query, self.block):
+            am_mode = self.attn_mask_mode
+            if attn_mask is not None and am_mode == 'mul' and self._is_causal(attn_mask, mask_owner):
+                am_mode = 'causal'
+            op = self._attn.get((num_heads, tgt_len, query.get_device())) or self._attn_op(query)
+            return fused.attention(op, query, key, value, scaling, rpe, key_padding_mask, attn_mask,
+                                   self.key_padding_mask_mode, am_mode, seq_first_out)
         sdd_nt, dsd_nn, softmax = self.get_ops(num_heads, tgt_len)
-        if self.fused:
-            from .fused import fused_attention, fused_supported
-            if fused_supported(query, self.block):
-                am_mode = self.attn_mask_mode
-                if attn_mask is not None and am_mode == 'mul' and self._is_causal(attn_mask, mask_owner):
-                    am_mode = 'causal'
-                return fused_attention(query, key, value, sdd_nt.meta, self.block, scaling, rpe,
-                                       key_padding_mask, attn_mask,
-                                       self.key_padding_mask_mode, am_mode,
-                                       tiles=self.tiles[(num_heads, tgt_len)], seq_first_out=seq_first_out)
         w = sdd_nt(query, key)
         w = softmax(w, scale=scaling, rpe=rpe, key_padding_mask=key_padding_mask, attn_mask=attn_mask,
                     key_padding_mask_mode=self.key_padding_mask_mode, attn_mask_mode=self.attn_mask_mode)

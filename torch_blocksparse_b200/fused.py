@@ -29,7 +29,7 @@ KERNELS_PER_BWD = 3
 
 
 def _timed(name, fn):
-    if PROFILE is None:
+    if PROFILE is None:                      # (a backward after the profile was switched off)
         return fn()
     t0 = torch.cuda.Event(enable_timing=True)
     t1 = torch.cuda.Event(enable_timing=True)
@@ -97,7 +97,8 @@ def _mask_args(Z, H, L, dtype, rpe, kpm, am, kp_mode, am_mode):
     return (r_ptr, rz, rh, rr, k_ptr, kz, 1 if kp_mode == 'mul' else 0, a_ptr, ar, am_flag), keep
 
 
-class _fused_attention(torch.autograd.Function):
+class _profiled_attention(torch.autograd.Function):
+    """What the native operation launches, with an event pair around every kernel (PROFILE)."""
 
     @staticmethod
     def forward(ctx, q, k, v, meta, tiles, block, scale, rpe, kpm, am, kp_mode, am_mode, seq_first_out=False):
@@ -143,12 +144,8 @@ class _fused_attention(torch.autograd.Function):
                 do.stride(0), do.stride(1), do.stride(2),
                 ctx.meta.hdr.data_ptr(), ctx.meta.on(q.device).data_ptr(), *_tile_args(ctx.tiles, q.device),
                 ctx.scale) + margs
-        L_ = _lib.lib()
-        if PROFILE is None:
-            _lib.check(L_.bsp_attn_bwd(*args, _stream(q)))
-        else:
-            for name, part in (('attn_bwd_delta', 1), ('attn_bwd_dkdv', 2), ('attn_bwd_dq', 4)):
-                _timed(name, lambda part=part: _lib.check(L_.bsp_attn_bwd_parts(*args, part, _stream(q))))
+        for name, part in (('attn_bwd_delta', 1), ('attn_bwd_dkdv', 2), ('attn_bwd_dq', 4)):
+            _timed(name, lambda part=part: _lib.check(_lib.lib().bsp_attn_bwd_parts(*args, part, _stream(q))))
         return (dq, dk, dv) + (None,) * 10
 
 
@@ -164,14 +161,39 @@ def device_status():
     return _lib.device_status()
 
 
+class Attention:
+    """The fused attention for one layout on one device: the native operation (csrc/torch/ops.cpp)
+    and the tables it holds."""
+
+    def __init__(self, meta, tiles, block, device):
+        self.meta, self.tiles, self.block = meta, tiles, block
+        dev = (None, None) if tiles is None else (tiles.hdr, tiles.on(device))
+        self.op = _lib.ops().AttentionOp(meta.hdr, meta.on(device), *dev, block)
+
+
+_AM_FLAG = {'add': 0, 'mul': 1, 'causal': 2}
+
+
+def attention(op, q, k, v, scale, rpe=None, key_padding_mask=None, attn_mask=None, key_padding_mask_mode='add',
+              attn_mask_mode='mul', seq_first_out=False):
+    """O = softmax(scale * Q K^T + rpe + masks, on the layout) V for [Z, H, L, D] operands; `op`: an
+    Attention."""
+    if key_padding_mask_mode not in ('add', 'mul'):
+        raise ValueError("key_padding_mask_mode must be 'add' or 'mul'")
+    if attn_mask_mode not in _AM_FLAG:
+        raise ValueError("attn_mask_mode must be 'add' or 'mul'")
+    if PROFILE is None:
+        return op.op(q, k, v, scale, rpe, key_padding_mask, attn_mask, key_padding_mask_mode == 'mul',
+                     _AM_FLAG[attn_mask_mode], PATH == 'tc', seq_first_out)
+    return _profiled_attention.apply(q, k, v, op.meta, op.tiles, op.block, float(scale), rpe, key_padding_mask, attn_mask,
+                                     key_padding_mask_mode, attn_mask_mode, seq_first_out)
+
+
 def fused_attention(q, k, v, meta, block, scale, rpe=None, key_padding_mask=None, attn_mask=None,
                     key_padding_mask_mode='add', attn_mask_mode='mul', tiles=None, seq_first_out=False):
-    """O = softmax(scale * Q K^T + rpe + masks, on the layout) V for [Z, H, L, D] operands."""
-    if meta.H != q.size(1) or meta.Mb != meta.Nb or meta.Mb * block != q.size(2):
-        raise ValueError('layout [%d,%d,%d] with block %d does not fit operands of shape %s'
-                         % (meta.H, meta.Mb, meta.Nb, block, tuple(q.shape)))
-    return _fused_attention.apply(q, k, v, meta, tiles, block, float(scale), rpe, key_padding_mask, attn_mask,
-                                  key_padding_mask_mode, attn_mask_mode, seq_first_out)
+    """attention() from a layout's tables."""
+    return attention(Attention(meta, tiles, block, q.device), q, k, v, scale, rpe, key_padding_mask, attn_mask,
+                     key_padding_mask_mode, attn_mask_mode, seq_first_out)
 
 
 class GraphedStep:
