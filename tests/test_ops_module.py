@@ -35,3 +35,62 @@ def test_timed_calls_and_versions(dtype):
         before = x._version
         y = sm(x)
         assert y is x and x._version > before and sm.time_y > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('block', [32, 64, 128])
+@pytest.mark.parametrize('heads', [1, 2])
+@pytest.mark.parametrize('free', [8, 72, 120, 136, 250, 264, 520])
+@pytest.mark.parametrize('trans', [False, True])
+def test_products_with_ragged_free_dimensions(block, heads, free, trans):
+    """dsd, dds and sdd at widths around the tiles of 128 and 256 columns and the 64 of a K stage, with
+    batch and heads of one (whose strides carry no meaning), against an FP32 dense product."""
+    g = torch.Generator().manual_seed(block + free)
+    nb = 5
+    layout = (torch.rand((heads, nb, nb), generator=g) > 0.5).long()
+    layout[:, 0, 0] = 1
+    n = nb * block
+    idx = layout.nonzero()
+
+    def dense(s):                                       # block format -> [1, heads, n, n]
+        d = torch.zeros(1, heads, nb, block, nb, block, device='cuda')
+        d[:, idx[:, 0], idx[:, 1], :, idx[:, 2]] = s.float().transpose(0, 1)
+        return d.reshape(1, heads, n, n)
+    rand = lambda *shape: torch.randn(shape, generator=g).half().cuda()
+    s = rand(1, len(idx), block, block)
+    # FP16 results of FP32 sums: one rounding (2^-11) of values of about sqrt(n)
+    close = lambda got, want: torch.testing.assert_close(got.float(), want, rtol=1e-3, atol=2e-3 * n ** 0.5)
+    x = rand(1, heads, free, n) if trans else rand(1, heads, n, free)
+    xn = x.transpose(2, 3) if trans else x
+    close(MatMul(layout, block, 'dsd', trans_b=trans)(s, x), dense(s) @ xn.float())
+    x = rand(1, heads, n, free) if trans else rand(1, heads, free, n)
+    xn = x.transpose(2, 3) if trans else x
+    close(MatMul(layout, block, 'dds', trans_a=trans)(x, s), xn.float() @ dense(s))
+    k = max(16, free // 16 * 16)
+    a, b = rand(1, heads, n, k), rand(1, heads, n, k) if trans else rand(1, heads, k, n)
+    want = a.float() @ (b.transpose(2, 3) if trans else b).float()
+    close(dense(MatMul(layout, block, 'sdd', trans_b=trans)(a, b)), want * dense(torch.ones_like(s)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('block', [16, 32, 128])
+@pytest.mark.parametrize('rows', [1, 7, 129, 1000])
+def test_linear_with_any_number_of_rows(block, rows):
+    """Forward and both gradients of Linear against the dense layer."""
+    from torch_blocksparse_b200 import Linear
+    g = torch.Generator().manual_seed(rows)
+    layout = (torch.rand((3, 4), generator=g) > 0.4).long()
+    layout[0, 0] = 1
+    lin = Linear(3 * block, 4 * block, block, layout).to('cuda', torch.float16)
+    x = torch.randn((2, rows, 3 * block), generator=g).half().cuda().requires_grad_()
+    dy = torch.randn((2, rows, 4 * block), generator=g).half().cuda()
+    idx = layout.nonzero()
+    w = torch.zeros(3, block, 4, block, device='cuda')
+    w[idx[:, 0], :, idx[:, 1]] = lin.weight.detach().float()
+    w = w.reshape(3 * block, 4 * block)
+    y = lin(x)
+    dx, dw = torch.autograd.grad(y, (x, lin.weight), dy)
+    x2, dy2 = x.detach().float().reshape(-1, 3 * block), dy.float().reshape(-1, 4 * block)
+    want_dw = (x2.T @ dy2).reshape(3, block, 4, block)[idx[:, 0], :, idx[:, 1]]
+    for got, want in ((y, (x2 @ w).view_as(y)), (dx, (dy2 @ w.T).view_as(dx)), (dw, want_dw)):
+        torch.testing.assert_close(got.float(), want, rtol=2e-3, atol=2e-3 * float(want.pow(2).mean().sqrt() + 1e-3))

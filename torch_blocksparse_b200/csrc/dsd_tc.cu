@@ -9,8 +9,8 @@
 // CSC side of the metadata).
 //
 // Geometry: every MMA has M = 128.  A tile is 128 rows of C (one block-row for block 128, two
-// for block 64, four for block 32) by TN = 256 columns (128 when the width is no multiple of
-// 256).  The block-rows of a tile are walked together, in
+// for block 64, four for block 32) by TN = 256 columns, or 128 for narrow or few tiles.
+// The block-rows of a tile are walked together, in
 // column order, over the UNION of their column lists; the piece of the A tile whose row has no
 // block in a column is zero (a non-finite value of the dense operand in such a place turns
 // into NaN where the mma.sync kernels, which skip absent blocks, give a finite result).  A
@@ -79,6 +79,7 @@ struct DsdTcArgs {
   void* c;
   int64_t c_sz, c_sh, c_sm, c_sn;
   int H, Mb, block, rows_total, nnz_rows;   // rows_total = Mb * block; nnz_rows = nnz * block (first out-of-range row of S)
+  int N;                                     // width of C; the columns of its last tile past N are computed on zeros and not stored
   int tiles_per_head, n_tiles, total_tiles;
   const int32_t *row_ptr, *blk_col;          // lists of a block-row of op(S): CSR of the layout, or (transposed use) its CSC
   const int32_t* blk_id;                     // storage index of every list entry (NULL: the entry's own position)
@@ -151,7 +152,7 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
   __shared__ uint64_t bar_plan_full[2], bar_plan_empty[2];
   __shared__ uint32_t row_mask[4][32];           // planning warp: block-row r has a block in column 32 * word + bit
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int block = a.block;
   const int R = 128 / block;
 
@@ -261,210 +262,206 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------------ sparse operand
-    // Lanes 0-7, one per piece of a stage's A part (block 64: two pieces of 8 KB, block 32: two
-    // sub-tiles of four pieces of 2 KB; block 128: lane 0, or lanes 0 and 1 for the two halves of
-    // a transposed block).  A piece without a block is loaded (as zeros, from past the last
-    // block) only if it held one.
-    if (lane < 8) {
-      const uint32_t m8 = 0xffu;
-      if (lane == 0) prefetch_map(&m_s);
-      uint32_t dirty = 0;                          // bit s: this lane's piece of ring slot s holds a block
-      int it = 0, cb = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; ok && t < a.total_tiles; t += gridDim.x) {
-        const Tile tc_ = tile_of(a, t);
-        int flags = kFirst, last_chunk = 0;
-        do {
-          const int buf = cb & 1;
-          int k = 1;
-          if (lane == 0) k = mbar_wait(&bar_plan_full[buf], (cb >> 1) & 1, fl) ? 1 : 0;
-          if (!__shfl_sync(m8, k, 0)) { ok = false; break; }
-          __syncwarp(m8);                              // lane 0 has acquired the plan; the other lanes read it after this
-          const int n = plan[buf].n;
-          last_chunk = plan[buf].last;
-          for (int e = 0; ok && e < n; ++e) {
-            const int* E = plan[buf].e[e];
-            const int mine = E[lane];
-            const bool half = block == 32 && E[9] < 0;
-            const bool last = last_chunk && e == n - 1;
-            const int reps = block == 128 ? 2 : 1;
-            for (int kh = 0; kh < reps; ++kh) {
-              const int s = it % S;
-              if (it >= S) {
-                // (every lane waits itself: cheaper than one waiting lane and a shuffle)
-                if (!__all_sync(m8, mbar_wait(&bar_empty[s], ((it / S) - 1) & 1, fl))) { ok = false; break; }
-              }
-              unsigned char* sp = smem + s * G::kStage;
-              if (block == 128) {
-                if (lane == 0) {
-                  stage_flags[s] = flags | ((last && kh) ? kLast : 0);
-                  mbar_expect_tx(&bar_full[s], kStageA);
-                }
-                __syncwarp(m8);
-                const int row = __shfl_sync(m8, mine, 0);
+    // A piece of a stage's A part is one block's rows (block 64: two pieces of 8 KB, block 32: two
+    // sub-tiles of four pieces of 2 KB; block 128: the whole part, or two halves of a transposed
+    // block).  A piece without a block is loaded (as zeros, from past the last block) only if
+    // the ring slot's piece held one.
+    constexpr uint32_t full = 0xffffffffu;
+    const bool me = elect_one();
+    if (me) prefetch_map(&m_s);
+    uint64_t dirty = 0;                            // bit 8 s + p: piece p of ring slot s holds a block
+    int it = 0, cb = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < a.total_tiles; t += gridDim.x) {
+      const int z = tile_of(a, t).z;
+      int flags = kFirst, last_chunk = 0;
+      do {
+        const int buf = cb & 1;
+        if (!mbar_wait_warp(&bar_plan_full[buf], (cb >> 1) & 1, fl)) { ok = false; break; }
+        const int n = __shfl_sync(full, plan[buf].n, 0);
+        last_chunk = __shfl_sync(full, plan[buf].last, 0);
+        for (int e = 0; ok && e < n; ++e) {
+          const int* E = plan[buf].e[e];
+          int row[8];
+#pragma unroll
+          for (int r = 0; r < 8; ++r) row[r] = E[r];
+          const bool half = block == 32 && E[9] < 0;
+          const bool last = last_chunk && e == n - 1;
+          const int reps = block == 128 ? 2 : 1;
+          for (int kh = 0; kh < reps; ++kh) {
+            const int s = it % S;
+            if (it >= S && !mbar_wait_warp(&bar_empty[s], ((it / S) - 1) & 1, fl)) { ok = false; break; }
+            unsigned char* sp = smem + s * G::kStage;
+            if (block == 128) {
+              if (me) {
+                stage_flags[s] = flags | ((last && kh) ? kLast : 0);
+                mbar_expect_tx(&bar_full[s], kStageA);
                 if (A_MN) {                          // rows kh * 64 .. of the stored block, its two halves of 64 columns
-                  if (lane < 2) tma_load_3d(sp + lane * 8192, &m_s, &bar_full[s], lane * 64, row + kh * 64, tc_.z);
-                } else if (lane == 0) {
-                  tma_load_3d(sp, &m_s, &bar_full[s], kh * 64, row, tc_.z);
+                  tma_load_3d(sp, &m_s, &bar_full[s], 0, row[0] + kh * 64, z);
+                  tma_load_3d(sp + 8192, &m_s, &bar_full[s], 64, row[0] + kh * 64, z);
+                } else {
+                  tma_load_3d(sp, &m_s, &bar_full[s], kh * 64, row[0], z);
                 }
-              } else {
-                const bool exists = block == 64 ? lane < 2 : !(half && lane >= 4);
-                bool ld = false;
-                if (exists) {
-                  if (mine >= 0) { ld = true; dirty |= 1u << s; }
-                  else if (dirty & (1u << s)) { ld = true; dirty &= ~(1u << s); }
-                }
-                const int piece = block == 64 ? 8192 : 2048;
-                const int nld = __popc(__ballot_sync(m8, ld));
-                if (lane == 0) {
-                  stage_flags[s] = flags | (last ? kLast : 0) | (half ? kHalf : 0);
-                  mbar_expect_tx(&bar_full[s], nld * piece);
-                }
-                __syncwarp(m8);
-                if (ld)
-                  tma_load_3d(sp + (block == 64 ? lane * 8192 : (lane >> 2) * 8192 + (lane & 3) * 2048), &m_s, &bar_full[s], 0,
-                              mine >= 0 ? mine : a.nnz_rows, tc_.z);
               }
-              flags = 0;
-              ++it;
+            } else {
+              uint32_t here = 0;                     // pieces that hold a block
+#pragma unroll
+              for (int r = 0; r < 8; ++r) here |= row[r] >= 0 ? 1u << r : 0u;
+              const uint32_t exist = block == 64 ? 3u : half ? 15u : 255u;
+              here &= exist;
+              const uint32_t ld = here | (static_cast<uint32_t>(dirty >> (8 * s)) & exist);
+              dirty = (dirty & ~(static_cast<uint64_t>(exist) << (8 * s))) | (static_cast<uint64_t>(here) << (8 * s));
+              if (me) {
+                stage_flags[s] = flags | (last ? kLast : 0) | (half ? kHalf : 0);
+                mbar_expect_tx(&bar_full[s], __popc(ld) * (block == 64 ? 8192 : 2048));
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                  if ((ld >> r) & 1u)
+                    tma_load_3d(sp + (block == 64 ? r * 8192 : r * 2048), &m_s, &bar_full[s], 0, row[r] >= 0 ? row[r] : a.nnz_rows, z);
+              }
             }
+            __syncwarp();
+            flags = 0;
+            ++it;
           }
-          __syncwarp(m8);
-          if (lane == 0) mbar_arrive(&bar_plan_empty[buf]);
-          ++cb;
-        } while (ok && !last_chunk);
-      }
-      if (ok && lane == 0) {                                     // tells the issuing thread that nothing follows
-        const int s = it % S;
-        if (it < S || mbar_wait(&bar_empty[s], ((it / S) - 1) & 1, fl)) {
-          stage_flags[s] = kEnd;
-          mbar_arrive(&bar_full[s]);
         }
+        __syncwarp();
+        if (me) mbar_arrive(&bar_plan_empty[buf]);
+        ++cb;
+      } while (ok && !last_chunk);
+    }
+    if (ok) {                                                    // tells the issuing thread that nothing follows
+      const int s = it % S;
+      if ((it < S || mbar_wait_warp(&bar_empty[s], ((it / S) - 1) & 1, fl)) && me) {
+        stage_flags[s] = kEnd;
+        mbar_arrive(&bar_full[s]);
       }
     }
   } else if (warp == 6) {
     // ------------------------------------------------------------------ dense operand
-    // k contiguous: one box of TN rows; n contiguous: one box of 64 columns per lane (the groups
-    // of 64 columns of the MN-major tile), issued together.  Lane 0 announces the bytes.
+    // k contiguous: one box of TN rows; n contiguous: one box per group of 64 columns of the
+    // MN-major tile.
+    constexpr uint32_t full = 0xffffffffu;
     constexpr int NG = B_KMAJOR ? 1 : TN / 64;
-    if (lane < NG) {
-      constexpr uint32_t mg = (1u << NG) - 1u;
-      if (lane == 0) prefetch_map(&m_b);
-      int it = 0, cb = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; ok && t < a.total_tiles; t += gridDim.x) {
-        const Tile tc_ = tile_of(a, t);
-        const int n0 = tc_.nt * TN;
-        int last_chunk = 0;
-        do {
-          const int buf = cb & 1;
-          int k = 1;
-          if (lane == 0) k = mbar_wait(&bar_plan_full[buf], (cb >> 1) & 1, fl) ? 1 : 0;
-          if (NG > 1) { k = __shfl_sync(mg, k, 0); __syncwarp(mg); }
-          if (!k) { ok = false; break; }
-          const int n = plan[buf].n;
-          last_chunk = plan[buf].last;
-          for (int e = 0; ok && e < n; ++e) {
-            const int c0 = plan[buf].e[e][8], c1 = plan[buf].e[e][9];
-            const int reps = block == 128 ? 2 : 1;
-            for (int kh = 0; kh < reps; ++kh) {
-              const int s = it % S;
-              if (it >= S) {
-                k = mbar_wait(&bar_empty[s], ((it / S) - 1) & 1, fl) ? 1 : 0;
-                if (NG > 1) k = __all_sync(mg, k);
-                if (!k) { ok = false; break; }
-              }
-              unsigned char* bp = smem + s * G::kStage + kStageA;
-              const bool two = block == 32 && c1 >= 0;
-              if (lane == 0) mbar_expect_tx(&bar_full[s], (block == 32 && !two) ? G::kStageB / 2 : G::kStageB);
-              if (NG > 1) __syncwarp(mg);
+    const bool me = elect_one();
+    if (me) prefetch_map(&m_b);
+    int it = 0, cb = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < a.total_tiles; t += gridDim.x) {
+      const Tile tc_ = tile_of(a, t);
+      const int n0 = tc_.nt * TN;
+      int last_chunk = 0;
+      do {
+        const int buf = cb & 1;
+        if (!mbar_wait_warp(&bar_plan_full[buf], (cb >> 1) & 1, fl)) { ok = false; break; }
+        const int n = __shfl_sync(full, plan[buf].n, 0);
+        last_chunk = __shfl_sync(full, plan[buf].last, 0);
+        for (int e = 0; ok && e < n; ++e) {
+          const int c0 = plan[buf].e[e][8], c1 = plan[buf].e[e][9];
+          const int reps = block == 128 ? 2 : 1;
+          for (int kh = 0; kh < reps; ++kh) {
+            const int s = it % S;
+            if (it >= S && !mbar_wait_warp(&bar_empty[s], ((it / S) - 1) & 1, fl)) { ok = false; break; }
+            unsigned char* bp = smem + s * G::kStage + kStageA;
+            const bool two = block == 32 && c1 >= 0;
+            if (me) {
+              mbar_expect_tx(&bar_full[s], (block == 32 && !two) ? G::kStageB / 2 : G::kStageB);
               if (block == 32) {
                 if (B_KMAJOR) {
                   tma_load_4d(bp, &m_b, &bar_full[s], c0 * 32, n0, tc_.h, tc_.z);
                   if (two) tma_load_4d(bp + G::kStageB / 2, &m_b, &bar_full[s], c1 * 32, n0, tc_.h, tc_.z);
                 } else {                                  // groups of 32 k-rows x 128 bytes: 4 KB apart
-                  tma_load_4d(bp + lane * 4096, &m_b, &bar_full[s], n0 + lane * 64, c0 * 32, tc_.h, tc_.z);
-                  if (two) tma_load_4d(bp + G::kStageB / 2 + lane * 4096, &m_b, &bar_full[s], n0 + lane * 64, c1 * 32, tc_.h, tc_.z);
+#pragma unroll
+                  for (int g = 0; g < NG; ++g) tma_load_4d(bp + g * 4096, &m_b, &bar_full[s], n0 + g * 64, c0 * 32, tc_.h, tc_.z);
+                  if (two) {
+#pragma unroll
+                    for (int g = 0; g < NG; ++g)
+                      tma_load_4d(bp + G::kStageB / 2 + g * 4096, &m_b, &bar_full[s], n0 + g * 64, c1 * 32, tc_.h, tc_.z);
+                  }
                 }
               } else {
                 const int krow = block == 128 ? c0 * 128 + kh * 64 : c0 * 64;
                 if (B_KMAJOR) tma_load_4d(bp, &m_b, &bar_full[s], krow, n0, tc_.h, tc_.z);
-                else tma_load_4d(bp + lane * 8192, &m_b, &bar_full[s], n0 + lane * 64, krow, tc_.h, tc_.z);
+                else {
+#pragma unroll
+                  for (int g = 0; g < NG; ++g) tma_load_4d(bp + g * 8192, &m_b, &bar_full[s], n0 + g * 64, krow, tc_.h, tc_.z);
+                }
               }
-              ++it;
             }
+            __syncwarp();
+            ++it;
           }
-          if (NG > 1) __syncwarp(mg);
-          if (lane == 0) mbar_arrive(&bar_plan_empty[buf]);
-          ++cb;
-        } while (ok && !last_chunk);
-      }
-      if (ok && lane == 0) {
-        const int s = it % S;
-        if (it < S || mbar_wait(&bar_empty[s], ((it / S) - 1) & 1, fl)) mbar_arrive(&bar_full[s]);
-      }
+        }
+        __syncwarp();
+        if (me) mbar_arrive(&bar_plan_empty[buf]);
+        ++cb;
+      } while (ok && !last_chunk);
+    }
+    if (ok) {
+      const int s = it % S;
+      if ((it < S || mbar_wait_warp(&bar_empty[s], ((it / S) - 1) & 1, fl)) && me) mbar_arrive(&bar_full[s]);
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = instr_desc(128, TN, B_KMAJOR ? 0 : 1, Bf<T>::v) | (A_MN ? 1u << 15 : 0u);
-      // Descriptors.  Blocks 64 / 128: 128-byte swizzle, K-major operands advance 32 bytes per
-      // K-step, MN-major ones 16 rows of 128 bytes; the groups of 64 columns (rows of A) of an
-      // MN-major operand lie 8 KB apart.  Block 32: the sparse operand and a K-major dense
-      // operand use the 64-byte swizzle (8-row groups of 512 bytes; an MN-major A has its
-      // groups of 32 rows 2 KB apart and advances 16 rows of 64 bytes per K-step); an MN-major
-      // dense sub-tile has 32 k-rows, so its groups of 64 columns lie 4 KB apart.
-      constexpr uint32_t kHi64 = (512u >> 4) | (1u << 14) | (4u << 29);
-      const bool b32 = block == 32;
-      const uint32_t a_hi = b32 ? kHi64 : kDescHi;
-      const uint32_t b_hi = (b32 && B_KMAJOR) ? kHi64 : kDescHi;
-      const uint32_t a_lbo = A_MN ? ((b32 ? 2048u : 8192u) >> 4) << 16 : 1u << 16;
-      const uint32_t b_lbo = B_KMAJOR ? 1u << 16 : ((b32 ? 4096u : 8192u) >> 4) << 16;
-      const uint32_t a_step = A_MN ? (b32 ? 64u : 128u) : 2u;
-      const uint32_t b_step = B_KMAJOR ? 2u : 128u;
-      const uint32_t sb = saddr(smem) >> 4;
-      int tiles = 0;
-      uint32_t d = tmem, ph = 0;
-      bool run = true;
-      // one pass of the loop body per ring slot, so that every descriptor is a constant offset from `sb`
-      while (run) {
+    const uint32_t idesc = instr_desc(128, TN, B_KMAJOR ? 0 : 1, Bf<T>::v) | (A_MN ? 1u << 15 : 0u);
+    // Descriptors.  Blocks 64 / 128: 128-byte swizzle, K-major operands advance 32 bytes per
+    // K-step, MN-major ones 16 rows of 128 bytes; the groups of 64 columns (rows of A) of an
+    // MN-major operand lie 8 KB apart.  Block 32: the sparse operand and a K-major dense
+    // operand use the 64-byte swizzle (8-row groups of 512 bytes; an MN-major A has its
+    // groups of 32 rows 2 KB apart and advances 16 rows of 64 bytes per K-step); an MN-major
+    // dense sub-tile has 32 k-rows, so its groups of 64 columns lie 4 KB apart.
+    constexpr uint32_t kHi64 = (512u >> 4) | (1u << 14) | (4u << 29);
+    const bool b32 = block == 32;
+    const uint32_t a_hi = b32 ? kHi64 : kDescHi;
+    const uint32_t b_hi = (b32 && B_KMAJOR) ? kHi64 : kDescHi;
+    const uint32_t a_lbo = A_MN ? ((b32 ? 2048u : 8192u) >> 4) << 16 : 1u << 16;
+    const uint32_t b_lbo = B_KMAJOR ? 1u << 16 : ((b32 ? 4096u : 8192u) >> 4) << 16;
+    const uint32_t a_step = A_MN ? (b32 ? 64u : 128u) : 2u;
+    const uint32_t b_step = B_KMAJOR ? 2u : 128u;
+    const uint32_t sb = saddr(smem) >> 4;
+    int tiles = 0;
+    uint32_t d = tmem, ph = 0;
+    bool run = true;
+    const bool me = elect_one();
+    // one pass of the loop body per ring slot, so that every descriptor is a constant offset from `sb`
+    while (run) {
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-          if (!mbar_wait(&bar_full[s], ph, fl)) { run = false; break; }
+      for (int s = 0; s < S; ++s) {
+        if (!mbar_wait_warp(&bar_full[s], ph, fl)) { run = false; break; }
+        fence_after();
+        const int f = __shfl_sync(0xffffffffu, stage_flags[s], 0);
+        if (f & kEnd) { run = false; break; }
+        if (f & kFirst) {
+          const int buf = tiles % kAcc;
+          if (tiles >= kAcc && !mbar_wait_warp(&bar_acc_empty[buf], ((tiles / kAcc) - 1) & 1, fl)) { run = false; break; }
           fence_after();
-          const int f = stage_flags[s];
-          if (f & kEnd) { run = false; break; }
-          if (f & kFirst) {
-            const int buf = tiles % kAcc;
-            if (tiles >= kAcc && !mbar_wait(&bar_acc_empty[buf], ((tiles / kAcc) - 1) & 1, fl)) { run = false; break; }
-            fence_after();
-            d = tmem + buf * TN;
-            ++tiles;
-          }
-          const uint32_t a0 = ((sb + ((s * G::kStage) >> 4)) & 0x3FFFu) | a_lbo;
-          const uint32_t b0 = ((sb + ((s * G::kStage + kStageA) >> 4)) & 0x3FFFu) | b_lbo;
-          {
-            if (!b32) {
-              mma_desc(d, a0, a_hi, b0, b_hi, idesc, (f & kFirst) ? 0u : 1u);
-              mma_desc_acc(d, a0 + a_step, a_hi, b0 + b_step, b_hi, idesc);
-              mma_desc_acc(d, a0 + 2 * a_step, a_hi, b0 + 2 * b_step, b_hi, idesc);
-              mma_desc_acc(d, a0 + 3 * a_step, a_hi, b0 + 3 * b_step, b_hi, idesc);
-            } else {
-              // K-steps 2, 3 belong to the second sub-tile (8 KB further in A, half a stage further in B)
-              mma_desc(d, a0, a_hi, b0, b_hi, idesc, (f & kFirst) ? 0u : 1u);
-              mma_desc_acc(d, a0 + a_step, a_hi, b0 + b_step, b_hi, idesc);
-              if (!(f & kHalf)) {
-                const uint32_t a1 = a0 + (8192u >> 4), b1 = b0 + ((uint32_t)(G::kStageB / 2) >> 4);
-                mma_desc_acc(d, a1, a_hi, b1, b_hi, idesc);
-                mma_desc_acc(d, a1 + a_step, a_hi, b1 + b_step, b_hi, idesc);
-              }
+          d = tmem + buf * TN;
+          ++tiles;
+        }
+        const uint32_t a0 = ((sb + ((s * G::kStage) >> 4)) & 0x3FFFu) | a_lbo;
+        const uint32_t b0 = ((sb + ((s * G::kStage + kStageA) >> 4)) & 0x3FFFu) | b_lbo;
+        if (me) {
+          if (!b32) {
+            mma_desc(d, a0, a_hi, b0, b_hi, idesc, (f & kFirst) ? 0u : 1u);
+            mma_desc_acc(d, a0 + a_step, a_hi, b0 + b_step, b_hi, idesc);
+            mma_desc_acc(d, a0 + 2 * a_step, a_hi, b0 + 2 * b_step, b_hi, idesc);
+            mma_desc_acc(d, a0 + 3 * a_step, a_hi, b0 + 3 * b_step, b_hi, idesc);
+          } else {
+            // K-steps 2, 3 belong to the second sub-tile (8 KB further in A, half a stage further in B)
+            mma_desc(d, a0, a_hi, b0, b_hi, idesc, (f & kFirst) ? 0u : 1u);
+            mma_desc_acc(d, a0 + a_step, a_hi, b0 + b_step, b_hi, idesc);
+            if (!(f & kHalf)) {
+              const uint32_t a1 = a0 + (8192u >> 4), b1 = b0 + ((uint32_t)(G::kStageB / 2) >> 4);
+              mma_desc_acc(d, a1, a_hi, b1, b_hi, idesc);
+              mma_desc_acc(d, a1 + a_step, a_hi, b1 + b_step, b_hi, idesc);
             }
           }
           commit(&bar_empty[s]);                                    // the stage is free once these MMAs have read it
           if (f & kLast) commit(&bar_acc_full[(tiles - 1) % kAcc]);
         }
-        ph ^= 1;
+        __syncwarp();
       }
+      ph ^= 1;
     }
   } else if (warp < 4) {
     // ------------------------------------------------------------------ write-back
@@ -497,8 +494,13 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = 0u;                   // block-rows without blocks: zeros, as the reference gives
         }
-        if (row_ok) {
-          if (C_ROWS) {
+        const int left = a.N - (tc_.nt * TN + c);                   // columns of C from here on
+        if (row_ok && left > 0) {
+          if (left < 32) {                                          // the last columns one by one
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i < left) crow[(int64_t)(c + i) * a.c_sn] = cvt1<T>(__uint_as_float(r[i]));
+          } else if (C_ROWS) {
 #pragma unroll
             for (int i = 0; i < 32; i += 8) {
               uint4 v;
@@ -569,18 +571,19 @@ int sm_count() {
 
 }  // namespace
 
-// True when dsd_tc covers the case: FP16 / BF16, block 32 / 64 / 128, N a multiple of 128, both dense tensors with
-// one unit inner stride and 16-byte friendly addresses and strides.
-bool dsd_tc_eligible(const void* s, const void* b, const void* c, int dtype, int block, int N, int trans_s, int64_t s_sz,
+// True when dsd_tc covers the case: FP16 / BF16, block 32 / 64 / 128, any N, both dense tensors with one unit inner stride and 16-byte friendly
+// addresses and strides.  Strides of dimensions of extent 1 carry no meaning.
+bool dsd_tc_eligible(const void* s, const void* b, const void* c, int dtype, int block, int Z, int H, int N, int64_t s_sz,
                      int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn,
                      int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn) {
   if (dtype != BSP_F16 && dtype != BSP_BF16) return false;
-  if ((block != 32 && block != 64 && block != 128) || N % 128) return false;
+  if (block != 32 && block != 64 && block != 128) return false;
   if ((b_sk != 1) == (b_sn != 1) || (c_sm != 1) == (c_sn != 1)) return false;
   const int64_t b_outer = b_sk == 1 ? b_sn : b_sk;
   if ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) return false;
   if ((s_sz | b_sz | b_sh | b_outer) & 7) return false;
-  if (s_sz <= 0 || b_sz <= 0 || b_sh <= 0 || b_outer <= 0) return false;     // TMA strides: no broadcast
+  if ((Z > 1 && (s_sz <= 0 || b_sz <= 0)) || (H > 1 && b_sh <= 0) || b_outer <= 0) return false;     // TMA strides: no broadcast
+  if (b_sn == 1 && (N & 7)) return false;            // (a row of the operand ends inside a 16-byte piece)
   if (c_sn == 1 && ((c_sz | c_sh | c_sm) & 7)) return false;
   return true;
 }
@@ -589,7 +592,12 @@ int dsd_tc(const void* s, const void* b, void* c, int dtype, int block, int Z, i
            int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn,
            int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn, const Meta& m, cudaStream_t st) {
   const bool bk = b_sk == 1, cr = c_sn == 1;
-  const int TN = N % 256 == 0 ? 256 : 128;
+  // Tiles of 256 columns, unless they would leave SMs without a tile (two persistent CTAs per SM)
+  // or be mostly padding: a stage of a 128-column tile costs nearly as much as one of 256.
+  const int sms = sm_count();
+  if (sms <= 0) return fail(BSP_ERR_CUDA, "dsd (tcgen05): cannot query the device");
+  const int64_t rows_t = (int64_t)Z * m.H * (((trans_s ? m.Nb : m.Mb) * block + 127) / 128);
+  const int TN = N <= 128 || rows_t * ((N + 255) / 256) <= sms || (N % 256 != 0 && N % 256 <= 128 && N < 512) ? 128 : 256;
   // op(S) has the layout's rows (and walks its CSR) or, transposed, its columns (CSC)
   const int out_b = trans_s ? m.Nb : m.Mb, red_b = trans_s ? m.Mb : m.Nb;
   const int64_t ktot = (int64_t)red_b * block;
@@ -620,14 +628,13 @@ int dsd_tc(const void* s, const void* b, void* c, int dtype, int block, int Z, i
   a.c = c; a.c_sz = c_sz; a.c_sh = c_sh; a.c_sm = c_sm; a.c_sn = c_sn;
   a.H = m.H; a.Mb = out_b; a.block = block; a.rows_total = out_b * block; a.nnz_rows = m.nnz * block;
   a.tiles_per_head = (out_b * block + 127) / 128;
-  a.n_tiles = N / TN;
+  a.N = N;
+  a.n_tiles = (N + TN - 1) / TN;
   const int64_t total = (int64_t)Z * m.H * a.tiles_per_head * a.n_tiles;
   if (total > 0x7fffffff) return fail(BSP_ERR_INVALID, "dsd: too many tiles");
   a.total_tiles = (int)total;
   if (trans_s) { a.row_ptr = m.col_ptr; a.blk_col = m.col_row; a.blk_id = m.col_bid; }
   else { a.row_ptr = m.row_ptr; a.blk_col = m.blk_col; a.blk_id = nullptr; }
-  const int sms = sm_count();
-  if (sms <= 0) return fail(BSP_ERR_CUDA, "dsd (tcgen05): cannot query the device");
   if (dtype == BSP_F16)
     return TN == 256 ? launch_t<__half, 256>(trans_s != 0, bk, cr, ms, mb, a, sms, st)
                      : launch_t<__half, 128>(trans_s != 0, bk, cr, ms, mb, a, sms, st);

@@ -20,14 +20,14 @@ int dsd_mma_t(const void* s, const void* b, void* c, int block, int Z, int N,
               int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn,
               const Meta& m, cudaStream_t st);
 
-bool dsd_tc_eligible(const void* s, const void* b, const void* c, int dtype, int block, int N, int trans_s, int64_t s_sz,
+bool dsd_tc_eligible(const void* s, const void* b, const void* c, int dtype, int block, int Z, int H, int N, int64_t s_sz,
                      int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn,
                      int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn);
 int dsd_tc(const void* s, const void* b, void* c, int dtype, int block, int Z, int N, int64_t s_sz, int trans_s,
            int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn,
            int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn, const Meta& m, cudaStream_t st);
 
-bool sdd_tc_eligible(const void* a, const void* b, const void* c, int dtype, int block, int K,
+bool sdd_tc_eligible(const void* a, const void* b, const void* c, int dtype, int block, int Z, int H,
                      int64_t a_sz, int64_t a_sh, int64_t a_sm, int64_t a_sk,
                      int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn, int64_t c_sz);
 int sdd_tc(const void* a, const void* b, void* c, int dtype, int block, int Z, int K,
@@ -88,7 +88,7 @@ int run_dsd(const void* s, const void* b, void* c, int dtype, int block, int Z, 
   // mma.sync kernel writes the zeros)
   // (the tcgen05 kernel plans a tile with one bit per block of the reduction side, 1024 at most)
   if (g_matmul_tc.load() && m.nnz > 0 && (trans_s ? m.Mb : m.Nb) <= 1024 &&
-      dsd_tc_eligible(s, b, c, dtype, block, N, trans_s, s_sz, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn))
+      dsd_tc_eligible(s, b, c, dtype, block, Z, m.H, N, s_sz, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn))
     return dsd_tc(s, b, c, dtype, block, Z, N, s_sz, trans_s, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn, m, st);
   if (dtype == BSP_F32)
     return dsd_mma_t<float>(s, b, c, block, Z, N, s_sz, trans_s, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn, m, st);
@@ -110,7 +110,8 @@ extern "C" int bsp_sdd(const void* a, const void* b, void* c, int dtype, int blo
   Meta m;
   if (int rc = decode_meta(meta_hdr, meta, m)) return rc;
   if (int rc = check_basic("sdd", dtype, block, Z, H, m)) return rc;
-  if (K <= 0 || K % 16) return fail(BSP_ERR_INVALID, "Reduction size for SDD must be a multiple of 16");
+  // (k-contiguous operands are read in pieces of 16; with both operands k-strided any K is fine)
+  if (K <= 0 || (K % 16 && !(a_sk != 1 && b_sk != 1))) return fail(BSP_ERR_INVALID, "Reduction size for SDD must be a multiple of 16");
   if (int rc = check_dense("sdd", "a", a, dtype, a_sz, a_sh, a_sm, a_sk)) return rc;
   if (int rc = check_dense("sdd", "b", b, dtype, b_sz, b_sh, b_sk, b_sn)) return rc;
   if (int rc = check_sparse("sdd", "c", c, dtype, c_sz)) return rc;
@@ -118,7 +119,7 @@ extern "C" int bsp_sdd(const void* a, const void* b, void* c, int dtype, int blo
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // (the tcgen05 kernel's grid: groups of 128 rows per head in y, the batch in z)
   if (g_matmul_tc.load() && Z <= 65535 && (int64_t)m.H * ((m.Mb * block + 127) / 128) <= 65535 &&
-      sdd_tc_eligible(a, b, c, dtype, block, K, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz))
+      sdd_tc_eligible(a, b, c, dtype, block, Z, m.H, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz))
     return sdd_tc(a, b, c, dtype, block, Z, K, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz, m, st);
   if (dtype == BSP_F32)
     return sdd_mma_t<float>(a, b, c, block, Z, K, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz, m, st);
@@ -136,7 +137,8 @@ extern "C" int bsp_dsd(const void* s, const void* b, void* c, int dtype, int blo
   if (int rc = decode_meta(meta_hdr, meta, m)) return rc;
   if (int rc = check_basic("dsd", dtype, block, Z, H, m)) return rc;
   const int vec = dtype == BSP_F32 ? 4 : 8;
-  if (N <= 0 || N % vec) return fail(BSP_ERR_INVALID, "dsd: dense width %d must be a positive multiple of %d", N, vec);
+  if (N <= 0 || (N % vec && !(b_sk == 1 && b_sn != 1)))
+    return fail(BSP_ERR_INVALID, "dsd: dense width %d must be positive, and a multiple of %d where b has unit stride along it", N, vec);
   if (m.nnz > 0)                 // (a layout without blocks has an empty sparse operand, never dereferenced)
     if (int rc = check_sparse("dsd", "a", s, dtype, s_sz)) return rc;
   if (int rc = check_dense("dsd", "b", b, dtype, b_sz, b_sh, b_sk, b_sn)) return rc;
@@ -158,7 +160,8 @@ extern "C" int bsp_dds(const void* a, const void* s, void* c, int dtype, int blo
   if (int rc = decode_meta(meta_hdr, meta, m)) return rc;
   if (int rc = check_basic("dds", dtype, block, Z, H, m)) return rc;
   const int vec = dtype == BSP_F32 ? 4 : 8;
-  if (M <= 0 || M % vec) return fail(BSP_ERR_INVALID, "dds: dense height %d must be a positive multiple of %d", M, vec);
+  if (M <= 0 || (M % vec && !(a_sk == 1 && a_sm != 1)))
+    return fail(BSP_ERR_INVALID, "dds: dense height %d must be positive, and a multiple of %d where a has unit stride along it", M, vec);
   if (int rc = check_dense("dds", "a", a, dtype, a_sz, a_sh, a_sm, a_sk)) return rc;
   if (m.nnz > 0)
     if (int rc = check_sparse("dds", "b", s, dtype, s_sz)) return rc;

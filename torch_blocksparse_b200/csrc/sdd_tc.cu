@@ -65,7 +65,7 @@ sdd_tc_kernel(const __grid_constant__ CUtensorMap m_a, const __grid_constant__ C
   __shared__ int w_h, w_m0, w_cols, w_n[8], w_id[4][8];
   __shared__ uint32_t row_mask[4][32];          // set-up: block-row r has a block in column 32 * word + bit
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int z = blockIdx.z, block = a.block;
   const int R = 128 / block, NC = 2 * R;        // block-rows of a tile, column blocks of a group
 
@@ -178,7 +178,7 @@ sdd_tc_kernel(const __grid_constant__ CUtensorMap m_a, const __grid_constant__ C
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_slot;
-  const int ns = a.K / 64;
+  const int ns = (a.K + 63) / 64;              // (past K both operands are filled with zeros)
   const int h = w_h, m0 = w_m0;
   // columns computed: 128 when the group's column blocks fill at most half of the accumulator
   const int ncomp = w_cols * block <= 128 ? 128 : 256;
@@ -186,59 +186,57 @@ sdd_tc_kernel(const __grid_constant__ CUtensorMap m_a, const __grid_constant__ C
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer
-    // lanes 0-7: the boxes of B (block 128 with n contiguous: two per column block; else one per
-    // column block), lanes 8 and 9: the two boxes of A
-    if (lane < 10) {
-      const uint32_t m10 = 0x3ffu;
-      if (lane == 0) { prefetch_map(&m_a); prefetch_map(&m_b); }
-      const bool split = block == 128 && B_MN;                    // a column block of 128 n-contiguous columns takes two boxes of 64
-      const int nbox = split ? 2 * w_cols : w_cols;               // boxes of B that exist
-      const int box_bytes = split ? 8192 : block * 128;
-      const int cj = split ? lane >> 1 : lane;                    // column block of this lane's box
-      const bool mine = lane < 8 && lane < nbox && (split ? lane < 4 : true);
-      const int n_first = mine ? w_n[cj] + (split ? (lane & 1) * 64 : 0) : 0;
-      const uint32_t tx = kStageA + nbox * box_bytes;
-      int ok = 1;
-      for (int it = 0; it < ns; ++it) {
-        const int s = it % kStages, k0 = it * 64;
-        if (it >= kStages) {
-          if (lane == 0) ok = mbar_wait(&bar_empty[s], ((it / kStages) - 1) & 1, fl) ? 1 : 0;
-          ok = __shfl_sync(m10, ok, 0);
-          if (!ok) break;
-        }
-        unsigned char* sp = smem + s * kStageBytes;
-        if (lane == 0) mbar_expect_tx(&bar_full[s], tx);
-        __syncwarp(m10);
-        if (lane >= 8) {
-          const int half = lane - 8;
+    // boxes of B: one per column block (block 128 with n contiguous: two); two boxes of A
+    const bool me = elect_one();
+    if (me) { prefetch_map(&m_a); prefetch_map(&m_b); }
+    const bool split = block == 128 && B_MN;                    // a column block of 128 n-contiguous columns takes two boxes of 64
+    const int nbox = split ? 2 * w_cols : w_cols;               // boxes of B that exist
+    const int box_bytes = split ? 8192 : block * 128;
+    const uint32_t tx = kStageA + nbox * box_bytes;
+    int n_first[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) n_first[j] = j < nbox ? (split ? w_n[j >> 1] + (j & 1) * 64 : w_n[j]) : 0;
+    for (int it = 0; it < ns; ++it) {
+      const int s = it % kStages, k0 = it * 64;
+      if (it >= kStages && !mbar_wait_warp(&bar_empty[s], ((it / kStages) - 1) & 1, fl)) break;
+      unsigned char* sp = smem + s * kStageBytes;
+      if (me) {
+        mbar_expect_tx(&bar_full[s], tx);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
           if (A_MN) tma_load_4d(sp + half * 8192, &m_a, &bar_full[s], m0 + half * 64, k0, h, z);   // [k][m]: 64 m x 64 k-rows
           else tma_load_4d(sp + half * 8192, &m_a, &bar_full[s], k0, m0 + half * 64, h, z);        // [m][k]: 64 k x 64 m-rows
-        } else if (mine) {
-          unsigned char* bp = sp + kStageA + lane * box_bytes;
-          if (B_MN) tma_load_4d(bp, &m_b, &bar_full[s], n_first, k0, h, z);                        // [k][n]
-          else tma_load_4d(bp, &m_b, &bar_full[s], k0, n_first, h, z);                             // [n][k]
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (j >= nbox) break;
+          unsigned char* bp = sp + kStageA + j * box_bytes;
+          if (B_MN) tma_load_4d(bp, &m_b, &bar_full[s], n_first[j], k0, h, z);                      // [k][n]
+          else tma_load_4d(bp, &m_b, &bar_full[s], k0, n_first[j], h, z);                           // [n][k]
         }
       }
+      __syncwarp();
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = instr_desc(128, ncomp, B_MN ? 1 : 0, Bf<T>::v) | (A_MN ? 1u << 15 : 0u);
-      bool ok = true;
-      for (int it = 0; ok && it < ns; ++it) {
-        const int s = it % kStages;
-        // (MN-major A: 8 KB between its two groups of 64 rows, in the leading-offset field)
-        const uint32_t a_lo = A_MN ? (((saddr(smem + s * kStageBytes) & 0x3FFFF) >> 4) | (512u << 16))
-                                   : desc_lo(saddr(smem + s * kStageBytes));
-        // (block 32, MN-major B: groups of 32 columns in the 64-byte swizzle, 64 k-rows of 64 bytes
-        // = 4 KB apart, 8-row groups of 512 bytes, 16 rows = 1 KB per K-step)
-        const bool b64s = B_MN && block == 32;
-        const uint32_t b_lo = B_MN ? (((saddr(smem + s * kStageBytes + kStageA) & 0x3FFFF) >> 4) | ((b64s ? 256u : 512u) << 16))
-                                   : desc_lo(saddr(smem + s * kStageBytes + kStageA));
-        const uint32_t b_hi = b64s ? ((512u >> 4) | (1u << 14) | (4u << 29)) : kDescHi;
-        ok = mbar_wait(&bar_full[s], (it / kStages) & 1, fl);
-        if (!ok) break;
-        fence_after();
+    const bool me = elect_one();
+    const uint32_t idesc = instr_desc(128, ncomp, B_MN ? 1 : 0, Bf<T>::v) | (A_MN ? 1u << 15 : 0u);
+    bool ok = true;
+    for (int it = 0; it < ns; ++it) {
+      const int s = it % kStages;
+      // (MN-major A: 8 KB between its two groups of 64 rows, in the leading-offset field)
+      const uint32_t a_lo = A_MN ? (((saddr(smem + s * kStageBytes) & 0x3FFFF) >> 4) | (512u << 16))
+                                 : desc_lo(saddr(smem + s * kStageBytes));
+      // (block 32, MN-major B: groups of 32 columns in the 64-byte swizzle, 64 k-rows of 64 bytes
+      // = 4 KB apart, 8-row groups of 512 bytes, 16 rows = 1 KB per K-step)
+      const bool b64s = B_MN && block == 32;
+      const uint32_t b_lo = B_MN ? (((saddr(smem + s * kStageBytes + kStageA) & 0x3FFFF) >> 4) | ((b64s ? 256u : 512u) << 16))
+                                 : desc_lo(saddr(smem + s * kStageBytes + kStageA));
+      const uint32_t b_hi = b64s ? ((512u >> 4) | (1u << 14) | (4u << 29)) : kDescHi;
+      ok = mbar_wait_warp(&bar_full[s], (it / kStages) & 1, fl);
+      if (!ok) break;
+      fence_after();
+      if (me) {
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
           const uint32_t acc = (it > 0 || ks > 0) ? 1u : 0u;
@@ -248,8 +246,9 @@ sdd_tc_kernel(const __grid_constant__ CUtensorMap m_a, const __grid_constant__ C
         }
         commit(&bar_empty[s]);
       }
-      if (ok) commit(&bar_done);
+      __syncwarp();
     }
+    if (ok && me) commit(&bar_done);
   } else {
     // ------------------------------------------------------------------ write-back
     const int row = warp * 32 + lane;
@@ -317,18 +316,20 @@ int dense_map(CUtensorMap* m, const void* p, int dtype, int Z, int H, int64_t in
 
 }  // namespace
 
-// True when sdd_tc covers the case: FP16 / BF16, block 32 / 64 / 128, K a multiple of 64, dense
-// operands with one unit inner stride and 16-byte friendly addresses and strides.
-bool sdd_tc_eligible(const void* a, const void* b, const void* c, int dtype, int block, int K,
+// True when sdd_tc covers the case: FP16 / BF16, block 32 / 64 / 128, dense operands with one unit
+// inner stride and 16-byte friendly addresses and strides.  Strides of dimensions of extent 1 carry
+// no meaning.
+bool sdd_tc_eligible(const void* a, const void* b, const void* c, int dtype, int block, int Z, int H,
                      int64_t a_sz, int64_t a_sh, int64_t a_sm, int64_t a_sk,
                      int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn, int64_t c_sz) {
   if (dtype != BSP_F16 && dtype != BSP_BF16) return false;
-  if ((block != 32 && block != 64 && block != 128) || K % 64) return false;
+  if (block != 32 && block != 64 && block != 128) return false;
   if ((a_sm != 1) == (a_sk != 1) || (b_sk != 1) == (b_sn != 1)) return false;
   const int64_t a_outer = a_sk == 1 ? a_sm : a_sk, b_outer = b_sk == 1 ? b_sn : b_sk;
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) return false;
   if ((a_sz | a_sh | a_outer | b_sz | b_sh | b_outer | c_sz) & 7) return false;
-  if (a_sz <= 0 || a_sh <= 0 || a_outer <= 0 || b_sz <= 0 || b_sh <= 0 || b_outer <= 0) return false;   // TMA strides: no broadcast
+  // TMA strides: no broadcast
+  if ((Z > 1 && (a_sz <= 0 || b_sz <= 0)) || (H > 1 && (a_sh <= 0 || b_sh <= 0)) || a_outer <= 0 || b_outer <= 0) return false;
   return true;
 }
 

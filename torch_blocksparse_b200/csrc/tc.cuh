@@ -82,6 +82,18 @@ BSP_DEVI bool mbar_wait_warp_idle(uint64_t* bar, uint32_t parity, volatile int* 
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// ---- roles of whole warps -----------------------------------------------------
+// Loops that issue loads or MMAs are run by all 32 lanes, which wait together; only the
+// instructions that act are executed by one lane (elect_one).  The operands of such instructions
+// live in the warp's uniform registers: inside a branch of one lane every one of them would first
+// have to be moved there.
+BSP_DEVI int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+BSP_DEVI bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+  return is != 0;
+}
+
 // ---- TMA ----------------------------------------------------------------------
 BSP_DEVI void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"

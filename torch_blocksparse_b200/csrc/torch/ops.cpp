@@ -130,7 +130,8 @@ bool block_format(const Tensor& x, int64_t block) {
 }
 Tensor prep_sparse(const Tensor& x, int64_t block) { return block_format(x, block) ? x : x.contiguous(); }
 
-Tensor sdd(const MatMulOp& p, Tensor a, Tensor b, bool ta, bool tb, bool tc, double* time) {
+// `any_k`: the reduction size need not be a multiple of 16 (both operands must be k-strided then).
+Tensor sdd(const MatMulOp& p, Tensor a, Tensor b, bool ta, bool tb, bool tc, double* time, bool any_k = false) {
   if (tc) {
     std::swap(a, b);
     const bool t = ta;
@@ -139,7 +140,7 @@ Tensor sdd(const MatMulOp& p, Tensor a, Tensor b, bool ta, bool tb, bool tc, dou
   }
   const Dense A = prep_dense(a), B = prep_dense(b);
   const int64_t Z = a.size(0), K = a.size(ta ? 2 : 3), M = a.size(ta ? 3 : 2), N = b.size(tb ? 2 : 3);
-  TORCH_CHECK_VALUE(K % 16 == 0, "Reduction size for SDD must be a multiple of 16");
+  TORCH_CHECK_VALUE(any_k || K % 16 == 0, "Reduction size for SDD must be a multiple of 16");
   TORCH_CHECK_VALUE(b.size(0) == Z && b.size(1) == a.size(1) && a.size(1) == p.H && b.size(tb ? 3 : 2) == K &&
                         M == p.Mb * p.block && N == p.Nb * p.block,
                     "sdd: operand shapes ", a.sizes(), ", ", b.sizes(), " do not match layout [", p.H, ", ", p.Mb, ", ", p.Nb,
@@ -153,49 +154,61 @@ Tensor sdd(const MatMulOp& p, Tensor a, Tensor b, bool ta, bool tb, bool tc, dou
   return c;
 }
 
-// The free dimension of the dense operand, padded with zeros to a multiple of 16 bytes (the kernels
-// read and write it in 16-byte pieces); the result is cut back to the caller's size.
-Tensor pad_free(const Tensor& x, int64_t dim, int64_t* pad) {
-  const int64_t vec = x.scalar_type() == at::kFloat ? 4 : 8;
-  *pad = (vec - x.size(dim) % vec) % vec;
-  if (*pad == 0) return x;
-  return dim == 3 ? at::constant_pad_nd(x, {0, *pad}) : at::constant_pad_nd(x, {0, 0, 0, *pad});
+// A dense operand whose free dimension `dim` is contiguous and no multiple of 16 bytes is padded with
+// zeros (its rows would end inside a 16-byte piece); the result is cut back to the caller's size.
+Tensor pad_free(const Tensor& x, int64_t dim, int64_t vec) {
+  const int64_t pad = (vec - x.size(dim) % vec) % vec;
+  if (pad == 0 || (x.stride(5 - dim) == 1 && x.stride(dim) != 1)) return x;
+  return dim == 3 ? at::constant_pad_nd(x, {0, pad}) : at::constant_pad_nd(x, {0, 0, 0, pad});
+}
+// The result of dsd / dds, [Z, H, rows, cols], for kernels that compute `n` entries of the free
+// dimension of which the caller sees `keep`.  Rows along a free dimension are a multiple of 16 bytes apart.
+struct Out {
+  Tensor c;
+  int64_t free_dim, keep;
+  Tensor cut() const { return c.size(free_dim) == keep ? c : c.narrow(free_dim, 0, keep); }
+};
+Out make_out(const Tensor& like, int64_t Z, int64_t H, int64_t rows, int64_t cols, int64_t free_dim, int64_t keep, int64_t vec) {
+  if (free_dim == 3) cols = (cols + vec - 1) / vec * vec;
+  return {at::empty({Z, H, rows, cols}, like.options()), free_dim, keep};
 }
 
 Tensor dsd(const MatMulOp& p, const Tensor& a, const Tensor& b0, bool ta, bool tb, bool tc, double* time) {
-  int64_t pad = 0;
-  const Tensor s = prep_sparse(a, p.block), b = pad_free(b0, tb ? 2 : 3, &pad);
+  const int64_t vec = vec_of(b0), fd = tb ? 2 : 3;
+  const Tensor s = prep_sparse(a, p.block), b = pad_free(b0, fd, vec);
   const Dense B = prep_dense(b);
-  const int64_t Z = b.size(0), H = b.size(1), M = p.block * (ta ? p.Nb : p.Mb), N = b.size(tb ? 2 : 3);
+  const int64_t Z = b.size(0), H = b.size(1), M = p.block * (ta ? p.Nb : p.Mb), N = b.size(fd);
   TORCH_CHECK_VALUE(a.size(0) == Z && a.size(1) == p.nnz && a.size(2) == p.block && a.size(3) == p.block && H == p.H &&
                         b.size(tb ? 3 : 2) == p.block * (ta ? p.Mb : p.Nb),
                     "dsd: operand shapes ", a.sizes(), ", ", b.sizes(), " do not match layout [", p.H, ", ", p.Mb, ", ", p.Nb,
                     "] with block ", p.block);
-  Tensor c = tc ? at::empty({Z, H, N, M}, a.options()) : at::empty({Z, H, M, N}, a.options());
+  const Out o = make_out(a, Z, H, tc ? N : M, tc ? M : N, tc ? 2 : 3, b0.size(fd), vec);
+  const Tensor& c = o.c;
   Timer timer(time, c);
   check(bsp_dsd(s.const_data_ptr(), B.t.const_data_ptr(), c.mutable_data_ptr(), dtype_code(a), p.block, Z, H, N, s.stride(0), ta,
                 B.s[0], B.s[1], B.s[tb ? 3 : 2], B.s[tb ? 2 : 3], c.stride(0), c.stride(1), c.stride(tc ? 3 : 2),
                 c.stride(tc ? 2 : 3), p.h(), p.d(), stream_of(c)));
   timer.stop();
-  return pad ? c.narrow(tc ? 2 : 3, 0, N - pad) : c;
+  return o.cut();
 }
 
 Tensor dds(const MatMulOp& p, const Tensor& a0, const Tensor& b, bool ta, bool tb, bool tc, double* time) {
-  int64_t pad = 0;
-  const Tensor a = pad_free(a0, ta ? 3 : 2, &pad), s = prep_sparse(b, p.block);
+  const int64_t vec = vec_of(a0), fd = ta ? 3 : 2;
+  const Tensor a = pad_free(a0, fd, vec), s = prep_sparse(b, p.block);
   const Dense A = prep_dense(a);
-  const int64_t Z = a.size(0), H = a.size(1), M = a.size(ta ? 3 : 2), N = p.block * (tb ? p.Mb : p.Nb);
+  const int64_t Z = a.size(0), H = a.size(1), M = a.size(fd), N = p.block * (tb ? p.Mb : p.Nb);
   TORCH_CHECK_VALUE(b.size(0) == Z && b.size(1) == p.nnz && b.size(2) == p.block && b.size(3) == p.block && H == p.H &&
                         a.size(ta ? 2 : 3) == p.block * (tb ? p.Nb : p.Mb),
                     "dds: operand shapes ", a.sizes(), ", ", b.sizes(), " do not match layout [", p.H, ", ", p.Mb, ", ", p.Nb,
                     "] with block ", p.block);
-  Tensor c = tc ? at::empty({Z, H, N, M}, a.options()) : at::empty({Z, H, M, N}, a.options());
+  const Out o = make_out(a, Z, H, tc ? N : M, tc ? M : N, tc ? 3 : 2, a0.size(fd), vec);
+  const Tensor& c = o.c;
   Timer timer(time, c);
   check(bsp_dds(A.t.const_data_ptr(), s.const_data_ptr(), c.mutable_data_ptr(), dtype_code(a), p.block, Z, H, M, A.s[0], A.s[1],
                 A.s[ta ? 3 : 2], A.s[ta ? 2 : 3], s.stride(0), tb, c.stride(0), c.stride(1), c.stride(tc ? 3 : 2),
                 c.stride(tc ? 2 : 3), p.h(), p.d(), stream_of(c)));
   timer.stop();
-  return pad ? c.narrow(tc ? 3 : 2, 0, M - pad) : c;
+  return o.cut();
 }
 
 Tensor product(char c, char a, char b, const MatMulOp& p, const Tensor& x, const Tensor& y, bool tx, bool ty, bool tc, double* time) {
@@ -246,6 +259,49 @@ Tensor matmul_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& a0, cons
   const c10::cuda::CUDAGuard guard(a.device());
   if (at::GradMode::is_enabled() && (a.requires_grad() || b.requires_grad())) return MatMulFn::apply(a, b, p, times);
   return product(p->mode[0], p->mode[1], p->mode[2], *p, a, b, p->trans_a, p->trans_b, false, times ? &times->c : nullptr);
+}
+
+// y = x . W for x [..., in_features] and the nonzero blocks of W ([in, out], one head): the dds
+// product on the rows of x, without copies for rows of any number; the weight's gradient reduces
+// over the rows (torch_blocksparse/matmul.py:693-709).
+struct LinearFn : torch::autograd::Function<LinearFn> {
+  static Tensor run(const MatMulOp& p, const Tensor& x, const Tensor& w, double* time) {
+    std::vector<int64_t> shape = x.sizes().vec();
+    const Tensor y = dds(p, x.reshape({1, 1, -1, x.size(-1)}), w.unsqueeze(0), false, false, false, time);
+    shape.back() = y.size(3);
+    return y.view(shape);
+  }
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const c10::intrusive_ptr<MatMulOp>& p,
+                        double* time) {
+    ctx->save_for_backward({x, w});
+    ctx->saved_data["p"] = c10::IValue::make_capsule(p);
+    return run(*p, x, w, time);
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+    const auto p = c10::static_intrusive_pointer_cast<MatMulOp>(ctx->saved_data["p"].toCapsule());
+    const variable_list s = ctx->get_saved_variables();
+    const c10::cuda::CUDAGuard guard(s[0].device());
+    const Tensor x = s[0].reshape({1, 1, -1, s[0].size(-1)}), w = s[1].unsqueeze(0);
+    const Tensor dy = grads[0].reshape({1, 1, -1, grads[0].size(-1)});
+    variable_list out(4);
+    if (ctx->needs_input_grad(0)) out[0] = dds(*p, dy, w, false, true, false, nullptr).view(s[0].sizes());
+    if (ctx->needs_input_grad(1)) {
+      // (the kernels read x and dy k-strided here, so any number of rows; other strides are copied)
+      const bool strided = x.stride(3) == 1 && dy.stride(3) == 1;
+      out[1] = sdd(*p, strided ? x : x.contiguous(), strided ? dy : dy.contiguous(), true, false, false, nullptr, true).squeeze(0);
+    }
+    return out;
+  }
+};
+
+Tensor linear_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& x, const Tensor& w0, const c10::intrusive_ptr<Times>& times) {
+  require_cuda(x);
+  require_cuda(w0);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Tensor w = w0.scalar_type() == x.scalar_type() ? w0 : w0.to(x.scalar_type());
+  double* time = times ? &times->c : nullptr;
+  if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad())) return LinearFn::apply(x, w, p, time);
+  return LinearFn::run(*p, x, w, time);
 }
 
 // ---- rpe and masks -----------------------------------------------------------------------------
@@ -510,7 +566,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         return p;
       }))
       .def("__call__", &matmul_call, py::arg("a"), py::arg("b"), py::arg("times") = c10::intrusive_ptr<Times>(),
-           py::call_guard<py::gil_scoped_release>());
+           py::call_guard<py::gil_scoped_release>())
+      .def("linear", &linear_call, py::call_guard<py::gil_scoped_release>());
   py::class_<SoftmaxOp, c10::intrusive_ptr<SoftmaxOp>>(m, "SoftmaxOp")
       .def(py::init([](Tensor lut, int64_t maxlut, int64_t H, int64_t Mb, int64_t Nb, int64_t block) {
         auto p = c10::make_intrusive<SoftmaxOp>();

@@ -154,14 +154,10 @@ class Linear(torch.nn.Module):
     def forward(self, input):
         if input.size(-1) != self.in_features:
             raise ValueError('Linear: expected %d input features, got %d' % (self.in_features, input.size(-1)))
-        lead = input.shape[:-1]
-        x = input.reshape(1, 1, -1, self.in_features)
-        # rows are the reduction dimension of the weight gradient (an sdd product), which must be
-        # a multiple of 16 (matmul.py:318-319); zero rows change nothing
-        pad = (-x.size(2)) % 16
-        if pad:
-            x = torch.nn.functional.pad(x, (0, 0, 0, pad))
-        y = self.matmul(x, self.weight.to(x.dtype))
-        if pad:
-            y = y[:, :, :y.size(2) - pad]
-        return y.reshape(*lead, self.out_features)
+        mm = self.matmul
+        op = mm._ops.get(input.get_device()) or mm._op(input.device)
+        times = _lib.ops().Times() if mm.bench else None
+        y = op.linear(input, self.weight, times)
+        if times is not None:
+            mm.time_c = times.c
+        return y
