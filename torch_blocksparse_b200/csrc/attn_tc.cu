@@ -315,7 +315,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
   __shared__ uint32_t tmem_slot;
   __shared__ int failed[2];
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   // One-dimensional grid, batch entries of a tile adjacent: CTAs start in the order of the
   // tiles' lengths (longest first) over the whole launch, not per batch entry.
   const int z = blockIdx.x % a.Z;
@@ -412,7 +412,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
 
   if (warp >= NC) {
     // ------------------------------------------------------------------ loader and MMA issuers
-    if (lane == 0) {
+    {
+      const bool me = elect_one();            // the lane that issues; all lanes wait (tc.cuh)
       const uint32_t idesc_kk = instr_desc(128, 64, 0, IsBf16<T>::v);   // A, B K-major
       const uint32_t idesc_mn = instr_desc(128, 64, 1, IsBf16<T>::v);   // B MN-major
       // Descriptor low words: a K-step advances a K-major operand by 32 bytes (2 units of 16
@@ -445,6 +446,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       // part: 1 = first product (S), 2 = second (dP), 3 = both, one commit each call
       auto scores = [&](int t, int part, uint64_t* bar) {
         const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS;
+        if (!me) return;
         if (C::RES_T) {
           const uint32_t tq = tmem + C::RES_BASE;
           if (part & 1) {
@@ -489,6 +491,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       const uint32_t idesc_acc = WIDE ? instr_desc(128, 128, 1, IsBf16<T>::v) : idesc_mn;
       auto wide = [](uint64_t d) { return WIDE ? ((d & ~0x3FFF0000ull) | (512ull << 16)) : d; };
       auto accumulate = [&](int t) {
+        if (!me) return;
         const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS;
         const uint32_t ta = tmem + C::ACC_BASE;
         const uint32_t later = t > 0 ? 1u : 0u;
@@ -525,21 +528,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       // only for the compute warps; neither queues behind the other's barrier.  The accumulate
       // issuer, which has less to issue, also refills the ring of chunk operands.
       if (warp == NC) {
-        bool ok = mbar_wait(C::RES_T ? &bar_rt : &bar_res, 0, fl);
+        bool ok = mbar_wait_warp(C::RES_T ? &bar_rt : &bar_res, 0, fl);
         for (int t = 0; ok && t < ntiles; ++t) {
           prep_scores(t);
-          ok = mbar_wait(&bar_full[t % ST], (t / ST) & 1, fl);
+          ok = mbar_wait_warp(&bar_full[t % ST], (t / ST) & 1, fl);
           if (C::ER || C::ER2) {
-            if (ok && t >= 1) ok = mbar_wait(&bar_rd, (t - 1) & 1, fl);     // scores of chunk t - 1 are in registers
+            if (ok && t >= 1) ok = mbar_wait_warp(&bar_rd, (t - 1) & 1, fl);     // scores of chunk t - 1 are in registers
           } else {
-            if (ok && t >= NBUF) ok = mbar_wait(&bar_acc[(t - NBUF) & 3], ((t - NBUF) >> 2) & 1, fl);
+            if (ok && t >= NBUF) ok = mbar_wait_warp(&bar_acc[(t - NBUF) & 3], ((t - NBUF) >> 2) & 1, fl);
           }
           if (!ok) break;
           fence_after();
           if (C::ER2) {
             scores(t, 1, &bar_s[0]);
             if (t >= 1) {                                   // dP^T's columns still hold the operands of chunk t - 1
-              ok = mbar_wait(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
+              ok = mbar_wait_warp(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
               if (!ok) break;
               fence_after();
             }
@@ -547,6 +550,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
           } else {
             scores(t, 3, &bar_s[t % NBUF]);
           }
+          __syncwarp();
         }
       } else {
         bool ok = true;
@@ -556,18 +560,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
           const int tn = t - 1 + ST;
           if (t >= 1 && tn < ntiles) {
             const int crow_n = a.chunk[first + tn] * 64;
-            ok = mbar_wait(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
+            ok = mbar_wait_warp(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
             if (!ok) break;
-            load_chunk(tn, crow_n);
+            if (me) load_chunk(tn, crow_n);
+            __syncwarp();
           }
           prep_acc(t);
-          ok = mbar_wait(&bar_full[t % ST], (t / ST) & 1, fl) &&
-               (C::ER ? mbar_wait(&bar_p[t & 1], (t >> 1) & 1, fl) : mbar_wait(&bar_p[t % NBUF], (t / NBUF) & 1, fl));
+          ok = mbar_wait_warp(&bar_full[t % ST], (t / ST) & 1, fl) &&
+               (C::ER ? mbar_wait_warp(&bar_p[t & 1], (t >> 1) & 1, fl) : mbar_wait_warp(&bar_p[t % NBUF], (t / NBUF) & 1, fl));
           if (!ok) break;
           fence_after();
           accumulate(t);
+          __syncwarp();
         }
-        if (ok) commit(&bar_done);
+        if (ok && me) commit(&bar_done);
       }
     }
   } else {
