@@ -190,8 +190,8 @@ int bsp_softmax_lut_from_meta(const int32_t* meta_hdr, const int32_t* meta, int3
  *   chunk [E]  mask [E]  sub [E]  order [n] (tiles sorted longest first)
  *   sub: per half of the tile 16 bits saying which 16 x 16 pieces of the 64 x
  *   64 position lie in a nonzero block (all ones for blocks 64 and 128).
- * block must be 16, 32, 64 or 128, and L a multiple of 64 (else
- * BSP_ERR_UNSUPPORTED).
+ * block must be 16, 32, 64 or 128 (else BSP_ERR_UNSUPPORTED).  When L is no
+ * multiple of 64 the pieces of the last position past L are absent.
  */
 #define BSP_TILES_MAGIC 0x42535054
 #define BSP_TILES_HEADER 8
@@ -320,7 +320,7 @@ int bsp_attn_tiles_validate(const int32_t* tiles, int64_t len, int* code, int* p
  * (torch_blocksparse/deepspeedsparseselfattention.py:157-166) without writing
  * the score tensor to memory.  q, k, v, o are [Z, H, L, D] with unit stride on
  * D and the given z / h / row strides; lse is FP32 [Z, H, L]: per row
- * log2(sum_j exp(f_j)) of the pre-softmax values f, consumed by the backward.  D is 64 or 128; dtype F16 or BF16.
+ * log2(sum_j exp(f_j)) of the pre-softmax values f, consumed by the backward.  D is a multiple of 8 up to 128 (64 or 128 on the mma.sync kernels); dtype F16 or BF16.
  * tiles / tiles_hdr: optional device copy of the buffer written by
  * bsp_attn_tiles_build and a HOST pointer to its first BSP_TILES_HEADER ints.
  * When given (lists built for this block size; q, k, v with positive strides;

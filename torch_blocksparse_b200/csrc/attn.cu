@@ -37,10 +37,10 @@ namespace {
 // position bias and an attention mask are taken when they can be fetched in 16-byte pieces
 // (aligned base, strides that are multiples of 8 elements); an attention mask the caller vouches
 // to be the causal one (flag 2) is derived from the indices instead of being read.
-bool tc_eligible(const int32_t* tiles_hdr, const int32_t* tiles, int block, int L, int D,
+bool tc_eligible(const int32_t* tiles_hdr, const int32_t* tiles, int block,
                  const void* rpe, int64_t rpe_sz, int64_t rpe_sh, int64_t rpe_sr,
                  const void* kpm, int64_t kpm_sz, const void* am, int64_t am_sr) {
-  if (!(tiles_hdr && tiles && (D == 64 || D == 128))) return false;
+  if (!(tiles_hdr && tiles)) return false;
   // the lists were built for this block size (blocks 16 and 32 run on 64-wide lists with masks of 16 x 16 pieces)
   if (!((block == 16 || block == 32 || block == 64 || block == 128) && tiles_hdr[7] == block)) return false;
   if (kpm && ((reinterpret_cast<uintptr_t>(kpm) & 15) || (kpm_sz & 7))) return false;
@@ -112,7 +112,7 @@ int fill_common(AttnArgs& p, int dtype, int block, int Z, int H, int L, int D,
   if (dtype != BSP_F16 && dtype != BSP_BF16)
     return fail(BSP_ERR_UNSUPPORTED, "fused attention supports FP16 and BF16 (use the three-op chain for FP32)");
   if (!valid_block(block)) return fail(BSP_ERR_INVALID, "attention: block must be 16, 32, 64 or 128 (got %d)", block);
-  if (D != 64 && D != 128) return fail(BSP_ERR_UNSUPPORTED, "fused attention supports head dimensions 64 and 128 (got %d)", D);
+  if (D <= 0 || D > 128 || D % 8) return fail(BSP_ERR_UNSUPPORTED, "fused attention supports head dimensions that are multiples of 8 up to 128 (got %d)", D);
   if (Z <= 0 || Z > 65535) return fail(BSP_ERR_INVALID, "attention: batch %d outside [1, 65535]", Z);
   if (!hdr || !meta) return fail(BSP_ERR_INVALID, "attention: metadata pointer is NULL");
   if (hdr[0] != BSP_META_MAGIC) return fail(BSP_ERR_INVALID, "attention: metadata header is corrupt (bad magic)");
@@ -157,7 +157,7 @@ extern "C" int bsp_attn_fwd(const void* q, const void* k, const void* v, void* o
   p.q_sz = q_sz; p.q_sh = q_sh; p.q_sr = q_sr; p.k_sz = k_sz; p.k_sh = k_sh; p.k_sr = k_sr;
   p.v_sz = v_sz; p.v_sh = v_sh; p.v_sr = v_sr; p.o_sz = o_sz; p.o_sh = o_sh; p.o_sr = o_sr;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (tc_eligible(tiles_hdr, tiles, block, L, D, rpe, rpe_sz, rpe_sh, rpe_sr, kpm, kpm_sz, am, am_sr) &&
+  if (tc_eligible(tiles_hdr, tiles, block, rpe, rpe_sz, rpe_sh, rpe_sr, kpm, kpm_sz, am, am_sr) &&
       tma_strides(Z, H, q_sz, q_sh, q_sr) && tma_strides(Z, H, k_sz, k_sh, k_sr) && tma_strides(Z, H, v_sz, v_sh, v_sr)) {
     const XtHost xt = xt_of(rpe, rpe_sz, rpe_sh, rpe_sr, am, am_sr, am_mul);
     return attn_fwd_tc(q, k, v, o, lse, dtype, Z, H, L, D, q_sz, q_sh, q_sr, k_sz, k_sh, k_sr, v_sz, v_sh, v_sr,
@@ -200,12 +200,12 @@ extern "C" int bsp_attn_bwd_parts(const void* q, const void* k, const void* v, c
   p.v_sz = v_sz; p.v_sh = v_sh; p.v_sr = v_sr; p.o_sz = o_sz; p.o_sh = o_sh; p.o_sr = o_sr;
   p.do_sz = do_sz; p.do_sh = do_sh; p.do_sr = do_sr;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (tc_eligible(tiles_hdr, tiles, block, L, D, rpe, rpe_sz, rpe_sh, rpe_sr, kpm, kpm_sz, am, am_sr) &&
+  if (tc_eligible(tiles_hdr, tiles, block, rpe, rpe_sz, rpe_sh, rpe_sr, kpm, kpm_sz, am, am_sr) &&
       tma_strides(Z, H, q_sz, q_sh, q_sr) && tma_strides(Z, H, k_sz, k_sh, k_sr) && tma_strides(Z, H, v_sz, v_sh, v_sr) &&
       tma_strides(Z, H, do_sz, do_sh, do_sr)) {
     // delta = rowsum(o * do) by the streaming kernel, the two matrix kernels on tcgen05
     if (parts & 1) {
-      const int rc = dtype == BSP_F16 ? attn_bwd_t<__half>(p, block, D, Z, 1, st) : attn_bwd_t<__nv_bfloat16>(p, block, D, Z, 1, st);
+      const int rc = dtype == BSP_F16 ? attn_delta_t<__half>(p, D, Z, st) : attn_delta_t<__nv_bfloat16>(p, D, Z, st);
       if (rc) return rc;
     }
     if (!(parts & 6)) return BSP_OK;

@@ -265,36 +265,19 @@ __global__ void __launch_bounds__(AttnCfg<B, D>::NT) attn_fwd_kernel(AttnArgs p)
 // ---------------------------------------------------------------------------
 // backward (1): delta[z, h, row] = sum_d O * dO
 // ---------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void attn_delta_kernel(AttnArgs p, int rows_total) {
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= rows_total) return;
-  const int lane = threadIdx.x & 31;
-  const int r = row % p.L, zh = row / p.L, h = zh % p.H, z = zh / p.H;
-  const T* o = reinterpret_cast<const T*>(p.o) + z * p.o_sz + h * p.o_sh + (int64_t)r * p.o_sr;
-  const T* d = reinterpret_cast<const T*>(p.dout) + z * p.do_sz + h * p.do_sh + (int64_t)r * p.do_sr;
-  float acc = 0.f;
-  for (int c = lane * 2; c < D; c += 64) {
-    acc += ldf(o + c) * ldf(d + c) + ldf(o + c + 1) * ldf(d + c + 1);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) p.delta[row] = acc;
-}
-
-// The same with 16-byte loads: D / 8 lanes per row, several rows per warp.  Needs 16-byte
-// aligned rows of O and dO (checked by the launcher).
-template <typename T, int D>
-__global__ void __launch_bounds__(256) attn_delta_vec_kernel(AttnArgs p, int rows_total) {
-  constexpr int LPR = D / 8, RPW = 32 / LPR;
+// LPR lanes per row of at most 8 LPR elements, a 16-byte load each, several rows per warp.  Rows of
+// O and dO are 16-byte aligned (checked by the callers), the head dimension is a multiple of 8.
+template <typename T, int LPR>
+__global__ void __launch_bounds__(256) attn_delta_vec_kernel(AttnArgs p, int rows_total, int d) {
+  constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * RPW + lane / LPR;
   float acc = 0.f;
-  if (row < rows_total) {
+  if (row < rows_total && (lane % LPR) * 8 < d) {
     const int r = row % p.L, zh = row / p.L, h = zh % p.H, z = zh / p.H;
-    const T* o = reinterpret_cast<const T*>(p.o) + z * p.o_sz + h * p.o_sh + (int64_t)r * p.o_sr + (lane % LPR) * 8;
-    const T* d = reinterpret_cast<const T*>(p.dout) + z * p.do_sz + h * p.do_sh + (int64_t)r * p.do_sr + (lane % LPR) * 8;
-    const uint4 ov = __ldg(reinterpret_cast<const uint4*>(o)), dv = __ldg(reinterpret_cast<const uint4*>(d));
+    const T* op = reinterpret_cast<const T*>(p.o) + z * p.o_sz + h * p.o_sh + (int64_t)r * p.o_sr + (lane % LPR) * 8;
+    const T* dp = reinterpret_cast<const T*>(p.dout) + z * p.do_sz + h * p.do_sh + (int64_t)r * p.do_sr + (lane % LPR) * 8;
+    const uint4 ov = __ldg(reinterpret_cast<const uint4*>(op)), dv = __ldg(reinterpret_cast<const uint4*>(dp));
     const T* oe = reinterpret_cast<const T*>(&ov);
     const T* de = reinterpret_cast<const T*>(&dv);
 #pragma unroll
@@ -527,6 +510,21 @@ __global__ void __launch_bounds__(AttnCfg<B, D>::NT) attn_bwd_q_kernel(AttnArgs 
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+}  // namespace
+
+// delta = rowsum(O * dO)
+template <typename T>
+int attn_delta_t(const AttnArgs& p, int D, int Z, cudaStream_t st) {
+  const int rows = Z * p.H * p.L;
+  if (D <= 64) attn_delta_vec_kernel<T, 8><<<(rows + 31) / 32, 256, 0, st>>>(p, rows, D);
+  else attn_delta_vec_kernel<T, 16><<<(rows + 15) / 16, 256, 0, st>>>(p, rows, D);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(BSP_ERR_CUDA, "attention delta launch failed: %s", cudaGetErrorString(e));
+  return BSP_OK;
+}
+
+namespace {
+
 template <typename K>
 int set_smem(K kern, int bytes, const char* what) {
   if (bytes > 48 * 1024) {
@@ -555,15 +553,8 @@ int attn_fwd_launch(const AttnArgs& p, int Z, cudaStream_t st) {
 template <typename T, int B, int D>
 int attn_bwd_launch(const AttnArgs& p, int Z, int parts, cudaStream_t st) {
   using C = AttnCfg<B, D>;
-  const int rows = Z * p.H * p.L;
-  if (parts & 1) {
-    const bool vec = ((reinterpret_cast<uintptr_t>(p.o) | reinterpret_cast<uintptr_t>(p.dout)) & 15) == 0 &&
-                     ((p.o_sz | p.o_sh | p.o_sr | p.do_sz | p.do_sh | p.do_sr) & 7) == 0;
-    constexpr int RPC = 8 * (32 / (D / 8));               // rows per CTA of the vector kernel
-    if (vec) attn_delta_vec_kernel<T, D><<<(rows + RPC - 1) / RPC, 256, 0, st>>>(p, rows);
-    else attn_delta_kernel<T, D><<<(rows + 7) / 8, 256, 0, st>>>(p, rows);
-    if (int rc = launched("attention delta")) return rc;
-  }
+  if (parts & 1)
+    if (int rc = attn_delta_t<T>(p, D, Z, st)) return rc;
   constexpr int BT = (D > 64 && B > 32) ? 32 : C::BN;
   if (parts & 2) {
     const int bytes = (2 * B + 4 * BT) * C::PD * int(sizeof(T)) + 4 * BT * int(sizeof(float));
@@ -590,7 +581,7 @@ int attn_fwd_t(const AttnArgs& p, int block, int D, int Z, cudaStream_t st) {
   BSP_ATTN_CASE(16, 64) BSP_ATTN_CASE(32, 64) BSP_ATTN_CASE(64, 64) BSP_ATTN_CASE(128, 64)
   BSP_ATTN_CASE(16, 128) BSP_ATTN_CASE(32, 128) BSP_ATTN_CASE(64, 128) BSP_ATTN_CASE(128, 128)
 #undef BSP_ATTN_CASE
-  return fail(BSP_ERR_UNSUPPORTED, "fused attention supports head dimensions 64 and 128 (got %d)", D);
+  return fail(BSP_ERR_UNSUPPORTED, "without tile lists the fused attention supports head dimensions 64 and 128 (got %d)", D);
 }
 
 template <typename T>
@@ -599,7 +590,7 @@ int attn_bwd_t(const AttnArgs& p, int block, int D, int Z, int parts, cudaStream
   BSP_ATTN_CASE(16, 64) BSP_ATTN_CASE(32, 64) BSP_ATTN_CASE(64, 64) BSP_ATTN_CASE(128, 64)
   BSP_ATTN_CASE(16, 128) BSP_ATTN_CASE(32, 128) BSP_ATTN_CASE(64, 128) BSP_ATTN_CASE(128, 128)
 #undef BSP_ATTN_CASE
-  return fail(BSP_ERR_UNSUPPORTED, "fused attention supports head dimensions 64 and 128 (got %d)", D);
+  return fail(BSP_ERR_UNSUPPORTED, "without tile lists the fused attention supports head dimensions 64 and 128 (got %d)", D);
 }
 
 }  // namespace bsp

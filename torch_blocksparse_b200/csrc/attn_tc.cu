@@ -4,11 +4,15 @@
 // Same contract as the mma.sync kernels of attn_impl.cuh (which replace the
 // sdd -> softmax -> dsd chain of
 // torch_blocksparse/deepspeedsparseselfattention.py:157-166 and its backward);
-// this path covers head dimension 64 and 128, FP16 / BF16, without rpe and
-// attention mask; a key-padding mask is a per-key bias here.  Blocks 64 and
-// 128 map onto its tiles directly; blocks 16 and 32 run on the lists of the
-// layout coarsened to 64, with the 16 x 16 pieces that no block covers masked
-// out of the scores.
+// this path covers head dimensions up to 128 (multiples of 8), FP16 / BF16.
+// Blocks 64 and 128 map onto its tiles directly; blocks 16 and 32 run on the
+// lists of the layout coarsened to 64, with the 16 x 16 pieces that no block
+// covers masked out of the scores.  The kernels are compiled for head dimensions
+// 64 and 128; smaller ones run on the next one with the missing columns zero:
+// TMA fills what lies outside a tensor with zeros, and the write-back stops at
+// the head dimension (32 instead of 64: the exponentials, not the products, bound
+// both).  A sequence that ends inside a chunk of 64 (blocks 16 and 32) works the
+// same way: its last pieces are absent from the lists.
 //
 // Geometry: every MMA has M = 128.  A CTA owns a tile of 128 rows of the
 // "outer" operand(s), resident in shared memory, made of two 64-row chunks (one
@@ -66,8 +70,8 @@ struct TcArgs {
   void* out0; void* out1;             // FWD: O | DQ: dQ | DKV: dK, dV
   float* lse_out;                     // FWD
   const float* lse; const float* delta;   // backward
-  int64_t o_sz, o_sh, o_sr;           // strides of O (FWD); gradients are contiguous [Z, H, L, D]
-  int Z, H, L, tiles_per_head;
+  int64_t o_sz, o_sh, o_sr;           // strides of the results
+  int Z, H, L, d, tiles_per_head;     // d: head dimension (D: what the kernel is compiled for)
   float scale, scale_log2;
   const int32_t *c01, *ptr, *chunk, *mask, *sub, *order;
   int fine;                            // the layout's blocks are smaller than 64: pieces of a position may be absent
@@ -242,7 +246,6 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   // stages (0.97 against 1.02 ms).
   static constexpr int XT_OFF = 2 * CH_BYTES + 1024;
   static constexpr int STAGE = 2 * CH_BYTES + ((MODE == DKV || BIAS || XT) ? 1024 : 0) + XT * 2 * 8192;   // + lse / delta, or the bias, of the chunk
-  static constexpr int TAIL_BYTES = MODE == DKV ? 512 : (BIAS ? 128 : 0);
   // score buffers in tensor memory: two (scores of the next chunk are computed while this
   // one is consumed) where the columns allow it with two CTAs per SM, else one
   static constexpr int NBUF = MODE == FWD ? 2 : (D == 64 ? 1 : 2);
@@ -277,15 +280,18 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   static constexpr int CTAS = (D == 64 && (XT == 0 || XT1_PAIR)) ? 2 : 1;
 };
 
-// Writes accumulator columns [c0, c0 + n) of this thread's tensor-memory lane to dst[c0 .. c0 + n) as 16-bit values.
+// Writes accumulator columns [c0, c0 + n) of this thread's tensor-memory lane to dst[c0 .. c0 + n) as 16-bit values
+// (`row` says whether this thread's row exists; columns from d on are not written)
 template <typename T>
-BSP_DEVI void store_acc(T* dst, uint32_t taddr, int c0, int n, float mul) {
+BSP_DEVI void store_acc(T* dst, uint32_t taddr, int c0, int n, int d, bool row, float mul) {
   for (int c = c0; c < c0 + n; c += 32) {
     uint32_t r[32];
     tmem_ld32(taddr + c, r);
     tmem_ld_wait();
+    if (!row) continue;
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
+      if (c + i >= d) break;
       uint4 v;
       v.x = pack16<T>(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul);
       v.y = pack16<T>(__uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul);
@@ -330,15 +336,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
   const int trow = quarter * 32 + lane;
   const int mychunk = trow < 64 ? c0 : c1;
   const int64_t grow = (int64_t)(mychunk < 0 ? 0 : mychunk) * 64 + (trow & 63);
-  const bool row_ok = mychunk >= 0 && warp < NC;
+  const bool row_ok = mychunk >= 0 && warp < NC && (!FINE || grow < a.L);   // (L is a multiple of 64 unless the blocks are smaller)
 
   if (ntiles == 0) {                                          // nothing in this tile: zeros, as the reference's products give
     if (row_ok && chalf == 0) {
-      T* o0 = MODE == FWD ? reinterpret_cast<T*>(a.out0) + z * a.o_sz + h * a.o_sh + grow * a.o_sr
-                          : reinterpret_cast<T*>(a.out0) + (zh + grow) * D;
-      for (int c = 0; c < D; c += 8) {
-        *reinterpret_cast<uint4*>(o0 + c) = make_uint4(0, 0, 0, 0);
-        if (MODE == DKV) *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out1) + (zh + grow) * D + c) = make_uint4(0, 0, 0, 0);
+      const int64_t at = z * a.o_sz + h * a.o_sh + grow * a.o_sr;
+      for (int c = 0; c < a.d; c += 8) {
+        *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out0) + at + c) = make_uint4(0, 0, 0, 0);
+        if (MODE == DKV) *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out1) + at + c) = make_uint4(0, 0, 0, 0);
       }
       if (MODE == FWD) a.lse_out[zh + grow] = kNegInfT;
     }
@@ -348,7 +353,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
   auto load_chunk = [&](int t, int crow) {
     const int stage = t % ST;
     unsigned char* sp = stg + stage * C::STAGE;
-    uint32_t bytes = 2 * C::CH_BYTES + C::TAIL_BYTES;
+    const int nr = FINE ? min(64, a.L - crow) : 64;             // rows of the chunk inside the sequence
+    uint32_t bytes = 2 * C::CH_BYTES + (MODE == DKV ? 8 : C::BIAS ? 2 : 0) * nr;
     if constexpr (XT) bytes += (uint32_t)((c1 < 0 ? 1 : 2) * 8192 * ((a.has_rpe ? 1 : 0) + (a.am_mode ? 1 : 0)));
     mbar_expect_tx(&bar_full[stage], bytes);
     if (t == a.skip_chunk) return;                             // (test hook: this stage never fills, its consumers' waits run out)
@@ -357,10 +363,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       tma_load_4d(sp + C::CH_BYTES + at * 8192, &m_ch1, &bar_full[stage], at * 64, crow, h, z);
     }
     if (MODE == DKV) {
-      bulk_load(sp + 2 * C::CH_BYTES, a.lse + zh + crow, 256, &bar_full[stage]);
-      bulk_load(sp + 2 * C::CH_BYTES + 256, a.delta + zh + crow, 256, &bar_full[stage]);
+      bulk_load(sp + 2 * C::CH_BYTES, a.lse + zh + crow, 4 * nr, &bar_full[stage]);
+      bulk_load(sp + 2 * C::CH_BYTES + 256, a.delta + zh + crow, 4 * nr, &bar_full[stage]);
     }
-    if (C::BIAS) bulk_load(sp + 2 * C::CH_BYTES, reinterpret_cast<const T*>(a.kpm) + z * a.kpm_sz + crow, 128, &bar_full[stage]);
+    if (C::BIAS) bulk_load(sp + 2 * C::CH_BYTES, reinterpret_cast<const T*>(a.kpm) + z * a.kpm_sz + crow, 2 * nr, &bar_full[stage]);
     if constexpr (XT) {
       // rows of rpe / the mask are queries, columns keys: the tile's rows are queries in the
       // forward and in dQ (the chunk brings keys), keys in dK / dV (the chunk brings queries)
@@ -375,6 +381,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
   // The thread that issues the loads sets up their barriers itself and starts the resident
   // operands and the first chunks at once: their latency overlaps the rest of the set-up
   // (other barriers, tensor-memory allocation, the block-wide synchronisation).
+  if (FINE && (MODE == DKV || C::BIAS) && (a.L & 63) && warp == NC) {
+    // the last chunk of a sequence fills only part of its lse / delta or bias values: the rest has
+    // to be finite (its scores are -inf)
+    for (int i = lane; i < ST * 64; i += 32)
+      *reinterpret_cast<uint4*>(stg + (i / 64) * C::STAGE + 2 * C::CH_BYTES + (i % 64) * 16) = make_uint4(0, 0, 0, 0);
+    fence_async_smem();
+    __syncwarp();
+  }
   if (tid == NC * 32) {
     mbar_init(&bar_res, 1);
     for (int s = 0; s < ST; ++s) mbar_init(&bar_full[s], 1);
@@ -731,10 +745,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
               uint4 v;
               v.x = pack16<T>(o[0], o[1]); v.y = pack16<T>(o[2], o[3]);
               v.z = pack16<T>(o[4], o[5]); v.w = pack16<T>(o[6], o[7]);
-              *reinterpret_cast<uint4*>(orow + c + i) = v;
+              if (row_ok && c + i < a.d) *reinterpret_cast<uint4*>(orow + c + i) = v;
             }
           }
-          if (chalf == 0) a.lse_out[zh + grow] = lsum > 0.f ? m + log2f(lsum) : kNegInfT;
+          if (chalf == 0 && row_ok) a.lse_out[zh + grow] = lsum > 0.f ? m + log2f(lsum) : kNegInfT;
         }
       }
     } else {
@@ -958,15 +972,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
         if (mychunk >= 0) {                                   // uniform per warp
           // the two threads of a row split the D output columns
           const uint32_t ta = tmem + C::ACC_BASE + lane_base;
-          T* o0 = reinterpret_cast<T*>(a.out0) + (zh + grow) * D;
+          const int64_t at = z * a.o_sz + h * a.o_sh + grow * a.o_sr;
+          T* o0 = reinterpret_cast<T*>(a.out0) + at;
           // (dS is formed without the score scale, which is applied here)
           const float ds_scale = a.scale;
           if (MODE == DQ) {
-            store_acc<T>(o0, ta, chalf * (D / 2), D / 2, ds_scale);
+            store_acc<T>(o0, ta, chalf * (D / 2), D / 2, a.d, row_ok, ds_scale);
           } else {
-            T* o1 = reinterpret_cast<T*>(a.out1) + (zh + grow) * D;
-            store_acc<T>(o1, ta, chalf * (D / 2), D / 2, 1.f);            // dV: accumulator columns [0, D)
-            store_acc<T>(o0 - D, ta, D + chalf * (D / 2), D / 2, ds_scale);    // dK: accumulator columns [D, 2D)
+            T* o1 = reinterpret_cast<T*>(a.out1) + at;
+            store_acc<T>(o1, ta, chalf * (D / 2), D / 2, a.d, row_ok, 1.f);            // dV: accumulator columns [0, D)
+            store_acc<T>(o0, ta + D, chalf * (D / 2), D / 2, a.d, row_ok, ds_scale);    // dK: accumulator columns [D, 2D)
           }
         }
       }
@@ -1082,10 +1097,10 @@ int launch(const Maps& m, const TcArgs& a, int n_tiles, int Z, cudaStream_t st, 
 template <int MODE, bool KPM, bool FINE, int XT>
 int launch_dt(int dtype, int D, const Maps& m, const TcArgs& a, int n_tiles, int Z, cudaStream_t st, const char* what) {
   if (dtype == BSP_F16) {
-    if (D == 64) return launch<__half, 64, MODE, KPM, FINE, XT>(m, a, n_tiles, Z, st, what);
+    if (D <= 64) return launch<__half, 64, MODE, KPM, FINE, XT>(m, a, n_tiles, Z, st, what);
     return launch<__half, 128, MODE, KPM, FINE, XT>(m, a, n_tiles, Z, st, what);
   }
-  if (D == 64) return launch<__nv_bfloat16, 64, MODE, KPM, FINE, XT>(m, a, n_tiles, Z, st, what);
+  if (D <= 64) return launch<__nv_bfloat16, 64, MODE, KPM, FINE, XT>(m, a, n_tiles, Z, st, what);
   return launch<__nv_bfloat16, 128, MODE, KPM, FINE, XT>(m, a, n_tiles, Z, st, what);
 }
 template <int MODE>
@@ -1153,8 +1168,7 @@ void fill_tiles(TcArgs& a, const TilesView& tv, const TileSet& s) {
 }  // namespace
 
 // Forward on the tcgen05 path.  Preconditions (checked by the caller): dtype F16 / BF16,
-// D in {64, 128}, block in {64, 128}, no rpe / attention mask, unit stride on D; kpm (optional)
-// is the key-padding mask [Z, L] in the operands' type with 16-byte aligned rows.
+// D a multiple of 8 up to 128, unit stride on D; kpm (optional) is the key-padding mask [Z, L] in the operands' type with 16-byte aligned rows.
 int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse,
                 int dtype, int Z, int H, int L, int D,
                 int64_t q_sz, int64_t q_sh, int64_t q_sr, int64_t k_sz, int64_t k_sh, int64_t k_sr,
@@ -1163,7 +1177,7 @@ int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse
                 const void* kpm, int64_t kpm_sz, int kpm_mul, int causal, const XtHost* xt, cudaStream_t st) {
   TilesView tv;
   if (int rc = decode_tiles(tiles_hdr, tiles, tv)) return rc;
-  if (tv.H != H || tv.nb * tv.block != L) return fail(BSP_ERR_INVALID, "attention tile lists do not fit %d heads of length %d", H, L);
+  if (tv.H != H || tv.nb != (L + tv.block - 1) / tv.block) return fail(BSP_ERR_INVALID, "attention tile lists do not fit %d heads of length %d", H, L);
   CUtensorMap mq, mk, mv;
   if (int rc = make_map(&mq, q, dtype, Z, H, L, D, q_sz, q_sh, q_sr)) return rc;
   if (int rc = make_map(&mk, k, dtype, Z, H, L, D, k_sz, k_sh, k_sr)) return rc;
@@ -1173,7 +1187,7 @@ int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse
   TcArgs a = {};
   if (int rc = xt_maps(m, a, xt, mq, dtype, Z, H, L)) return rc;
   a.out0 = o; a.lse_out = lse; a.o_sz = o_sz; a.o_sh = o_sh; a.o_sr = o_sr;
-  a.H = H; a.L = L; a.scale = scale; a.scale_log2 = scale * kLog2eT;
+  a.H = H; a.L = L; a.d = D; a.scale = scale; a.scale_log2 = scale * kLog2eT;
   a.kpm = kpm; a.kpm_sz = kpm_sz; a.kpm_mul = kpm_mul; a.causal = causal;
   fill_tiles(a, tv, tv.rt);
   return launch_any<FWD>(dtype, D, m, a, H * tv.tiles_per_head, Z, st, "forward");
@@ -1189,7 +1203,7 @@ int attn_bwd_tc(const void* q, const void* k, const void* v, const void* dout, c
                 cudaStream_t st) {
   TilesView tv;
   if (int rc = decode_tiles(tiles_hdr, tiles, tv)) return rc;
-  if (tv.H != H || tv.nb * tv.block != L) return fail(BSP_ERR_INVALID, "attention tile lists do not fit %d heads of length %d", H, L);
+  if (tv.H != H || tv.nb != (L + tv.block - 1) / tv.block) return fail(BSP_ERR_INVALID, "attention tile lists do not fit %d heads of length %d", H, L);
   CUtensorMap mq, mk, mv, md;
   if (int rc = make_map(&mq, q, dtype, Z, H, L, D, q_sz, q_sh, q_sr)) return rc;
   if (int rc = make_map(&mk, k, dtype, Z, H, L, D, k_sz, k_sh, k_sr)) return rc;
@@ -1198,7 +1212,9 @@ int attn_bwd_tc(const void* q, const void* k, const void* v, const void* dout, c
   Maps m;
   TcArgs a = {};
   if (int rc = xt_maps(m, a, xt, mq, dtype, Z, H, L)) return rc;
-  a.lse = lse; a.delta = delta; a.H = H; a.L = L; a.scale = scale; a.scale_log2 = scale * kLog2eT;
+  a.lse = lse; a.delta = delta; a.H = H; a.L = L; a.d = D;
+  a.o_sz = (int64_t)H * L * D; a.o_sh = (int64_t)L * D; a.o_sr = D;       // gradients are contiguous [Z, H, L, D]
+  a.scale = scale; a.scale_log2 = scale * kLog2eT;
   a.kpm = kpm; a.kpm_sz = kpm_sz; a.kpm_mul = kpm_mul; a.causal = causal;
   const int n_tiles = H * tv.tiles_per_head;
   // dK / dV on the caller's stream; dQ beside it on the thread's second stream when both are

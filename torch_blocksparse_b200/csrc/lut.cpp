@@ -540,8 +540,7 @@ int bsp_attn_tiles_build(const int64_t* layout, int H, int nb, int block,
   // blocks 16 and 32 are handled as block 64 on the coarsened layout, with the presence of the
   // 16 x 16 pieces of every position in `sub`
   const int fine_nb = nb, fine_block = block, f = block < 64 ? 64 / block : 1;
-  if (nb % f) return fail(BSP_ERR_UNSUPPORTED, "attention tiles for block %d need a number of blocks per side that is a multiple of %d (got %d)", block, f, nb);
-  if (f > 1) { nb /= f; block = 64; }
+  if (f > 1) { nb = (nb + f - 1) / f; block = 64; }   // (the last position of a side may have pieces past the end: absent)
   const int nt = block == 128 ? nb : (nb + 1) / 2;   // tiles per head
   std::vector<TileLists> rt(H), ct(H);
   parallel_heads(H, [&](int h) {
@@ -557,7 +556,7 @@ int bsp_attn_tiles_build(const int64_t* layout, int H, int nb, int block,
       // 16 bits of a coarse position: piece (a, b) of 16 rows x 16 columns lies in fine block (a * block16, ...)
       auto piece = [&](int i, int j, int a, int b) {   // a, b: groups of 16 inside coarse position (i, j)
         const int fi = (i * 64 + a * 16) / fine_block, fj = (j * 64 + b * 16) / fine_block;
-        return lay[size_t(fi) * fine_nb + fj] != 0 ? 1 : 0;
+        return fi < fine_nb && fj < fine_nb && lay[size_t(fi) * fine_nb + fj] != 0 ? 1 : 0;
       };
       const std::function<int(int, int)> by_row = [&](int i, int j) {   // outer = query block, inner = key block
         int v = 0;

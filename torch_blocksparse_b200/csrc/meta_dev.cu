@@ -475,7 +475,7 @@ __global__ void tiles_coarsen_kernel(const L* __restrict__ lay, int H, int nbf, 
   for (int a = 0; a < 4; ++a)
     for (int b = 0; b < 4; ++b) {
       const int fi = (i * 64 + a * 16) / fine_block, fj = (j * 64 + b * 16) / fine_block;
-      if (hl[(size_t)fi * nbf + fj] != 0) { vr |= 1 << (4 * a + b); vc |= 1 << (4 * b + a); }
+      if (fi < nbf && fj < nbf && hl[(size_t)fi * nbf + fj] != 0) { vr |= 1 << (4 * a + b); vc |= 1 << (4 * b + a); }
     }
   coarse[idx] = vr != 0;
   pr[idx] = (uint16_t)vr;
@@ -533,8 +533,7 @@ extern "C" int64_t bsp_attn_tiles_device_capacity(int H, int nb, int block) {
   int64_t extra = 0;
   if (block < 64) {                                                          // coarsened layout and piece masks
     const int f = 64 / block;
-    if (nb % f) return 0;
-    nb /= f; block = 64;
+    nb = (nb + f - 1) / f; block = 64;
     extra = (5 * (int64_t)H * nb * nb + 3) / 4 + 4;
   }
   const int64_t nt = block == 128 ? nb : (nb + 1) / 2;
@@ -548,8 +547,7 @@ extern "C" int bsp_attn_tiles_build_device(const void* layout, int elem_bytes, i
   if (block != 16 && block != 32 && block != 64 && block != 128)
     return fail(BSP_ERR_UNSUPPORTED, "attention tiles exist for block 16, 32, 64 and 128 (got %d)", block);
   const int fine_block = block, nbf = nb, f = block < 64 ? 64 / block : 1;
-  if (nb % f) return fail(BSP_ERR_UNSUPPORTED, "attention tiles for block %d need a number of blocks per side that is a multiple of %d (got %d)", block, f, nb);
-  if (f > 1) { nb /= f; block = 64; }
+  if (f > 1) { nb = (nb + f - 1) / f; block = 64; }
   if (nb > kTilesMaxNb) return fail(BSP_ERR_UNSUPPORTED, "device tile-list build: at most %d positions of 64 or 128 per side (got %d)", kTilesMaxNb, nb);
   if (elem_bytes != 1 && elem_bytes != 4 && elem_bytes != 8)
     return fail(BSP_ERR_INVALID, "device tile-list build: layout elements of 1, 4 or 8 bytes (got %d)", elem_bytes);

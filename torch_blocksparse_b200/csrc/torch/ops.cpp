@@ -486,7 +486,9 @@ struct AttentionFn : torch::autograd::Function<AttentionFn> {
     if (c->has_am) set_am(m, am = s[at++], L, L);
     m.kpm_mul = c->kpm_mul;
     m.am_mul = c->am_mul;
-    const Tensor dout = rows(grads[0]);
+    Tensor dout = rows(grads[0]);
+    if (D != 64 && D != 128 && ((dout.stride(0) == 0 && Z > 1) || (dout.stride(1) == 0 && H > 1) || dout.stride(2) == 0))
+      dout = dout.contiguous();
     const Tensor dq = at::empty({Z, H, L, D}, q.options()), dk = at::empty({Z, H, L, D}, q.options()),
                  dv = at::empty({Z, H, L, D}, q.options()), delta = at::empty({Z, H, L}, lse.options());
     const AttentionOp& p = *c->p;
@@ -517,7 +519,19 @@ Tensor attention_call(const c10::intrusive_ptr<AttentionOp>& p, const Tensor& q0
                     " does not fit operands of shape ", q0.sizes());
   check_mask_dtypes(rpe, kpm, am, q0.scalar_type());
   const c10::cuda::CUDAGuard guard(q0.device());
-  const Tensor q = rows(q0), k = rows(k0), v = rows(v0);
+  Tensor q = rows(q0), k = rows(k0), v = rows(v0);
+  const int64_t D = q0.size(3);
+  if (D != 64 && D != 128) {
+    // only the kernels that read through tensor maps take these head dimensions: whatever such a map
+    // cannot describe (a broadcast operand, a mask off the 16-byte grid) is copied
+    for (Tensor* t : {&q, &k, &v})
+      if ((t->stride(0) == 0 && Z > 1) || (t->stride(1) == 0 && H > 1) || t->stride(2) == 0) *t = t->contiguous();
+    if (rpe && !(aligned16(*rpe) && rpe->stride(-1) == 1 && rpe->stride(-2) % 8 == 0 && rpe->stride(-2) > 0 &&
+                 rpe->stride(-3) % 8 == 0 && rpe->stride(-3) > 0 && (rpe->dim() < 4 || rpe->stride(0) % 8 == 0)))
+      rpe = rpe->clone(at::MemoryFormat::Contiguous);
+    if (kpm && !(aligned16(*kpm) && kpm->stride(0) % 8 == 0)) kpm = kpm->clone(at::MemoryFormat::Contiguous);
+    if (am && !(aligned16(*am) && am->stride(0) % 8 == 0 && am->stride(0) > 0)) am = am->clone(at::MemoryFormat::Contiguous);
+  }
   Masks m;
   set_rpe(m, rpe, Z, H, L, L);
   set_kpm(m, kpm, Z, L);

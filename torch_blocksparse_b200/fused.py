@@ -19,8 +19,8 @@ from .matmul import _dtype_code, _require_cuda, _stream
 # benchmark to time each kernel inside a full step; None costs nothing.
 PROFILE = None
 
-# Kernel family: 'tc' (tcgen05, tensor memory, TMA; FP16 / BF16, head dimension 64 / 128, layouts
-# for which tile lists exist, operands and masks TMA can describe) or 'mma' (mma.sync).  What 'tc'
+# Kernel family: 'tc' (tcgen05, tensor memory, TMA; FP16 / BF16, operands and masks TMA can
+# describe) or 'mma' (mma.sync, head dimension 64 / 128).  What 'tc'
 # does not cover always runs on 'mma'; the library decides per call.
 PATH = 'tc'
 
@@ -41,7 +41,9 @@ def _timed(name, fn):
 
 
 def fused_supported(q, block):
-    return q.dtype in (torch.float16, torch.bfloat16) and q.size(-1) in (64, 128) and block in (16, 32, 64, 128)
+    D = q.size(-1)
+    return q.dtype in (torch.float16, torch.bfloat16) and block in (16, 32, 64, 128) and \
+        (D in (64, 128) or (PATH == 'tc' and D % 8 == 0 and 0 < D < 128))
 
 
 def _rows(x):
@@ -211,7 +213,7 @@ class GraphedStep:
     def __init__(self, meta, tiles, block, scale, q, k, v, do):
         _require_cuda(q, k, v, do)
         if not fused_supported(q, block):
-            raise NotImplementedError('graphed step: FP16 / BF16 operands with head dimension 64 or 128')
+            raise NotImplementedError('graphed step: FP16 / BF16 operands with a head dimension that is a multiple of 8 up to 128')
         self.q, self.k, self.v, self.do = (_rows(t) for t in (q, k, v, do))
         for a, b in zip((self.q, self.k, self.v, self.do), (q, k, v, do)):
             if a is not b:

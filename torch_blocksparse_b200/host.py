@@ -91,8 +91,8 @@ class HostAttention:
         lists are used); slice_batch: batch entries per pipeline slice; depth: slices in flight."""
         if dtype not in (torch.float16, torch.bfloat16):
             raise ValueError('host pipeline: FP16 or BF16 operands')
-        if head_dim not in (64, 128):
-            raise NotImplementedError('host pipeline: head dimensions 64 and 128')
+        if head_dim % 8 or not 0 < head_dim <= 128:
+            raise NotImplementedError('host pipeline: head dimensions that are multiples of 8 up to 128')
         self.device = torch.device(device)
         if self.device.type != 'cuda':
             raise ValueError('host pipeline: a CUDA device is required')

@@ -312,16 +312,16 @@ def build_attn_tiles_device(layout, block):
 
 def build_attn_tiles(layout, block):
     """Returns the AttnTiles of a square [H, nb, nb] layout (from the process-wide cache when the
-    same content has been seen), or None when the tcgen05 kernels do not cover it (blocks 64 and
-    128, and blocks 16 / 32 whose count per side is a multiple of 4 / 2, are covered)."""
+    same content has been seen), or None when the tcgen05 kernels do not cover it (a layout that is
+    not square)."""
     if layout.dim() != 3:
         raise ValueError('layout must be a [H, Mb, Nb] tensor')
     H, Mb, Nb = layout.shape
-    if Mb != Nb or block not in (16, 32, 64, 128) or (block < 64 and Mb % (64 // block)):
+    if Mb != Nb or block not in (16, 32, 64, 128):
         return None
 
     def build():
-        if layout.is_cuda and Mb // max(1, 64 // block) <= TILES_DEVICE_MAX_BLOCKS:
+        if layout.is_cuda and -(-Mb // max(1, 64 // block)) <= TILES_DEVICE_MAX_BLOCKS:
             return build_attn_tiles_device(layout, block)
         lay, H, Mb_, Nb_ = _layout_i64(layout)
         L = _lib.lib()
