@@ -77,3 +77,18 @@ def test_tile_lists_of_ragged_layouts_device_against_host(block, nb):
     want, got = tables.build_attn_tiles(layout, block), tables.build_attn_tiles_device(layout.cuda(), block)
     assert torch.equal(want.hdr, got.hdr) and torch.equal(want.host, got.host[:want.host.numel()])
     tables.validate_device_buffer(got.on('cuda'), tiles=True)
+
+
+@pytest.mark.parametrize('which', ['none', 'padding', 'causal'])
+@pytest.mark.parametrize('D', [96, 128])
+def test_tiles_of_few_chunks(D, which):
+    """Two groups of warps on alternating chunks: tiles of 1 to 9 chunks of keys (a second group with
+    nothing to do, rings that do and do not wrap), and of queries in the gradients."""
+    Z, H, nb = 2, 2, 17
+    layout = torch.zeros((H, nb, nb), dtype=torch.long)
+    for i in range(nb):
+        layout[0, i, :i // 2 + 1] = 1
+        layout[1, :i // 2 + 1, nb - 1 - i] = 1
+    q, k, v, do = rand_qkv(Z, H, nb * 64, D, torch.float16, seed=D)
+    kw, km, am = masks_of(which, Z, H, nb * 64, torch.float16, seed=5)
+    check(layout, 64, q, k, v, do, True, km, am, **kw)

@@ -27,18 +27,18 @@
 // tensor core then computes the scores of chunk t+1 while the compute warps turn
 // chunk t into P / dS); P / dS are written back (16-bit, packed) over the scores
 // they came from and feed the accumulating products as the A operand straight
-// from tensor memory.  Two threads share a tile row, 32 columns of a chunk each;
-// in the forward each keeps its own running maximum, sum and O accumulator (the
-// two halves of a chunk are two K-slices of the P V product) and the halves are
-// merged when the tile is done.  For block = 64 a 2-bit mask per chunk says
+// from tensor memory.  At head dimension 64 two threads share a tile row, 32 columns
+// of a chunk each; at 128 two groups of warps take alternating chunks.  In the
+// forward each of the two keeps its own running maximum, sum and O accumulator and
+// they are merged when the tile is done.  For block = 64 a 2-bit mask per chunk says
 // which half of the tile owns the block; the other half contributes zeros.
 // Where tensor memory has columns to spare the packed operands get columns of
 // their own, so that the score columns are free again as soon as they have been
 // read (Cfg::ER, Cfg::ER2).
 //
-// Warp roles: eight compute warps and two issuing warps (one thread each): one
-// issues the score products, the other the accumulating products and the TMA
-// loads of the ring of inner chunks.  They talk through mbarriers only (one
+// Warp roles: eight compute warps (sixteen in the backward at 128) and two issuing
+// warps (one lane acts): one issues the score products, the other the accumulating
+// products and (a third warp at 128) the TMA loads of the ring of inner chunks.  They talk through mbarriers only (one
 // arrival per warp); every wait is bounded (tc.cuh) and a wait that expires
 // sets the device status word.
 #include <atomic>
@@ -231,8 +231,20 @@ template <> struct IsBf16<__nv_bfloat16> { static constexpr int v = 1; };
 template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   static constexpr int ATOMS = D / 64;                         // 64-element (128-byte) column groups
   static constexpr int NRES = MODE == FWD ? 1 : 2;             // resident 128-row operands
-  static constexpr int NC = 8;                                 // compute warps: two threads per tile row
-  static constexpr int NT = (NC + 2) * 32;                     // + loader / score issuer, accumulate issuer
+  // Groups of compute warps; group g owns the chunks t with t % G == g.  At head dimension 128 one
+  // CTA fills the SM, and with all its warps on the same chunk every hand-off (score commit, reads of
+  // tensor memory, write of P / dS, accumulation) was waited for by everybody.  Two groups on
+  // alternating chunks fill each other's waits.  At 64 the second CTA of the SM does that.
+  // BigBird, 4 x 16 x 16384 x 128 (us): forward 998 -> 862, dQ 1119 -> 969, dK/dV 1469 -> 1463;
+  // fixed layout, 1 x 16 x 8192 x 128: 152 -> 109, 166 -> 125, 222 -> 193.
+  static constexpr int G = D == 128 ? 2 : 1;
+  // Forward with two groups: a thread owns all 64 columns of its row of the chunk, and the two O
+  // accumulators (running maxima, sums) belong to the groups instead of to the halves of a chunk.
+  static constexpr int NH = (MODE == FWD && G == 2) ? 2 : 1;   // pieces of 32 columns per thread
+  static constexpr int NC = MODE == FWD ? 8 : 8 * G;           // compute warps
+  static constexpr int GW = NC / G;                            // ... of a group
+  static constexpr bool LOADER = G == 2;                       // the ring is refilled by a warp of its own
+  static constexpr int NT = (NC + 2 + (LOADER ? 1 : 0)) * 32;  // + score issuer, accumulate issuer (, loader)
   static constexpr int RES_BYTES = ATOMS * 128 * 128;
   static constexpr int CH_BYTES = ATOMS * 64 * 128;
   // A key-padding mask is a bias per key: per column of the scores in the forward and in dQ
@@ -252,7 +264,7 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   static constexpr bool XT1_PAIR = XT == 1 && D == 64 && MODE != DKV;
   static constexpr int NSTAGE = XT == 2 ? (D == 64 ? (MODE == FWD ? 4 : 3) : 2)
                                 : XT == 1 ? (D == 64 ? (XT1_PAIR ? 2 : 4) : 3)
-                                          : ((MODE != FWD && D == 128) ? 3 : 4);
+                                          : 4;
   static constexpr int SMEM = NRES * RES_BYTES + NSTAGE * STAGE + 1024;
   static constexpr int SCORE_COLS = MODE == FWD ? 64 : 128;    // per buffer: S (and dP)
   // Early release (dQ at head_dim 64): the packed dS operand of the accumulating product gets
@@ -264,16 +276,20 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   // dP^T's columns (a thread's 32 columns of dP^T hold its 16 + 16 packed columns), so S^T's
   // columns are released after the read and only dP^T waits for the accumulation.
   static constexpr bool ER2 = MODE == DKV && D == 64;
+  // Forward with two groups: the packed P of either group has its own 32 columns, so the scores of
+  // chunk t + 2 are computed during the exponentials of chunk t.
+  static constexpr bool ERF = MODE == FWD && G == 2;
   static constexpr int PK_BASE = NBUF * SCORE_COLS;
-  static constexpr int ACC_BASE = PK_BASE + (ER ? 64 : 0);
-  // forward: one O accumulator per half of the key chunk (the two threads of a row keep
-  // independent running maxima); dK/dV: dV and dK
+  static constexpr int ACC_BASE = PK_BASE + (ER || ERF ? 64 : 0);
+  // forward: one O accumulator per half of the key chunk or per group (the two threads of a row
+  // keep independent running maxima); dK/dV: dV and dK
   static constexpr int ACC_COLS = MODE == DQ ? D : 2 * D;
   // Resident operands that are the A side of the score products are copied to tensor memory
   // once per tile where the columns allow it: an MMA whose A comes from shared memory reads
   // 4 KB of A and 2 KB of B per K-step and is bound by that traffic (48 cycles at N = 64
   // instead of 32 with two CTAs issuing).
   static constexpr bool RES_T = (MODE == DQ || MODE == FWD) && D == 128;
+  static constexpr int RES_SHARE = (G == 2 && NRES == 2) ? 2 : 1;
   static constexpr int RES_BASE = ACC_BASE + ACC_COLS;
   static constexpr int RES_COLS = RES_T ? NRES * (D / 2) : 0;
   static constexpr int TMEM = RES_BASE + RES_COLS <= 256 ? 256 : 512;
@@ -311,13 +327,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
                const __grid_constant__ CUtensorMap m_rpe, const __grid_constant__ CUtensorMap m_am, TcArgs a) {
   using C = Cfg<D, MODE, KPM, XT>;
   static_assert(!XT || FINE, "the variants with rpe / attention mask use the masked code path");
-  constexpr int ATOMS = C::ATOMS, ST = C::NSTAGE, NC = C::NC, NBUF = C::NBUF;
+  constexpr int ATOMS = C::ATOMS, ST = C::NSTAGE, NC = C::NC, NBUF = C::NBUF, G = C::G, NH = C::NH;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024 - (saddr(smem_raw) & 1023)) & 1023);
   unsigned char* res = smem;                                   // [NRES][ATOMS][128 rows][128 B]
   unsigned char* stg = res + C::NRES * C::RES_BYTES;           // [ST][ch0 | ch1 | lse, delta]
-  __shared__ uint64_t bar_res, bar_rt, bar_rd, bar_full[ST], bar_s[4], bar_p[4], bar_acc[4], bar_done;
-  __shared__ float xch[2][2][128];                           // forward: (max, sum) of the two halves of every row
+  __shared__ uint64_t bar_res, bar_rt, bar_rd[2], bar_full[ST], bar_s[4], bar_p[4], bar_acc[4], bar_done;
+  __shared__ float xch[2][2][128];                           // forward: (max, sum) of the two accumulators of every row
   __shared__ uint32_t tmem_slot;
   __shared__ int failed[2];
 
@@ -332,14 +348,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
   const int64_t zh = (int64_t)(z * a.H + h) * a.L;
 
   // row of the tile this thread works on (compute warps), its global row and whether it exists
-  const int quarter = warp & 3, chalf = (warp < NC) ? (warp >> 2) : 0;   // chalf: which 32 columns of a chunk
+  // part: which of the threads of this row; grp: the group it belongs to; chalf: which 32 columns of a chunk
+  const int quarter = warp & 3, part = (warp < NC) ? (warp >> 2) : 0;
+  const int grp = G == 1 ? 0 : part / (C::GW / 4), chalf = NH == 2 ? 0 : (part & 1);
   const int trow = quarter * 32 + lane;
   const int mychunk = trow < 64 ? c0 : c1;
   const int64_t grow = (int64_t)(mychunk < 0 ? 0 : mychunk) * 64 + (trow & 63);
   const bool row_ok = mychunk >= 0 && warp < NC && (!FINE || grow < a.L);   // (L is a multiple of 64 unless the blocks are smaller)
 
   if (ntiles == 0) {                                          // nothing in this tile: zeros, as the reference's products give
-    if (row_ok && chalf == 0) {
+    if (row_ok && part == 0) {
       const int64_t at = z * a.o_sz + h * a.o_sh + grow * a.o_sr;
       for (int c = 0; c < a.d; c += 8) {
         *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.out0) + at + c) = make_uint4(0, 0, 0, 0);
@@ -409,11 +427,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
     failed[0] = 0;
     failed[1] = a.wait_budget;
     mbar_init(&bar_rt, NC);
-    mbar_init(&bar_rd, NC);
+    for (int b = 0; b < 2; ++b) mbar_init(&bar_rd[b], C::GW);
     if (C::ER) mbar_init(&bar_p[1], NC);
     if (C::ER2) mbar_init(&bar_s[2], 1);
     for (int b = 0; b < 4; ++b) mbar_init(&bar_acc[b], 1);
-    for (int b = 0; b < NBUF; ++b) { mbar_init(&bar_s[b], 1); mbar_init(&bar_p[b], NC); }
+    for (int b = 0; b < NBUF; ++b) { mbar_init(&bar_s[b], 1); mbar_init(&bar_p[b], C::GW); }
     mbar_init(&bar_done, 1);
     mbar_init_fence();
   }
@@ -516,7 +534,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
             // packed 16-bit operand of K-step ks (16 rows of the chunk): 8 columns inside the
             // 32-column slice of the compute thread that produced it
             const uint32_t pa = ts + (ks >> 1) * 32 + (ks & 1) * 8;
-            if (MODE == FWD) {          // O_half += P_half . V_half: one accumulator per half of the chunk
+            if (C::ERF) {               // O_group += P V
+              const uint32_t pg = tmem + C::PK_BASE + (t & 1) * 32 + ks * 8;
+              if (ks > 0) mma_ts_acc(ta + (t & 1) * D + at * 64, pg, wide(vb1[at * 4 + ks]), idesc_acc);
+              else mma_ts(ta + (t & 1) * D + at * 64, pg, wide(vb1[at * 4 + ks]), idesc_acc, t >= G ? 1u : 0u);
+            } else if (MODE == FWD) {   // O_half += P_half . V_half: one accumulator per half of the chunk
               if (ks & 1) mma_ts_acc(ta + (ks >> 1) * D + at * 64, pa, wide(vb1[at * 4 + ks]), idesc_acc);
               else mma_ts(ta + (ks >> 1) * D + at * 64, pa, wide(vb1[at * 4 + ks]), idesc_acc, later);
             } else if (MODE == DQ) {    // dQ += dS . K
@@ -540,14 +562,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       // Two issuing threads, one per kind of product, each in its own warp: the scores of chunk
       // t only wait for their operands and for the score buffer, the accumulation of chunk t
       // only for the compute warps; neither queues behind the other's barrier.  The accumulate
-      // issuer, which has less to issue, also refills the ring of chunk operands.
+      // issuer, which has less to issue, also refills the ring of chunk operands, except with two
+      // groups, whose operands may be ready back to back: there a third warp does.
       if (warp == NC) {
         bool ok = mbar_wait_warp(C::RES_T ? &bar_rt : &bar_res, 0, fl);
         for (int t = 0; ok && t < ntiles; ++t) {
           prep_scores(t);
           ok = mbar_wait_warp(&bar_full[t % ST], (t / ST) & 1, fl);
           if (C::ER || C::ER2) {
-            if (ok && t >= 1) ok = mbar_wait_warp(&bar_rd, (t - 1) & 1, fl);     // scores of chunk t - 1 are in registers
+            if (ok && t >= 1) ok = mbar_wait_warp(&bar_rd[0], (t - 1) & 1, fl);  // scores of chunk t - 1 are in registers
+          } else if (C::ERF) {
+            if (ok && t >= 2) ok = mbar_wait_warp(&bar_rd[t & 1], ((t - 2) >> 1) & 1, fl);   // ... of chunk t - 2
           } else {
             if (ok && t >= NBUF) ok = mbar_wait_warp(&bar_acc[(t - NBUF) & 3], ((t - NBUF) >> 2) & 1, fl);
           }
@@ -566,13 +591,22 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
           }
           __syncwarp();
         }
+      } else if (C::LOADER && warp == NC + 2) {
+        bool ok = true;
+        for (int t = ST; t < ntiles; ++t) {                   // stage of chunk t - ST: free when that is accumulated
+          const int crow = a.chunk[first + t] * 64;
+          ok = mbar_wait_warp(&bar_acc[(t - ST) & 3], ((t - ST) >> 2) & 1, fl);
+          if (!ok) break;
+          if (me) load_chunk(t, crow);
+          __syncwarp();
+        }
       } else {
         bool ok = true;
         for (int t = 0; ok && t < ntiles; ++t) {
           // first the stage of chunk t - 1 is refilled: its accumulation, issued one iteration
           // ago, completes while the compute warps are still busy with chunk t
           const int tn = t - 1 + ST;
-          if (t >= 1 && tn < ntiles) {
+          if (!C::LOADER && t >= 1 && tn < ntiles) {
             const int crow_n = a.chunk[first + tn] * 64;
             ok = mbar_wait_warp(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
             if (!ok) break;
@@ -602,7 +636,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       if (ok) {
         constexpr int UNITS = D / 16;                            // 16-byte units per thread and operand
 #pragma unroll
-        for (int r = 0; r < C::NRES; ++r) {
+        for (int rr = 0; rr < C::NRES / C::RES_SHARE; ++rr) {
+          const int r = C::RES_SHARE == 2 ? grp : rr, chalf = part & 1;   // (a group copies one operand, if there are as many)
           const unsigned char* row = res + r * C::RES_BYTES + (D == 128 ? chalf * 16384 : 0) + trow * 128;
           uint32_t w[UNITS * 4];
 #pragma unroll
@@ -620,61 +655,89 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       }
     }
     if (MODE == FWD) {
-      // this thread owns 32 of the 64 key columns of its row, with its own running
-      // maximum, sum and O accumulator; the two halves are merged at the end
-      const uint32_t t_acc = tmem + C::ACC_BASE + chalf * D + lane_base;
+      // this thread owns 32 of the 64 key columns of its row, or (two groups) all 64 of every other
+      // chunk, with its own running maximum, sum and O accumulator; the two are merged at the end
+      const uint32_t t_acc = tmem + C::ACC_BASE + part * D + lane_base;
       float m_ref = kNegInfT, l = 0.f;
-      for (int t = 0; ok && t < ntiles; ++t) {
+      for (int t = grp; ok && t < ntiles; t += G) {
         const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS + lane_base + chalf * 32;
-        int pieces = 3;
+        int pieces[NH];
         bool valid, partial = false;
         if constexpr (FINE) {
-          pieces = chunk_pieces(a.mask[first + t], a.sub[first + t], half, trow, chalf);
-          valid = __any_sync(0xffffffffu, pieces != 0);               // per warp: something to compute
-          partial = __any_sync(0xffffffffu, pieces != 3);
+          int all = 3, any = 0;
+#pragma unroll
+          for (int hh = 0; hh < NH; ++hh) {
+            pieces[hh] = chunk_pieces(a.mask[first + t], a.sub[first + t], half, trow, chalf + hh);
+            all &= pieces[hh];
+            any |= pieces[hh];
+          }
+          valid = __any_sync(0xffffffffu, any != 0);                  // per warp: something to compute
+          partial = __any_sync(0xffffffffu, all != 3);
         } else {
           valid = (a.mask[first + t] >> half) & 1;                    // uniform per warp
         }
         ok = mbar_wait_warp(&bar_s[t % NBUF], (t / NBUF) & 1, fl);
         if (!ok) break;
         fence_after();
-        uint32_t sr[32];
-        tmem_ld32(ts, sr);
+        uint32_t sr[NH][32];
+#pragma unroll
+        for (int hh = 0; hh < NH; ++hh) tmem_ld32(ts + hh * 32, sr[hh]);
         tmem_ld_wait();
-        if (partial) mask_pieces(sr, pieces);
-        if (FINE && a.causal) mask_causal<32, false>(sr, a.chunk[first + t] * 64 + chalf * 32, (int)grow);
+        if (C::ERF) {
+          fence_before();
+          warp_arrive(&bar_rd[t & 1], lane);
+        }
+        if constexpr (FINE) {
+#pragma unroll
+          for (int hh = 0; hh < NH; ++hh) {
+            if (partial) mask_pieces(sr[hh], pieces[hh]);
+            if (a.causal) mask_causal<32, false>(sr[hh], a.chunk[first + t] * 64 + (chalf + hh) * 32, (int)grow);
+          }
+        }
         float mt = kNegInfT;
         if (valid) {
           if constexpr (KPM || XT) {                         // scores become s * scale + bias (base 2) in place
-            const unsigned char* bp = stg + (t % ST) * C::STAGE + 2 * C::CH_BYTES + chalf * 64;
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              float b[8];
-              if constexpr (KPM) kpm_terms8<T>(bp + g * 16, a.kpm_mul, b);
-              else {
+            for (int hh = 0; hh < NH; ++hh) {
+              const unsigned char* bp = stg + (t % ST) * C::STAGE + 2 * C::CH_BYTES + (chalf + hh) * 64;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) b[i] = 0.f;
-              }
-              if constexpr (XT) xt_add8<T>(stg + (t % ST) * C::STAGE + C::XT_OFF, a.has_rpe, a.am_mode, half, trow & 63, chalf * 4 + g, b);
+              for (int g = 0; g < 4; ++g) {
+                float b[8];
+                if constexpr (KPM) kpm_terms8<T>(bp + g * 16, a.kpm_mul, b);
+                else {
 #pragma unroll
-              for (int i = 0; i < 8; i += 2) {
-                const float2 y = __ffma2_rn(u2f(sr[8 * g + i], sr[8 * g + i + 1]), f2(a.scale_log2, a.scale_log2), f2(b[i], b[i + 1]));
-                sr[8 * g + i] = __float_as_uint(y.x); sr[8 * g + i + 1] = __float_as_uint(y.y);
+                  for (int i = 0; i < 8; ++i) b[i] = 0.f;
+                }
+                if constexpr (XT) xt_add8<T>(stg + (t % ST) * C::STAGE + C::XT_OFF, a.has_rpe, a.am_mode, half, trow & 63, (chalf + hh) * 4 + g, b);
+#pragma unroll
+                for (int i = 8 * g; i < 8 * g + 8; i += 2) {
+                  const float2 y = __ffma2_rn(u2f(sr[hh][i], sr[hh][i + 1]), f2(a.scale_log2, a.scale_log2), f2(b[i - 8 * g], b[i - 8 * g + 1]));
+                  sr[hh][i] = __float_as_uint(y.x); sr[hh][i + 1] = __float_as_uint(y.y);
+                }
               }
             }
           }
-          mt = max32(sr) * ((KPM || XT) ? 1.f : a.scale_log2);
+#pragma unroll
+          for (int hh = 0; hh < NH; ++hh) mt = fmaxf(mt, max32(sr[hh]) * ((KPM || XT) ? 1.f : a.scale_log2));
         }
+        // the accumulation of this thread's previous chunk, t - G, into its accumulator
+        bool prev = t < G;
+        auto wait_prev = [&]() {
+          if (!prev) {
+            ok = mbar_wait_warp(&bar_acc[(t - G) & 3], ((t - G) >> 2) & 1, fl);
+            fence_after();
+            prev = true;
+          }
+        };
         // the reference maximum is only raised when the row maximum outgrows it by 2^8
         const bool grow_m = mt > m_ref + 8.f;
         if (__any_sync(0xffffffffu, grow_m)) {
           const float m_new = grow_m ? mt : m_ref;
           const float alpha = grow_m ? fast_exp2(m_ref - m_new) : 1.f;      // 0 while m_ref is still -inf
           l *= alpha;
-          if (t > 0) {                                      // the accumulator must be complete up to chunk t-1
-            ok = mbar_wait_warp(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
+          if (t >= G) {                                     // the accumulator must be complete up to that chunk
+            wait_prev();
             if (!ok) break;
-            fence_after();
             for (int c = 0; c < D; c += 16) {               // (16 at a time: the scores stay in registers)
               uint32_t orr[16];
               tmem_ld16(t_acc + c, orr);
@@ -687,39 +750,45 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
           }
           m_ref = m_new;
         }
-        // exponentials in two halves of 16 columns: eight packed registers live at a time
+        if (C::ERF) {                                       // the packed columns are those of chunk t - G
+          wait_prev();
+          if (!ok) break;
+        }
+        const uint32_t tp = C::ERF ? tmem + C::PK_BASE + (t & 1) * 32 + lane_base : ts;
+        // exponentials in passes of 16 columns: eight packed registers live at a time
         if (valid) {
           float2 s2[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
           // (with a mask or absent pieces a row may still have seen -inf only: its reference stays 0 then)
           const float m_use = ((KPM || FINE) && m_ref == kNegInfT) ? 0.f : m_ref;
           const float2 nm2 = f2(-m_use, -m_use), sl2 = f2(a.scale_log2, a.scale_log2);
 #pragma unroll
-          for (int hp = 0; hp < 2; ++hp) {
+          for (int hp = 0; hp < 2 * NH; ++hp) {
             uint32_t ph[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const float2 s01 = u2f(sr[16 * hp + 2 * i], sr[16 * hp + 2 * i + 1]);
+              const float2 s01 = u2f(sr[hp / 2][16 * (hp & 1) + 2 * i], sr[hp / 2][16 * (hp & 1) + 2 * i + 1]);
               const float2 y = (KPM || XT) ? __fadd2_rn(s01, nm2) : __ffma2_rn(s01, sl2, nm2);
               const float2 p = exp2_pair<1>(y);
               s2[i & 1] = __fadd2_rn(s2[i & 1], p);
               ph[i] = pack16<T>(p.x, p.y);
             }
-            tmem_st8(ts + hp * 8, ph);
+            tmem_st8(tp + hp * 8, ph);
           }
           l += (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
         } else {
           uint32_t pz[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) pz[i] = 0u;
-          tmem_st16(ts, pz);
+#pragma unroll
+          for (int hh = 0; hh < NH; ++hh) tmem_st16(tp + hh * 16, pz);
         }
         tmem_st_wait();
         fence_before();
         warp_arrive(&bar_p[t % NBUF], lane);
       }
-      // merge the two halves of every row: O = (O_a 2^(m_a - m) + O_b 2^(m_b - m)) / l
-      xch[chalf][0][trow] = m_ref;
-      xch[chalf][1][trow] = l;
+      // merge the two accumulators of every row: O = (O_a 2^(m_a - m) + O_b 2^(m_b - m)) / l
+      xch[part][0][trow] = m_ref;
+      xch[part][1][trow] = l;
       asm volatile("bar.sync 1, 256;" ::: "memory");          // the eight compute warps, always executed
       if (ok && mbar_wait_warp(&bar_done, 0, fl)) {
         fence_after();
@@ -731,11 +800,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
           const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
           T* orow = reinterpret_cast<T*>(a.out0) + z * a.o_sz + h * a.o_sh + grow * a.o_sr;
           const uint32_t ta = tmem + C::ACC_BASE + lane_base;
-          for (int c = chalf * (D / 2); c < (chalf + 1) * (D / 2); c += 32) {
+          const bool two = G == 1 || ntiles > 1;                // (a single chunk leaves the second group's accumulator unwritten)
+          for (int c = part * (D / 2); c < (part + 1) * (D / 2); c += 32) {
             uint32_t ra[32], rb[32];
             tmem_ld32(ta + c, ra);
             tmem_ld32(ta + D + c, rb);
             tmem_ld_wait();
+            if (!two) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) rb[i] = 0u;
+            }
 #pragma unroll
             for (int i = 0; i < 32; i += 8) {
               float o[8];
@@ -748,7 +822,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
               if (row_ok && c + i < a.d) *reinterpret_cast<uint4*>(orow + c + i) = v;
             }
           }
-          if (chalf == 0 && row_ok) a.lse_out[zh + grow] = lsum > 0.f ? m + log2f(lsum) : kNegInfT;
+          if (part == 0 && row_ok) a.lse_out[zh + grow] = lsum > 0.f ? m + log2f(lsum) : kNegInfT;
         }
       }
     } else {
@@ -760,7 +834,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
           ? kpm_term(static_cast<float>(reinterpret_cast<const T*>(a.kpm)[z * a.kpm_sz + grow]), a.kpm_mul) : 0.f;
       const float my_d = (MODE == DQ && row_ok) ? a.delta[zh + grow] : 0.f;
       const float2 nd2 = f2(-my_d, -my_d), sl2 = f2(a.scale_log2, a.scale_log2);
-      for (int t = 0; ok && t < ntiles; ++t) {
+      for (int t = grp; ok && t < ntiles; t += G) {
         const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS + lane_base + chalf * 32;
         int pieces = 3;
         bool valid, partial = false;
@@ -783,7 +857,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
           tmem_ld32(ts + 64, qr);
           tmem_ld_wait();
           fence_before();
-          warp_arrive(&bar_rd, lane);
+          warp_arrive(&bar_rd[0], lane);
           if (partial) mask_pieces(sr, pieces);
           if (FINE && a.causal) mask_causal<32, false>(sr, a.chunk[first + t] * 64 + chalf * 32, (int)grow);
           if (valid) {
@@ -840,7 +914,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
             tmem_ld32(ts, sr);
             tmem_ld_wait();
             fence_before();
-            warp_arrive(&bar_rd, lane);
+            warp_arrive(&bar_rd[0], lane);
             if (partial) mask_pieces(sr, pieces);
             if (FINE && a.causal) mask_causal<32, true>(sr, a.chunk[first + t] * 64 + chalf * 32, (int)grow);
             const float2 nsl2 = f2(-a.scale_log2, -a.scale_log2);
@@ -867,7 +941,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
             }
           } else {
             fence_before();
-            warp_arrive(&bar_rd, lane);
+            warp_arrive(&bar_rd[0], lane);
 #pragma unroll
             for (int i = 0; i < 32; ++i) pf[i] = 0.f;
           }
@@ -970,18 +1044,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       if (ok && mbar_wait_warp(&bar_done, 0, fl)) {
         fence_after();
         if (mychunk >= 0) {                                   // uniform per warp
-          // the two threads of a row split the D output columns
+          // the threads of a row split the D output columns
+          constexpr int NCOL = D / (NC / 4);
           const uint32_t ta = tmem + C::ACC_BASE + lane_base;
           const int64_t at = z * a.o_sz + h * a.o_sh + grow * a.o_sr;
           T* o0 = reinterpret_cast<T*>(a.out0) + at;
           // (dS is formed without the score scale, which is applied here)
           const float ds_scale = a.scale;
           if (MODE == DQ) {
-            store_acc<T>(o0, ta, chalf * (D / 2), D / 2, a.d, row_ok, ds_scale);
+            store_acc<T>(o0, ta, part * NCOL, NCOL, a.d, row_ok, ds_scale);
           } else {
             T* o1 = reinterpret_cast<T*>(a.out1) + at;
-            store_acc<T>(o1, ta, chalf * (D / 2), D / 2, a.d, row_ok, 1.f);            // dV: accumulator columns [0, D)
-            store_acc<T>(o0, ta + D, chalf * (D / 2), D / 2, a.d, row_ok, ds_scale);    // dK: accumulator columns [D, 2D)
+            store_acc<T>(o1, ta, part * NCOL, NCOL, a.d, row_ok, 1.f);            // dV: accumulator columns [0, D)
+            store_acc<T>(o0, ta + D, part * NCOL, NCOL, a.d, row_ok, ds_scale);    // dK: accumulator columns [D, 2D)
           }
         }
       }
