@@ -235,15 +235,22 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   // CTA fills the SM, and with all its warps on the same chunk every hand-off (score commit, reads of
   // tensor memory, write of P / dS, accumulation) was waited for by everybody.  Two groups on
   // alternating chunks fill each other's waits.  At 64 the second CTA of the SM does that.
-  // BigBird, 4 x 16 x 16384 x 128 (us): forward 998 -> 862, dQ 1119 -> 969, dK/dV 1469 -> 1463;
-  // fixed layout, 1 x 16 x 8192 x 128: 152 -> 109, 166 -> 125, 222 -> 193.
-  static constexpr int G = D == 128 ? 2 : 1;
+  // Fixed layout, 1 x 16 x 8192 x 128 (us): forward 152 -> 109, dQ 166 -> 125, dK/dV 222 -> 193; BigBird,
+  // 4 x 16 x 16384 x 128: 998 -> 862, 1119 -> 969, 1469 -> 1463.
+  // Not with fewer than three stages, of which two are in use at a time (rpe and mask pieces), and not in
+  // the forward with one kind of pieces, which got slower (3 x 12 x 1664, block 16: 74 -> 78 us).
+  static constexpr int G = (D == 128 && (XT == 0 || (XT == 1 && MODE != FWD))) ? 2 : 1;
   // Forward with two groups: a thread owns all 64 columns of its row of the chunk, and the two O
   // accumulators (running maxima, sums) belong to the groups instead of to the halves of a chunk.
   static constexpr int NH = (MODE == FWD && G == 2) ? 2 : 1;   // pieces of 32 columns per thread
   static constexpr int NC = MODE == FWD ? 8 : 8 * G;           // compute warps
   static constexpr int GW = NC / G;                            // ... of a group
   static constexpr bool LOADER = G == 2;                       // the ring is refilled by a warp of its own
+  // With one CTA per SM nothing covers what a tile spends outside its chunks (set-up, first loads,
+  // write-back: about 8 000 cycles, as much as 8 chunks): there a CTA goes on with the tile of a CTA
+  // that has not started yet, whose operands are on their way before the present tile is done (the
+  // same two workloads, us: 113 -> 95, 130 -> 111, 199 -> 200; 973 -> 862, 1065 -> 967, 1705 -> 1585).
+  static constexpr bool PERSIST = G == 2;
   static constexpr int NT = (NC + 2 + (LOADER ? 1 : 0)) * 32;  // + score issuer, accumulate issuer (, loader)
   static constexpr int RES_BYTES = ATOMS * 128 * 128;
   static constexpr int CH_BYTES = ATOMS * 64 * 128;
@@ -260,7 +267,7 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   static constexpr int STAGE = 2 * CH_BYTES + ((MODE == DKV || BIAS || XT) ? 1024 : 0) + XT * 2 * 8192;   // + lse / delta, or the bias, of the chunk
   // score buffers in tensor memory: two (scores of the next chunk are computed while this
   // one is consumed) where the columns allow it with two CTAs per SM, else one
-  static constexpr int NBUF = MODE == FWD ? 2 : (D == 64 ? 1 : 2);
+  static constexpr int NBUF = MODE == FWD || D == 128 ? 2 : G;
   static constexpr bool XT1_PAIR = XT == 1 && D == 64 && MODE != DKV;
   static constexpr int NSTAGE = XT == 2 ? (D == 64 ? (MODE == FWD ? 4 : 3) : 2)
                                 : XT == 1 ? (D == 64 ? (XT1_PAIR ? 2 : 4) : 3)
@@ -275,7 +282,7 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   // dK/dV at head_dim 64 has no spare columns.  There the packed P^T and dS^T both go over
   // dP^T's columns (a thread's 32 columns of dP^T hold its 16 + 16 packed columns), so S^T's
   // columns are released after the read and only dP^T waits for the accumulation.
-  static constexpr bool ER2 = MODE == DKV && D == 64;
+  static constexpr bool ER2 = MODE == DKV && D == 64 && G == 1;
   // Forward with two groups: the packed P of either group has its own 32 columns, so the scores of
   // chunk t + 2 are computed during the exponentials of chunk t.
   static constexpr bool ERF = MODE == FWD && G == 2;
@@ -318,6 +325,15 @@ BSP_DEVI void store_acc(T* dst, uint32_t taddr, int c0, int n, int d, bool row, 
   }
 }
 
+// A tile of work: batch entry, head, its chunks (from `first`, `n` of them) and its two 64-row chunks.
+struct Tile { int z, h, first, n, c0, c1; };
+// One-dimensional grid, batch entries of a tile adjacent: CTAs start in the order of the
+// tiles' lengths (longest first) over the whole launch, not per batch entry.
+BSP_DEVI Tile tile_at(const TcArgs& a, uint32_t block) {
+  const int ti = a.order[block / a.Z];
+  return {(int)(block % a.Z), ti / a.tiles_per_head, a.ptr[ti], a.ptr[ti + 1] - a.ptr[ti], a.c01[2 * ti], a.c01[2 * ti + 1]};
+}
+
 // FINE: the lists come from a layout with blocks smaller than 64 (pieces of a position may be
 // absent); a separate instantiation keeps the other case free of that bookkeeping.
 template <typename T, int D, int MODE, bool KPM, bool FINE, int XT>
@@ -332,31 +348,35 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
   unsigned char* smem = smem_raw + ((1024 - (saddr(smem_raw) & 1023)) & 1023);
   unsigned char* res = smem;                                   // [NRES][ATOMS][128 rows][128 B]
   unsigned char* stg = res + C::NRES * C::RES_BYTES;           // [ST][ch0 | ch1 | lse, delta]
+  __shared__ uint64_t bar_next[2], bar_free[2], bar_clc, bar_x, bar_epi;   // (PERSIST)
+  __shared__ Tile next[2];                                   // (PERSIST) the tiles to come, n < 0: none
+  __shared__ uint4 clc;
   __shared__ uint64_t bar_res, bar_rt, bar_rd[2], bar_full[ST], bar_s[4], bar_p[4], bar_acc[4], bar_done;
   __shared__ float xch[2][2][128];                           // forward: (max, sum) of the two accumulators of every row
   __shared__ uint32_t tmem_slot;
   __shared__ int failed[2];
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
-  // One-dimensional grid, batch entries of a tile adjacent: CTAs start in the order of the
-  // tiles' lengths (longest first) over the whole launch, not per batch entry.
-  const int z = blockIdx.x % a.Z;
-  const int ti = a.order[blockIdx.x / a.Z];
-  const int h = ti / a.tiles_per_head;
-  const int first = a.ptr[ti], ntiles = a.ptr[ti + 1] - first;
-  const int c0 = a.c01[2 * ti], c1 = a.c01[2 * ti + 1];
-  const int64_t zh = (int64_t)(z * a.H + h) * a.L;
+  Tile w = tile_at(a, blockIdx.x);
+  const int &z = w.z, &h = w.h, &first = w.first, &ntiles = w.n, &c0 = w.c0, &c1 = w.c1;
 
   // row of the tile this thread works on (compute warps), its global row and whether it exists
   // part: which of the threads of this row; grp: the group it belongs to; chalf: which 32 columns of a chunk
   const int quarter = warp & 3, part = (warp < NC) ? (warp >> 2) : 0;
   const int grp = G == 1 ? 0 : part / (C::GW / 4), chalf = NH == 2 ? 0 : (part & 1);
   const int trow = quarter * 32 + lane;
-  const int mychunk = trow < 64 ? c0 : c1;
-  const int64_t grow = (int64_t)(mychunk < 0 ? 0 : mychunk) * 64 + (trow & 63);
-  const bool row_ok = mychunk >= 0 && warp < NC && (!FINE || grow < a.L);   // (L is a multiple of 64 unless the blocks are smaller)
+  int mychunk;
+  int64_t zh, grow;
+  bool row_ok;
+  auto use_tile = [&]() {
+    zh = (int64_t)(z * a.H + h) * a.L;
+    mychunk = trow < 64 ? c0 : c1;
+    grow = (int64_t)(mychunk < 0 ? 0 : mychunk) * 64 + (trow & 63);
+    row_ok = mychunk >= 0 && warp < NC && (!FINE || grow < a.L);   // (L is a multiple of 64 unless the blocks are smaller)
+  };
+  use_tile();
 
-  if (ntiles == 0) {                                          // nothing in this tile: zeros, as the reference's products give
+  auto store_zeros = [&]() {                                  // nothing in this tile: zeros, as the reference's products give
     if (row_ok && part == 0) {
       const int64_t at = z * a.o_sz + h * a.o_sh + grow * a.o_sr;
       for (int c = 0; c < a.d; c += 8) {
@@ -365,11 +385,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       }
       if (MODE == FWD) a.lse_out[zh + grow] = kNegInfT;
     }
-    return;
-  }
-  // One chunk of the other operand (and what travels with it) into its stage of the ring.
-  auto load_chunk = [&](int t, int crow) {
-    const int stage = t % ST;
+  };
+  if (!C::PERSIST && ntiles == 0) { store_zeros(); return; }
+  // Chunk t of the tile (and what travels with it) into its stage of the ring; u counts the chunks of
+  // all tiles of this CTA, as everywhere below.
+  auto load_chunk = [&](int t, int u, int crow) {
+    const int stage = u % ST;
     unsigned char* sp = stg + stage * C::STAGE;
     const int nr = FINE ? min(64, a.L - crow) : 64;             // rows of the chunk inside the sequence
     uint32_t bytes = 2 * C::CH_BYTES + (MODE == DKV ? 8 : C::BIAS ? 2 : 0) * nr;
@@ -396,6 +417,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       }
     }
   };
+  auto load_res = [&]() {
+    mbar_expect_tx(&bar_res, C::NRES * C::RES_BYTES);
+    for (int hf = 0; hf < 2; ++hf) {
+      const int crow = (hf == 0 || c1 < 0 ? c0 : c1) * 64;
+      for (int at = 0; at < ATOMS; ++at) {
+        tma_load_4d(res + at * 16384 + hf * 8192, &m_res0, &bar_res, at * 64, crow, h, z);
+        if (C::NRES == 2) tma_load_4d(res + C::RES_BYTES + at * 16384 + hf * 8192, &m_res1, &bar_res, at * 64, crow, h, z);
+      }
+    }
+  };
   // The thread that issues the loads sets up their barriers itself and starts the resident
   // operands and the first chunks at once: their latency overlaps the rest of the set-up
   // (other barriers, tensor-memory allocation, the block-wide synchronisation).
@@ -413,26 +444,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
     mbar_init_fence();
     prefetch_map(&m_res0); prefetch_map(&m_ch0); prefetch_map(&m_ch1);
     if constexpr (XT) { if (a.has_rpe) prefetch_map(&m_rpe); if (a.am_mode) prefetch_map(&m_am); }
-    mbar_expect_tx(&bar_res, C::NRES * C::RES_BYTES);
-    for (int hf = 0; hf < 2; ++hf) {
-      const int crow = (hf == 0 || c1 < 0 ? c0 : c1) * 64;
-      for (int at = 0; at < ATOMS; ++at) {
-        tma_load_4d(res + at * 16384 + hf * 8192, &m_res0, &bar_res, at * 64, crow, h, z);
-        if (C::NRES == 2) tma_load_4d(res + C::RES_BYTES + at * 16384 + hf * 8192, &m_res1, &bar_res, at * 64, crow, h, z);
-      }
-    }
-    for (int t = 0; t < ST && t < ntiles; ++t) load_chunk(t, a.chunk[first + t] * 64);
+    if (ntiles > 0) load_res();
+    for (int t = 0; t < ST && t < ntiles; ++t) load_chunk(t, t, a.chunk[first + t] * 64);
   }
   if (tid == 0) {
     failed[0] = 0;
     failed[1] = a.wait_budget;
-    mbar_init(&bar_rt, NC);
+    mbar_init(&bar_rt, C::RES_T ? NC : 1);
     for (int b = 0; b < 2; ++b) mbar_init(&bar_rd[b], C::GW);
     if (C::ER) mbar_init(&bar_p[1], NC);
     if (C::ER2) mbar_init(&bar_s[2], 1);
     for (int b = 0; b < 4; ++b) mbar_init(&bar_acc[b], 1);
     for (int b = 0; b < NBUF; ++b) { mbar_init(&bar_s[b], 1); mbar_init(&bar_p[b], C::GW); }
     mbar_init(&bar_done, 1);
+    if (C::PERSIST) {
+      for (int b = 0; b < 2; ++b) { mbar_init(&bar_next[b], 1); mbar_init(&bar_free[b], NC + 2); }
+      mbar_init(&bar_clc, 1);
+      mbar_init(&bar_x, NC);
+      mbar_init(&bar_epi, NC);
+    }
     mbar_init_fence();
   }
   if (warp == 1) { tmem_alloc(&tmem_slot, C::TMEM); tmem_relinquish(); }
@@ -441,6 +471,23 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
   fence_after();
   const uint32_t tmem = tmem_slot;
   volatile int* fl = failed;
+  bool ok = true;
+  // (A wait names a phase by its parity, so nobody may wait for a phase that another can overtake: every
+  // barrier's next phase needs something of each of its waiters.)
+  // Every role walks the CTA's tiles i = 0, 1, ...: `base` chunks and `done` tiles with chunks lie
+  // before the present one.  to_tile: tile i from the loader's slot; false when there is none.
+  int base = 0, done = 0;
+  auto to_tile = [&](int i) {
+    if (i == 0) return true;
+    if (!C::PERSIST || !ok) return false;
+    ok = mbar_wait_warp(&bar_next[i & 1], ((i - 1) >> 1) & 1, fl);
+    if (!ok) return false;
+    w = next[i & 1];
+    warp_arrive(&bar_free[i & 1], lane);
+    use_tile();
+    return ntiles >= 0;
+  };
+  auto tile_done = [&]() { base += ntiles; ++done; };
 
   if (warp >= NC) {
     // ------------------------------------------------------------------ loader and MMA issuers
@@ -467,8 +514,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
         if (MODE != FWD) a1[ks] = desc_from_lo(res_lo + C::RES_BYTES / 16 + (ks / 4) * 1024 + (ks % 4) * 2);
       }
       uint64_t sb0[KS], sb1[MODE == FWD ? 1 : KS];          // chunk operands of the scores being prepared
-      auto prep_scores = [&](int t) {
-        const uint32_t sp_lo = stg_lo + (t % ST) * (C::STAGE / 16);
+      auto prep_scores = [&](int u) {
+        const uint32_t sp_lo = stg_lo + (u % ST) * (C::STAGE / 16);
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
           sb0[ks] = desc_from_lo(sp_lo + (ks / 4) * 512 + (ks % 4) * 2);
@@ -476,8 +523,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
         }
       };
       // part: 1 = first product (S), 2 = second (dP), 3 = both, one commit each call
-      auto scores = [&](int t, int part, uint64_t* bar) {
-        const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS;
+      auto scores = [&](int u, int part, uint64_t* bar) {
+        const uint32_t ts = tmem + (u % NBUF) * C::SCORE_COLS;
         if (!me) return;
         if (C::RES_T) {
           const uint32_t tq = tmem + C::RES_BASE;
@@ -506,8 +553,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
         commit(bar);
       };
       uint64_t vb0[ATOMS * 4], vb1[ATOMS * 4];              // chunk operands of the accumulation being prepared
-      auto prep_acc = [&](int t) {
-        const uint32_t sp_lo = stg_lo + (t % ST) * (C::STAGE / 16);
+      auto prep_acc = [&](int u) {
+        const uint32_t sp_lo = stg_lo + (u % ST) * (C::STAGE / 16);
 #pragma unroll
         for (int at = 0; at < ATOMS; ++at)
 #pragma unroll
@@ -522,9 +569,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       constexpr bool WIDE = ATOMS == 2;
       const uint32_t idesc_acc = WIDE ? instr_desc(128, 128, 1, IsBf16<T>::v) : idesc_mn;
       auto wide = [](uint64_t d) { return WIDE ? ((d & ~0x3FFF0000ull) | (512ull << 16)) : d; };
-      auto accumulate = [&](int t) {
+      auto accumulate = [&](int t, int u) {
         if (!me) return;
-        const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS;
+        const uint32_t ts = tmem + (u % NBUF) * C::SCORE_COLS;
         const uint32_t ta = tmem + C::ACC_BASE;
         const uint32_t later = t > 0 ? 1u : 0u;
 #pragma unroll
@@ -535,14 +582,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
             // 32-column slice of the compute thread that produced it
             const uint32_t pa = ts + (ks >> 1) * 32 + (ks & 1) * 8;
             if (C::ERF) {               // O_group += P V
-              const uint32_t pg = tmem + C::PK_BASE + (t & 1) * 32 + ks * 8;
-              if (ks > 0) mma_ts_acc(ta + (t & 1) * D + at * 64, pg, wide(vb1[at * 4 + ks]), idesc_acc);
-              else mma_ts(ta + (t & 1) * D + at * 64, pg, wide(vb1[at * 4 + ks]), idesc_acc, t >= G ? 1u : 0u);
+              const uint32_t pg = tmem + C::PK_BASE + (u & 1) * 32 + ks * 8;
+              if (ks > 0) mma_ts_acc(ta + (u & 1) * D + at * 64, pg, wide(vb1[at * 4 + ks]), idesc_acc);
+              else mma_ts(ta + (u & 1) * D + at * 64, pg, wide(vb1[at * 4 + ks]), idesc_acc, t >= G ? 1u : 0u);
             } else if (MODE == FWD) {   // O_half += P_half . V_half: one accumulator per half of the chunk
               if (ks & 1) mma_ts_acc(ta + (ks >> 1) * D + at * 64, pa, wide(vb1[at * 4 + ks]), idesc_acc);
               else mma_ts(ta + (ks >> 1) * D + at * 64, pa, wide(vb1[at * 4 + ks]), idesc_acc, later);
             } else if (MODE == DQ) {    // dQ += dS . K
-              const uint32_t da = C::ER ? tmem + C::PK_BASE + (t & 1) * 32 + ks * 8 : pa + 64;
+              const uint32_t da = C::ER ? tmem + C::PK_BASE + (u & 1) * 32 + ks * 8 : pa + 64;
               if (ks > 0) mma_ts_acc(ta + at * 64, da, wide(vb0[at * 4 + ks]), idesc_acc);
               else mma_ts(ta + at * 64, da, wide(vb0[at * 4 + ks]), idesc_acc, later);
             } else {                    // dV += P^T . dO,  dK += dS^T . Q
@@ -557,7 +604,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
               }
             }
           }
-        commit(&bar_acc[t & 3]);      // chunk t fully consumed: its score buffer and its stage are free
+        commit(&bar_acc[u & 3]);      // chunk u fully consumed: its score buffer and its stage are free
       };
       // Two issuing threads, one per kind of product, each in its own warp: the scores of chunk
       // t only wait for their operands and for the score buffer, the accumulation of chunk t
@@ -565,501 +612,583 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
       // issuer, which has less to issue, also refills the ring of chunk operands, except with two
       // groups, whose operands may be ready back to back: there a third warp does.
       if (warp == NC) {
-        bool ok = mbar_wait_warp(C::RES_T ? &bar_rt : &bar_res, 0, fl);
-        for (int t = 0; ok && t < ntiles; ++t) {
-          prep_scores(t);
-          ok = mbar_wait_warp(&bar_full[t % ST], (t / ST) & 1, fl);
-          if (C::ER || C::ER2) {
-            if (ok && t >= 1) ok = mbar_wait_warp(&bar_rd[0], (t - 1) & 1, fl);  // scores of chunk t - 1 are in registers
-          } else if (C::ERF) {
-            if (ok && t >= 2) ok = mbar_wait_warp(&bar_rd[t & 1], ((t - 2) >> 1) & 1, fl);   // ... of chunk t - 2
-          } else {
-            if (ok && t >= NBUF) ok = mbar_wait_warp(&bar_acc[(t - NBUF) & 3], ((t - NBUF) >> 2) & 1, fl);
-          }
-          if (!ok) break;
-          fence_after();
-          if (C::ER2) {
-            scores(t, 1, &bar_s[0]);
-            if (t >= 1) {                                   // dP^T's columns still hold the operands of chunk t - 1
-              ok = mbar_wait_warp(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
-              if (!ok) break;
-              fence_after();
+        for (int i = 0; to_tile(i); ++i) {
+          if (ntiles == 0) continue;
+          ok = mbar_wait_warp(C::RES_T ? &bar_rt : &bar_res, done & 1, fl);
+          for (int t = 0; ok && t < ntiles; ++t) {
+            const int u = base + t;
+            prep_scores(u);
+            ok = mbar_wait_warp(&bar_full[u % ST], (u / ST) & 1, fl);
+            if (C::ER || C::ER2) {
+              if (ok && u >= 1) ok = mbar_wait_warp(&bar_rd[0], (u - 1) & 1, fl);  // scores of chunk u - 1 are in registers
+            } else if (C::ERF) {
+              if (ok && u >= 2) ok = mbar_wait_warp(&bar_rd[u & 1], ((u - 2) >> 1) & 1, fl);   // ... of chunk u - 2
+            } else {
+              if (ok && u >= NBUF) ok = mbar_wait_warp(&bar_acc[(u - NBUF) & 3], ((u - NBUF) >> 2) & 1, fl);
             }
-            scores(t, 2, &bar_s[2]);
-          } else {
-            scores(t, 3, &bar_s[t % NBUF]);
-          }
-          __syncwarp();
-        }
-      } else if (C::LOADER && warp == NC + 2) {
-        bool ok = true;
-        for (int t = ST; t < ntiles; ++t) {                   // stage of chunk t - ST: free when that is accumulated
-          const int crow = a.chunk[first + t] * 64;
-          ok = mbar_wait_warp(&bar_acc[(t - ST) & 3], ((t - ST) >> 2) & 1, fl);
-          if (!ok) break;
-          if (me) load_chunk(t, crow);
-          __syncwarp();
-        }
-      } else {
-        bool ok = true;
-        for (int t = 0; ok && t < ntiles; ++t) {
-          // first the stage of chunk t - 1 is refilled: its accumulation, issued one iteration
-          // ago, completes while the compute warps are still busy with chunk t
-          const int tn = t - 1 + ST;
-          if (!C::LOADER && t >= 1 && tn < ntiles) {
-            const int crow_n = a.chunk[first + tn] * 64;
-            ok = mbar_wait_warp(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
             if (!ok) break;
-            if (me) load_chunk(tn, crow_n);
+            fence_after();
+            if (C::ER2) {
+              scores(u, 1, &bar_s[0]);
+              if (u >= 1) {                                   // dP^T's columns still hold the operands of chunk u - 1
+                ok = mbar_wait_warp(&bar_acc[(u - 1) & 3], ((u - 1) >> 2) & 1, fl);
+                if (!ok) break;
+                fence_after();
+              }
+              scores(u, 2, &bar_s[2]);
+            } else {
+              scores(u, 3, &bar_s[u % NBUF]);
+            }
             __syncwarp();
           }
-          prep_acc(t);
-          ok = mbar_wait_warp(&bar_full[t % ST], (t / ST) & 1, fl) &&
-               (C::ER ? mbar_wait_warp(&bar_p[t & 1], (t >> 1) & 1, fl) : mbar_wait_warp(&bar_p[t % NBUF], (t / NBUF) & 1, fl));
           if (!ok) break;
-          fence_after();
-          accumulate(t);
+          if (C::PERSIST && !C::RES_T && me) commit(&bar_rt);   // (the last scores of the tile: its resident operands are free)
           __syncwarp();
+          tile_done();
         }
-        if (ok && me) commit(&bar_done);
+      } else if (C::LOADER && warp == NC + 2) {
+        // Loads the tiles' operands as far ahead as the buffers allow and hands the tiles out.
+        bool asked = true;
+        int i = 0;
+        if (me) clc_ask(&clc, &bar_clc);
+        for (;; ++i) {
+          if (i > 0 && ntiles > 0) {
+            if (done > 0) ok = mbar_wait_warp(&bar_rt, (done - 1) & 1, fl);   // the resident operands of the tile before are no longer read
+            if (ok && me) load_res();
+            __syncwarp();
+          }
+          for (int t = i == 0 ? ST : 0; ok && t < ntiles; ++t) {
+            const int u = base + t, crow = a.chunk[first + t] * 64;
+            if (u >= ST) ok = mbar_wait_warp(&bar_acc[(u - ST) & 3], ((u - ST) >> 2) & 1, fl);   // its stage is free
+            if (!ok) break;
+            if (FINE && (MODE == DKV || C::BIAS) && crow + 64 > a.L) {
+              // (the last chunk of a sequence fills only part of these: no values of other sequences in the rest)
+              unsigned char* vp = stg + (u % ST) * C::STAGE + 2 * C::CH_BYTES;
+              for (int c = a.L - crow + lane; c < 64; c += 32) {
+                if (MODE == DKV) { reinterpret_cast<float*>(vp)[c] = 0.f; reinterpret_cast<float*>(vp + 256)[c] = 0.f; }
+                else reinterpret_cast<uint16_t*>(vp)[c] = 0;
+              }
+              __syncwarp();
+            }
+            if (me) load_chunk(t, u, crow);
+            __syncwarp();
+          }
+          if (!ok) break;
+          if (ntiles > 0) tile_done();
+          ok = mbar_wait_warp(&bar_clc, i & 1, fl);
+          if (!ok) break;
+          asked = false;
+          uint32_t block;
+          const bool more = clc_answer(&clc, &block);
+          fence_async_smem();
+          if (more) w = tile_at(a, block); else w.n = -1;
+          use_tile();
+          if (i >= 2) ok = mbar_wait_warp(&bar_free[(i + 1) & 1], ((i - 2) >> 1) & 1, fl);   // tile i - 1 has been read
+          if (!ok) break;
+          if (me) {
+            next[(i + 1) & 1] = w;
+            mbar_arrive(&bar_next[(i + 1) & 1]);
+          }
+          __syncwarp();
+          if (!more) break;
+          if (me) clc_ask(&clc, &bar_clc);
+          asked = true;
+        }
+        if (asked) {                                          // (given up: the answer still writes into this CTA's memory)
+          for (int n = 0; n < kWaitBudget && !mbar_try_wait(&bar_clc, i & 1); ++n) {}
+        }
+      } else {
+        for (int i = 0; to_tile(i); ++i) {
+          if (ntiles == 0) continue;
+          for (int t = 0; ok && t < ntiles; ++t) {
+            const int u = base + t;
+            // first the stage of chunk t - 1 is refilled: its accumulation, issued one iteration
+            // ago, completes while the compute warps are still busy with chunk t
+            const int tn = t - 1 + ST;
+            if (!C::LOADER && t >= 1 && tn < ntiles) {
+              const int crow_n = a.chunk[first + tn] * 64;
+              ok = mbar_wait_warp(&bar_acc[(t - 1) & 3], ((t - 1) >> 2) & 1, fl);
+              if (!ok) break;
+              if (me) load_chunk(tn, tn, crow_n);
+              __syncwarp();
+            }
+            prep_acc(u);
+            ok = mbar_wait_warp(&bar_full[u % ST], (u / ST) & 1, fl) &&
+                 (C::ER ? mbar_wait_warp(&bar_p[u & 1], (u >> 1) & 1, fl) : mbar_wait_warp(&bar_p[u % NBUF], (u / NBUF) & 1, fl));
+            if (ok && t == 0 && done > 0) ok = mbar_wait_warp(&bar_epi, (done - 1) & 1, fl);   // the accumulators of the tile before are read
+            if (!ok) break;
+            fence_after();
+            accumulate(t, u);
+            __syncwarp();
+          }
+          if (!ok) break;
+          if (me) commit(&bar_done);
+          tile_done();
+        }
       }
     }
   } else {
     // ------------------------------------------------------------------ compute warps
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int half = trow >> 6;                               // which 64-row chunk of the tile
-    bool ok = true;
-    if (C::RES_T) {
-      // this thread's share of its row of the resident operands: shared memory (128-byte
-      // rows, 16-byte units swizzled by the row) -> tensor memory, two 16-bit values per column
-      ok = mbar_wait_warp(&bar_res, 0, fl);
-      if (ok) {
-        constexpr int UNITS = D / 16;                            // 16-byte units per thread and operand
+    for (int i = 0; to_tile(i); ++i) {
+      if (C::PERSIST && ntiles == 0) { store_zeros(); continue; }
+      if (C::RES_T) {
+        // this thread's share of its row of the resident operands: shared memory (128-byte
+        // rows, 16-byte units swizzled by the row) -> tensor memory, two 16-bit values per column
+        ok = mbar_wait_warp(&bar_res, done & 1, fl);
+        if (ok) {
+          constexpr int UNITS = D / 16;                            // 16-byte units per thread and operand
 #pragma unroll
-        for (int rr = 0; rr < C::NRES / C::RES_SHARE; ++rr) {
-          const int r = C::RES_SHARE == 2 ? grp : rr, chalf = part & 1;   // (a group copies one operand, if there are as many)
-          const unsigned char* row = res + r * C::RES_BYTES + (D == 128 ? chalf * 16384 : 0) + trow * 128;
-          uint32_t w[UNITS * 4];
+          for (int rr = 0; rr < C::NRES / C::RES_SHARE; ++rr) {
+            const int r = C::RES_SHARE == 2 ? grp : rr, chalf = part & 1;   // (a group copies one operand, if there are as many)
+            const unsigned char* row = res + r * C::RES_BYTES + (D == 128 ? chalf * 16384 : 0) + trow * 128;
+            uint32_t w[UNITS * 4];
 #pragma unroll
-          for (int u = 0; u < UNITS; ++u) {
-            const int unit = (D == 128 ? u : chalf * UNITS + u) ^ (trow & 7);
-            const uint4 v = *reinterpret_cast<const uint4*>(row + unit * 16);
-            w[4 * u] = v.x; w[4 * u + 1] = v.y; w[4 * u + 2] = v.z; w[4 * u + 3] = v.w;
-          }
-          const uint32_t tq = tmem + C::RES_BASE + r * (D / 2) + chalf * (D / 4) + lane_base;
-          if constexpr (D == 128) tmem_st32(tq, w); else tmem_st16(tq, w);
-        }
-        tmem_st_wait();
-        fence_before();
-        warp_arrive(&bar_rt, lane);
-      }
-    }
-    if (MODE == FWD) {
-      // this thread owns 32 of the 64 key columns of its row, or (two groups) all 64 of every other
-      // chunk, with its own running maximum, sum and O accumulator; the two are merged at the end
-      const uint32_t t_acc = tmem + C::ACC_BASE + part * D + lane_base;
-      float m_ref = kNegInfT, l = 0.f;
-      for (int t = grp; ok && t < ntiles; t += G) {
-        const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS + lane_base + chalf * 32;
-        int pieces[NH];
-        bool valid, partial = false;
-        if constexpr (FINE) {
-          int all = 3, any = 0;
-#pragma unroll
-          for (int hh = 0; hh < NH; ++hh) {
-            pieces[hh] = chunk_pieces(a.mask[first + t], a.sub[first + t], half, trow, chalf + hh);
-            all &= pieces[hh];
-            any |= pieces[hh];
-          }
-          valid = __any_sync(0xffffffffu, any != 0);                  // per warp: something to compute
-          partial = __any_sync(0xffffffffu, all != 3);
-        } else {
-          valid = (a.mask[first + t] >> half) & 1;                    // uniform per warp
-        }
-        ok = mbar_wait_warp(&bar_s[t % NBUF], (t / NBUF) & 1, fl);
-        if (!ok) break;
-        fence_after();
-        uint32_t sr[NH][32];
-#pragma unroll
-        for (int hh = 0; hh < NH; ++hh) tmem_ld32(ts + hh * 32, sr[hh]);
-        tmem_ld_wait();
-        if (C::ERF) {
-          fence_before();
-          warp_arrive(&bar_rd[t & 1], lane);
-        }
-        if constexpr (FINE) {
-#pragma unroll
-          for (int hh = 0; hh < NH; ++hh) {
-            if (partial) mask_pieces(sr[hh], pieces[hh]);
-            if (a.causal) mask_causal<32, false>(sr[hh], a.chunk[first + t] * 64 + (chalf + hh) * 32, (int)grow);
-          }
-        }
-        float mt = kNegInfT;
-        if (valid) {
-          if constexpr (KPM || XT) {                         // scores become s * scale + bias (base 2) in place
-#pragma unroll
-            for (int hh = 0; hh < NH; ++hh) {
-              const unsigned char* bp = stg + (t % ST) * C::STAGE + 2 * C::CH_BYTES + (chalf + hh) * 64;
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                float b[8];
-                if constexpr (KPM) kpm_terms8<T>(bp + g * 16, a.kpm_mul, b);
-                else {
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) b[i] = 0.f;
-                }
-                if constexpr (XT) xt_add8<T>(stg + (t % ST) * C::STAGE + C::XT_OFF, a.has_rpe, a.am_mode, half, trow & 63, (chalf + hh) * 4 + g, b);
-#pragma unroll
-                for (int i = 8 * g; i < 8 * g + 8; i += 2) {
-                  const float2 y = __ffma2_rn(u2f(sr[hh][i], sr[hh][i + 1]), f2(a.scale_log2, a.scale_log2), f2(b[i - 8 * g], b[i - 8 * g + 1]));
-                  sr[hh][i] = __float_as_uint(y.x); sr[hh][i + 1] = __float_as_uint(y.y);
-                }
-              }
+            for (int u = 0; u < UNITS; ++u) {
+              const int unit = (D == 128 ? u : chalf * UNITS + u) ^ (trow & 7);
+              const uint4 v = *reinterpret_cast<const uint4*>(row + unit * 16);
+              w[4 * u] = v.x; w[4 * u + 1] = v.y; w[4 * u + 2] = v.z; w[4 * u + 3] = v.w;
             }
+            const uint32_t tq = tmem + C::RES_BASE + r * (D / 2) + chalf * (D / 4) + lane_base;
+            if constexpr (D == 128) tmem_st32(tq, w); else tmem_st16(tq, w);
           }
-#pragma unroll
-          for (int hh = 0; hh < NH; ++hh) mt = fmaxf(mt, max32(sr[hh]) * ((KPM || XT) ? 1.f : a.scale_log2));
-        }
-        // the accumulation of this thread's previous chunk, t - G, into its accumulator
-        bool prev = t < G;
-        auto wait_prev = [&]() {
-          if (!prev) {
-            ok = mbar_wait_warp(&bar_acc[(t - G) & 3], ((t - G) >> 2) & 1, fl);
-            fence_after();
-            prev = true;
-          }
-        };
-        // the reference maximum is only raised when the row maximum outgrows it by 2^8
-        const bool grow_m = mt > m_ref + 8.f;
-        if (__any_sync(0xffffffffu, grow_m)) {
-          const float m_new = grow_m ? mt : m_ref;
-          const float alpha = grow_m ? fast_exp2(m_ref - m_new) : 1.f;      // 0 while m_ref is still -inf
-          l *= alpha;
-          if (t >= G) {                                     // the accumulator must be complete up to that chunk
-            wait_prev();
-            if (!ok) break;
-            for (int c = 0; c < D; c += 16) {               // (16 at a time: the scores stay in registers)
-              uint32_t orr[16];
-              tmem_ld16(t_acc + c, orr);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 16; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
-              tmem_st16(t_acc + c, orr);
-            }
-            tmem_st_wait();
-          }
-          m_ref = m_new;
-        }
-        if (C::ERF) {                                       // the packed columns are those of chunk t - G
-          wait_prev();
-          if (!ok) break;
-        }
-        const uint32_t tp = C::ERF ? tmem + C::PK_BASE + (t & 1) * 32 + lane_base : ts;
-        // exponentials in passes of 16 columns: eight packed registers live at a time
-        if (valid) {
-          float2 s2[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
-          // (with a mask or absent pieces a row may still have seen -inf only: its reference stays 0 then)
-          const float m_use = ((KPM || FINE) && m_ref == kNegInfT) ? 0.f : m_ref;
-          const float2 nm2 = f2(-m_use, -m_use), sl2 = f2(a.scale_log2, a.scale_log2);
-#pragma unroll
-          for (int hp = 0; hp < 2 * NH; ++hp) {
-            uint32_t ph[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const float2 s01 = u2f(sr[hp / 2][16 * (hp & 1) + 2 * i], sr[hp / 2][16 * (hp & 1) + 2 * i + 1]);
-              const float2 y = (KPM || XT) ? __fadd2_rn(s01, nm2) : __ffma2_rn(s01, sl2, nm2);
-              const float2 p = exp2_pair<1>(y);
-              s2[i & 1] = __fadd2_rn(s2[i & 1], p);
-              ph[i] = pack16<T>(p.x, p.y);
-            }
-            tmem_st8(tp + hp * 8, ph);
-          }
-          l += (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
-        } else {
-          uint32_t pz[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) pz[i] = 0u;
-#pragma unroll
-          for (int hh = 0; hh < NH; ++hh) tmem_st16(tp + hh * 16, pz);
-        }
-        tmem_st_wait();
-        fence_before();
-        warp_arrive(&bar_p[t % NBUF], lane);
-      }
-      // merge the two accumulators of every row: O = (O_a 2^(m_a - m) + O_b 2^(m_b - m)) / l
-      xch[part][0][trow] = m_ref;
-      xch[part][1][trow] = l;
-      asm volatile("bar.sync 1, 256;" ::: "memory");          // the eight compute warps, always executed
-      if (ok && mbar_wait_warp(&bar_done, 0, fl)) {
-        fence_after();
-        if (mychunk >= 0) {                                   // uniform per warp: a warp lies inside one chunk
-          const float ma = xch[0][0][trow], mb = xch[1][0][trow], la = xch[0][1][trow], lb = xch[1][1][trow];
-          const float m = fmaxf(ma, mb);
-          const float wa = ma == kNegInfT ? 0.f : fast_exp2(ma - m), wb = mb == kNegInfT ? 0.f : fast_exp2(mb - m);
-          const float lsum = la * wa + lb * wb;
-          const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
-          T* orow = reinterpret_cast<T*>(a.out0) + z * a.o_sz + h * a.o_sh + grow * a.o_sr;
-          const uint32_t ta = tmem + C::ACC_BASE + lane_base;
-          const bool two = G == 1 || ntiles > 1;                // (a single chunk leaves the second group's accumulator unwritten)
-          for (int c = part * (D / 2); c < (part + 1) * (D / 2); c += 32) {
-            uint32_t ra[32], rb[32];
-            tmem_ld32(ta + c, ra);
-            tmem_ld32(ta + D + c, rb);
-            tmem_ld_wait();
-            if (!two) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) rb[i] = 0u;
-            }
-#pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              float o[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                o[j] = (__uint_as_float(ra[i + j]) * wa + __uint_as_float(rb[i + j]) * wb) * inv;
-              uint4 v;
-              v.x = pack16<T>(o[0], o[1]); v.y = pack16<T>(o[2], o[3]);
-              v.z = pack16<T>(o[4], o[5]); v.w = pack16<T>(o[6], o[7]);
-              if (row_ok && c + i < a.d) *reinterpret_cast<uint4*>(orow + c + i) = v;
-            }
-          }
-          if (part == 0 && row_ok) a.lse_out[zh + grow] = lsum > 0.f ? m + log2f(lsum) : kNegInfT;
-        }
-      }
-    } else {
-      // (a fully masked query row has lse = -inf: +inf makes its probabilities 0, not NaN)
-      float my_lse = (MODE == DQ && row_ok) ? a.lse[zh + grow] : 0.f;
-      if ((KPM || FINE) && my_lse == kNegInfT) my_lse = -kNegInfT;
-      // dK/dV: the bias of this thread's key row
-      const float my_b = (KPM && MODE == DKV && row_ok)
-          ? kpm_term(static_cast<float>(reinterpret_cast<const T*>(a.kpm)[z * a.kpm_sz + grow]), a.kpm_mul) : 0.f;
-      const float my_d = (MODE == DQ && row_ok) ? a.delta[zh + grow] : 0.f;
-      const float2 nd2 = f2(-my_d, -my_d), sl2 = f2(a.scale_log2, a.scale_log2);
-      for (int t = grp; ok && t < ntiles; t += G) {
-        const uint32_t ts = tmem + (t % NBUF) * C::SCORE_COLS + lane_base + chalf * 32;
-        int pieces = 3;
-        bool valid, partial = false;
-        if constexpr (FINE) {
-          pieces = chunk_pieces(a.mask[first + t], a.sub[first + t], half, trow, chalf);
-          valid = __any_sync(0xffffffffu, pieces != 0);               // per warp: something to compute
-          partial = __any_sync(0xffffffffu, pieces != 3);
-        } else {
-          valid = (a.mask[first + t] >> half) & 1;                    // uniform per warp
-        }
-        const float4* vec = reinterpret_cast<const float4*>(stg + (t % ST) * C::STAGE + 2 * C::CH_BYTES) + chalf * 8;
-        ok = mbar_wait_warp(&bar_s[t % NBUF], (t / NBUF) & 1, fl);
-        if (!ok) break;
-        fence_after();
-        if constexpr (C::ER) {
-          // S and dP of this thread's 32 columns go to registers at once; the score buffer is
-          // then handed back, and the next scores are computed during the arithmetic below
-          uint32_t sr[32], qr[32], dr[16];
-          tmem_ld32(ts, sr);
-          tmem_ld32(ts + 64, qr);
-          tmem_ld_wait();
-          fence_before();
-          warp_arrive(&bar_rd[0], lane);
-          if (partial) mask_pieces(sr, pieces);
-          if (FINE && a.causal) mask_causal<32, false>(sr, a.chunk[first + t] * 64 + chalf * 32, (int)grow);
-          if (valid) {
-            const unsigned char* bp = stg + (t % ST) * C::STAGE + 2 * C::CH_BYTES + chalf * 64;
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              float b[8];
-              if constexpr (KPM || XT) {
-                if constexpr (KPM) kpm_terms8<T>(bp + g * 16, a.kpm_mul, b);
-                else {
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) b[i] = 0.f;
-                }
-                if constexpr (XT) xt_add8<T>(stg + (t % ST) * C::STAGE + C::XT_OFF, a.has_rpe, a.am_mode, half, trow & 63, chalf * 4 + g, b);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) b[i] -= my_lse;
-              } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) b[i] = -my_lse;
-              }
-#pragma unroll
-              for (int i = 8 * g; i < 8 * g + 8; i += 2) {
-                const float2 y = __ffma2_rn(u2f(sr[i], sr[i + 1]), sl2, f2(b[i - 8 * g], b[i + 1 - 8 * g]));
-                const float2 p = exp2_pair<1>(y);
-                const float2 d = __fmul2_rn(p, __fadd2_rn(u2f(qr[i], qr[i + 1]), nd2));   // P (dP - delta); the scale is applied to dQ
-                dr[i / 2] = pack16<T>(d.x, d.y);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) dr[i] = 0u;
-          }
-          if (t >= 2) {                                     // the accumulation of chunk t - 2 has read its operand
-            ok = mbar_wait_warp(&bar_acc[(t - 2) & 3], ((t - 2) >> 2) & 1, fl);
-            if (!ok) break;
-            fence_after();
-          }
-          tmem_st16(tmem + C::PK_BASE + (t & 1) * 32 + chalf * 16 + lane_base, dr);
           tmem_st_wait();
           fence_before();
-          warp_arrive(&bar_p[t & 1], lane);
-          continue;
+          warp_arrive(&bar_rt, lane);
         }
-        if constexpr (C::ER2) {
-          // First all of S^T: read, handed back, exponentials, P^T packed to 16 bits; this runs
-          // while dP^T is still being computed.  Then dP^T in two passes of 16 columns; pass
-          // hv leaves its part of the packed P^T in columns [16 hv, 16 hv + 8) and its packed
-          // dS^T in the next 8 columns of this thread's 32 columns of dP^T, all read before.
-          // dS is formed with P as the accumulating product sees it (rounded to 16 bits),
-          // which is also how a stored softmax output would enter the product.
-          float pf[32];                                        // P^T of this thread's 32 columns
+      }
+      const int t0 = G == 1 ? 0 : grp ^ (base & 1);           // this group's first chunk of the tile
+      if (MODE == FWD) {
+        // this thread owns 32 of the 64 key columns of its row, or (two groups) all 64 of every other
+        // chunk, with its own running maximum, sum and O accumulator; the two are merged at the end
+        const uint32_t t_acc = tmem + C::ACC_BASE + part * D + lane_base;
+        float m_ref = kNegInfT, l = 0.f;
+        for (int t = t0; ok && t < ntiles; t += G) {
+          const int u = base + t;
+          const uint32_t ts = tmem + (u % NBUF) * C::SCORE_COLS + lane_base + chalf * 32;
+          int pieces[NH];
+          bool valid, partial = false;
+          if constexpr (FINE) {
+            int all = 3, any = 0;
+#pragma unroll
+            for (int hh = 0; hh < NH; ++hh) {
+              pieces[hh] = chunk_pieces(a.mask[first + t], a.sub[first + t], half, trow, chalf + hh);
+              all &= pieces[hh];
+              any |= pieces[hh];
+            }
+            valid = __any_sync(0xffffffffu, any != 0);                  // per warp: something to compute
+            partial = __any_sync(0xffffffffu, all != 3);
+          } else {
+            valid = (a.mask[first + t] >> half) & 1;                    // uniform per warp
+          }
+          ok = mbar_wait_warp(&bar_s[u % NBUF], (u / NBUF) & 1, fl);
+          if (!ok) break;
+          fence_after();
+          uint32_t sr[NH][32];
+#pragma unroll
+          for (int hh = 0; hh < NH; ++hh) tmem_ld32(ts + hh * 32, sr[hh]);
+          tmem_ld_wait();
+          if (C::ERF) {
+            fence_before();
+            warp_arrive(&bar_rd[u & 1], lane);
+          }
+          if constexpr (FINE) {
+#pragma unroll
+            for (int hh = 0; hh < NH; ++hh) {
+              if (partial) mask_pieces(sr[hh], pieces[hh]);
+              if (a.causal) mask_causal<32, false>(sr[hh], a.chunk[first + t] * 64 + (chalf + hh) * 32, (int)grow);
+            }
+          }
+          float mt = kNegInfT;
           if (valid) {
-            uint32_t sr[32];
+            if constexpr (KPM || XT) {                         // scores become s * scale + bias (base 2) in place
+#pragma unroll
+              for (int hh = 0; hh < NH; ++hh) {
+                const unsigned char* bp = stg + (u % ST) * C::STAGE + 2 * C::CH_BYTES + (chalf + hh) * 64;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                  float b[8];
+                  if constexpr (KPM) kpm_terms8<T>(bp + g * 16, a.kpm_mul, b);
+                  else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) b[i] = 0.f;
+                  }
+                  if constexpr (XT) xt_add8<T>(stg + (u % ST) * C::STAGE + C::XT_OFF, a.has_rpe, a.am_mode, half, trow & 63, (chalf + hh) * 4 + g, b);
+#pragma unroll
+                  for (int i = 8 * g; i < 8 * g + 8; i += 2) {
+                    const float2 y = __ffma2_rn(u2f(sr[hh][i], sr[hh][i + 1]), f2(a.scale_log2, a.scale_log2), f2(b[i - 8 * g], b[i - 8 * g + 1]));
+                    sr[hh][i] = __float_as_uint(y.x); sr[hh][i + 1] = __float_as_uint(y.y);
+                  }
+                }
+              }
+            }
+#pragma unroll
+            for (int hh = 0; hh < NH; ++hh) mt = fmaxf(mt, max32(sr[hh]) * ((KPM || XT) ? 1.f : a.scale_log2));
+          }
+          // the accumulation of this thread's previous chunk, t - G, into its accumulator
+          bool prev = t < G;
+          auto wait_prev = [&]() {
+            if (!prev) {
+              ok = mbar_wait_warp(&bar_acc[(u - G) & 3], ((u - G) >> 2) & 1, fl);
+              fence_after();
+              prev = true;
+            }
+          };
+          // the reference maximum is only raised when the row maximum outgrows it by 2^8
+          const bool grow_m = mt > m_ref + 8.f;
+          if (__any_sync(0xffffffffu, grow_m)) {
+            const float m_new = grow_m ? mt : m_ref;
+            const float alpha = grow_m ? fast_exp2(m_ref - m_new) : 1.f;      // 0 while m_ref is still -inf
+            l *= alpha;
+            if (t >= G) {                                     // the accumulator must be complete up to that chunk
+              wait_prev();
+              if (!ok) break;
+              for (int c = 0; c < D; c += 16) {               // (16 at a time: the scores stay in registers)
+                uint32_t orr[16];
+                tmem_ld16(t_acc + c, orr);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
+                tmem_st16(t_acc + c, orr);
+              }
+              tmem_st_wait();
+            }
+            m_ref = m_new;
+          }
+          if (C::ERF) {                                       // the packed columns are those of chunk t - G
+            wait_prev();
+            if (!ok) break;
+          }
+          const uint32_t tp = C::ERF ? tmem + C::PK_BASE + (u & 1) * 32 + lane_base : ts;
+          // exponentials in passes of 16 columns: eight packed registers live at a time
+          if (valid) {
+            float2 s2[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
+            // (with a mask or absent pieces a row may still have seen -inf only: its reference stays 0 then)
+            const float m_use = ((KPM || FINE) && m_ref == kNegInfT) ? 0.f : m_ref;
+            const float2 nm2 = f2(-m_use, -m_use), sl2 = f2(a.scale_log2, a.scale_log2);
+#pragma unroll
+            for (int hp = 0; hp < 2 * NH; ++hp) {
+              uint32_t ph[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float2 s01 = u2f(sr[hp / 2][16 * (hp & 1) + 2 * i], sr[hp / 2][16 * (hp & 1) + 2 * i + 1]);
+                const float2 y = (KPM || XT) ? __fadd2_rn(s01, nm2) : __ffma2_rn(s01, sl2, nm2);
+                const float2 p = exp2_pair<1>(y);
+                s2[i & 1] = __fadd2_rn(s2[i & 1], p);
+                ph[i] = pack16<T>(p.x, p.y);
+              }
+              tmem_st8(tp + hp * 8, ph);
+            }
+            l += (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
+          } else {
+            uint32_t pz[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pz[i] = 0u;
+#pragma unroll
+            for (int hh = 0; hh < NH; ++hh) tmem_st16(tp + hh * 16, pz);
+          }
+          tmem_st_wait();
+          fence_before();
+          warp_arrive(&bar_p[u % NBUF], lane);
+        }
+        // merge the two accumulators of every row: O = (O_a 2^(m_a - m) + O_b 2^(m_b - m)) / l
+        if (C::PERSIST) {
+          if (ok && done > 0) ok = mbar_wait_warp(&bar_epi, (done - 1) & 1, fl);    // (read by everybody for the tile before)
+          if (!ok) break;
+        }
+        xch[part][0][trow] = m_ref;
+        xch[part][1][trow] = l;
+        if (C::PERSIST) {
+          warp_arrive(&bar_x, lane);
+          ok = mbar_wait_warp(&bar_x, done & 1, fl);
+        } else {
+          asm volatile("bar.sync 1, 256;" ::: "memory");        // the eight compute warps, always executed
+        }
+        if (ok) ok = mbar_wait_warp(&bar_done, done & 1, fl);
+        if (ok) {
+          fence_after();
+          if (mychunk >= 0) {                                   // uniform per warp: a warp lies inside one chunk
+            const float ma = xch[0][0][trow], mb = xch[1][0][trow], la = xch[0][1][trow], lb = xch[1][1][trow];
+            const float m = fmaxf(ma, mb);
+            const float wa = ma == kNegInfT ? 0.f : fast_exp2(ma - m), wb = mb == kNegInfT ? 0.f : fast_exp2(mb - m);
+            const float lsum = la * wa + lb * wb;
+            const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
+            T* orow = reinterpret_cast<T*>(a.out0) + z * a.o_sz + h * a.o_sh + grow * a.o_sr;
+            const uint32_t ta = tmem + C::ACC_BASE + lane_base;
+            // (a tile of one chunk leaves the other group's accumulator as it was)
+            const bool use_a = G == 1 || ntiles > 1 || !(base & 1), use_b = G == 1 || ntiles > 1 || (base & 1);
+            for (int c = part * (D / 2); c < (part + 1) * (D / 2); c += 32) {
+              uint32_t ra[32], rb[32];
+              tmem_ld32(ta + c, ra);
+              tmem_ld32(ta + D + c, rb);
+              tmem_ld_wait();
+              if (!use_a || !use_b) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                  if (!use_a) ra[i] = 0u;
+                  if (!use_b) rb[i] = 0u;
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 32; i += 8) {
+                float o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  o[j] = (__uint_as_float(ra[i + j]) * wa + __uint_as_float(rb[i + j]) * wb) * inv;
+                uint4 v;
+                v.x = pack16<T>(o[0], o[1]); v.y = pack16<T>(o[2], o[3]);
+                v.z = pack16<T>(o[4], o[5]); v.w = pack16<T>(o[6], o[7]);
+                if (row_ok && c + i < a.d) *reinterpret_cast<uint4*>(orow + c + i) = v;
+              }
+            }
+            if (part == 0 && row_ok) a.lse_out[zh + grow] = lsum > 0.f ? m + log2f(lsum) : kNegInfT;
+          }
+        }
+      } else {
+        // (a fully masked query row has lse = -inf: +inf makes its probabilities 0, not NaN)
+        float my_lse = (MODE == DQ && row_ok) ? a.lse[zh + grow] : 0.f;
+        if ((KPM || FINE) && my_lse == kNegInfT) my_lse = -kNegInfT;
+        // dK/dV: the bias of this thread's key row
+        const float my_b = (KPM && MODE == DKV && row_ok)
+            ? kpm_term(static_cast<float>(reinterpret_cast<const T*>(a.kpm)[z * a.kpm_sz + grow]), a.kpm_mul) : 0.f;
+        const float my_d = (MODE == DQ && row_ok) ? a.delta[zh + grow] : 0.f;
+        const float2 nd2 = f2(-my_d, -my_d), sl2 = f2(a.scale_log2, a.scale_log2);
+        for (int t = t0; ok && t < ntiles; t += G) {
+          const int u = base + t;
+          const uint32_t ts = tmem + (u % NBUF) * C::SCORE_COLS + lane_base + chalf * 32;
+          int pieces = 3;
+          bool valid, partial = false;
+          if constexpr (FINE) {
+            pieces = chunk_pieces(a.mask[first + t], a.sub[first + t], half, trow, chalf);
+            valid = __any_sync(0xffffffffu, pieces != 0);               // per warp: something to compute
+            partial = __any_sync(0xffffffffu, pieces != 3);
+          } else {
+            valid = (a.mask[first + t] >> half) & 1;                    // uniform per warp
+          }
+          const float4* vec = reinterpret_cast<const float4*>(stg + (u % ST) * C::STAGE + 2 * C::CH_BYTES) + chalf * 8;
+          ok = mbar_wait_warp(&bar_s[u % NBUF], (u / NBUF) & 1, fl);
+          if (!ok) break;
+          fence_after();
+          if constexpr (C::ER) {
+            // S and dP of this thread's 32 columns go to registers at once; the score buffer is
+            // then handed back, and the next scores are computed during the arithmetic below
+            uint32_t sr[32], qr[32], dr[16];
             tmem_ld32(ts, sr);
+            tmem_ld32(ts + 64, qr);
             tmem_ld_wait();
             fence_before();
             warp_arrive(&bar_rd[0], lane);
             if (partial) mask_pieces(sr, pieces);
-            if (FINE && a.causal) mask_causal<32, true>(sr, a.chunk[first + t] * 64 + chalf * 32, (int)grow);
-            const float2 nsl2 = f2(-a.scale_log2, -a.scale_log2);
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              float4 lv = vec[i / 4];                           // per-query lse of this chunk
-              if (KPM || FINE) {                              // own bias; a query row without any key counts as +inf
-                lv.x = lv.x == kNegInfT ? -kNegInfT : lv.x - my_b; lv.y = lv.y == kNegInfT ? -kNegInfT : lv.y - my_b;
-                lv.z = lv.z == kNegInfT ? -kNegInfT : lv.z - my_b; lv.w = lv.w == kNegInfT ? -kNegInfT : lv.w - my_b;
-              }
-              if constexpr (XT) {                             // rpe / mask of (query chalf * 32 + i .. + 3, this key)
-                const unsigned char* xt = stg + (t % ST) * C::STAGE + C::XT_OFF;
-                lv.x -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i, trow & 63);
-                lv.y -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 1, trow & 63);
-                lv.z -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 2, trow & 63);
-                lv.w -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 3, trow & 63);
-              }
-              // the negated exponent lse - s c: the lse comes from shared memory as it is
-              const float2 z0 = __ffma2_rn(u2f(sr[i], sr[i + 1]), nsl2, f2(lv.x, lv.y));
-              const float2 z1 = __ffma2_rn(u2f(sr[i + 2], sr[i + 3]), nsl2, f2(lv.z, lv.w));
-              const float2 p0 = exp2_pair<-1>(z0);
-              const float2 p1 = exp2_pair<-1>(z1);
-              pf[i] = p0.x; pf[i + 1] = p0.y; pf[i + 2] = p1.x; pf[i + 3] = p1.y;
-            }
-          } else {
-            fence_before();
-            warp_arrive(&bar_rd[0], lane);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) pf[i] = 0.f;
-          }
-          ok = mbar_wait_warp(&bar_s[2], t & 1, fl);
-          if (!ok) break;
-          fence_after();
-#pragma unroll
-          for (int hv = 0; hv < 2; ++hv) {
-            uint32_t qr[16], dr[8], ph[8];
+            if (FINE && a.causal) mask_causal<32, false>(sr, a.chunk[first + t] * 64 + chalf * 32, (int)grow);
             if (valid) {
-              tmem_ld16(ts + 64 + hv * 16, qr);
-              tmem_ld_wait();
+              const unsigned char* bp = stg + (u % ST) * C::STAGE + 2 * C::CH_BYTES + chalf * 64;
 #pragma unroll
-              for (int i = 0; i < 16; i += 4) {
-                const float4 ev = vec[16 + hv * 4 + i / 4];     // per-query delta of this chunk
-                const float2 pa = f2(pf[hv * 16 + i], pf[hv * 16 + i + 1]), pb = f2(pf[hv * 16 + i + 2], pf[hv * 16 + i + 3]);
-                // P (dP - delta); the score scale is applied to dK when it is stored
-                const float2 d0 = __fmul2_rn(pa, __ffma2_rn(f2(ev.x, ev.y), f2(-1.f, -1.f), u2f(qr[i], qr[i + 1])));
-                const float2 d1 = __fmul2_rn(pb, __ffma2_rn(f2(ev.z, ev.w), f2(-1.f, -1.f), u2f(qr[i + 2], qr[i + 3])));
-                dr[i / 2] = pack16<T>(d0.x, d0.y); dr[i / 2 + 1] = pack16<T>(d1.x, d1.y);
-                ph[i / 2] = pack16<T>(pa.x, pa.y); ph[i / 2 + 1] = pack16<T>(pb.x, pb.y);
+              for (int g = 0; g < 4; ++g) {
+                float b[8];
+                if constexpr (KPM || XT) {
+                  if constexpr (KPM) kpm_terms8<T>(bp + g * 16, a.kpm_mul, b);
+                  else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) b[i] = 0.f;
+                  }
+                  if constexpr (XT) xt_add8<T>(stg + (u % ST) * C::STAGE + C::XT_OFF, a.has_rpe, a.am_mode, half, trow & 63, chalf * 4 + g, b);
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) b[i] -= my_lse;
+                } else {
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) b[i] = -my_lse;
+                }
+#pragma unroll
+                for (int i = 8 * g; i < 8 * g + 8; i += 2) {
+                  const float2 y = __ffma2_rn(u2f(sr[i], sr[i + 1]), sl2, f2(b[i - 8 * g], b[i + 1 - 8 * g]));
+                  const float2 p = exp2_pair<1>(y);
+                  const float2 d = __fmul2_rn(p, __fadd2_rn(u2f(qr[i], qr[i + 1]), nd2));   // P (dP - delta); the scale is applied to dQ
+                  dr[i / 2] = pack16<T>(d.x, d.y);
+                }
               }
             } else {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) { dr[i] = 0u; ph[i] = 0u; }
+              for (int i = 0; i < 16; ++i) dr[i] = 0u;
             }
-            tmem_st8(ts + 64 + hv * 16, ph);
-            tmem_st8(ts + 64 + hv * 16 + 8, dr);
+            if (u >= 2) {                                     // the accumulation of chunk u - 2 has read its operand
+              ok = mbar_wait_warp(&bar_acc[(u - 2) & 3], ((u - 2) >> 2) & 1, fl);
+              if (!ok) break;
+              fence_after();
+            }
+            tmem_st16(tmem + C::PK_BASE + (u & 1) * 32 + chalf * 16 + lane_base, dr);
+            tmem_st_wait();
+            fence_before();
+            warp_arrive(&bar_p[u & 1], lane);
+            continue;
           }
-          tmem_st_wait();
-          fence_before();
-          warp_arrive(&bar_p[0], lane);
-          continue;
-        }
-        // Two passes of 16 columns keep the live registers of a pass at 48.  The packed
-        // 16-bit results of pass hv go to columns [8 hv, 8 hv + 8) of this thread's own
-        // 32-column slice: pass 0 only overwrites columns it has already read.
+          if constexpr (C::ER2) {
+            // First all of S^T: read, handed back, exponentials, P^T packed to 16 bits; this runs
+            // while dP^T is still being computed.  Then dP^T in two passes of 16 columns; pass
+            // hv leaves its part of the packed P^T in columns [16 hv, 16 hv + 8) and its packed
+            // dS^T in the next 8 columns of this thread's 32 columns of dP^T, all read before.
+            // dS is formed with P as the accumulating product sees it (rounded to 16 bits),
+            // which is also how a stored softmax output would enter the product.
+            float pf[32];                                        // P^T of this thread's 32 columns
+            if (valid) {
+              uint32_t sr[32];
+              tmem_ld32(ts, sr);
+              tmem_ld_wait();
+              fence_before();
+              warp_arrive(&bar_rd[0], lane);
+              if (partial) mask_pieces(sr, pieces);
+              if (FINE && a.causal) mask_causal<32, true>(sr, a.chunk[first + t] * 64 + chalf * 32, (int)grow);
+              const float2 nsl2 = f2(-a.scale_log2, -a.scale_log2);
 #pragma unroll
-        for (int hv = 0; hv < 2; ++hv) {
-          uint32_t sr[16], qr[16], pr[8], dr[8];
-          if (valid) {
-            tmem_ld16(ts + hv * 16, sr);
-            tmem_ld16(ts + 64 + hv * 16, qr);
-            tmem_ld_wait();
-            if (partial && !((pieces >> hv) & 1)) {             // this pass is one group of 16 columns
+              for (int i = 0; i < 32; i += 4) {
+                float4 lv = vec[i / 4];                           // per-query lse of this chunk
+                if (KPM || FINE) {                              // own bias; a query row without any key counts as +inf
+                  lv.x = lv.x == kNegInfT ? -kNegInfT : lv.x - my_b; lv.y = lv.y == kNegInfT ? -kNegInfT : lv.y - my_b;
+                  lv.z = lv.z == kNegInfT ? -kNegInfT : lv.z - my_b; lv.w = lv.w == kNegInfT ? -kNegInfT : lv.w - my_b;
+                }
+                if constexpr (XT) {                             // rpe / mask of (query chalf * 32 + i .. + 3, this key)
+                  const unsigned char* xt = stg + (u % ST) * C::STAGE + C::XT_OFF;
+                  lv.x -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i, trow & 63);
+                  lv.y -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 1, trow & 63);
+                  lv.z -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 2, trow & 63);
+                  lv.w -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 3, trow & 63);
+                }
+                // the negated exponent lse - s c: the lse comes from shared memory as it is
+                const float2 z0 = __ffma2_rn(u2f(sr[i], sr[i + 1]), nsl2, f2(lv.x, lv.y));
+                const float2 z1 = __ffma2_rn(u2f(sr[i + 2], sr[i + 3]), nsl2, f2(lv.z, lv.w));
+                const float2 p0 = exp2_pair<-1>(z0);
+                const float2 p1 = exp2_pair<-1>(z1);
+                pf[i] = p0.x; pf[i + 1] = p0.y; pf[i + 2] = p1.x; pf[i + 3] = p1.y;
+              }
+            } else {
+              fence_before();
+              warp_arrive(&bar_rd[0], lane);
 #pragma unroll
-              for (int i = 0; i < 16; ++i) sr[i] = kNegInfBits;
+              for (int i = 0; i < 32; ++i) pf[i] = 0.f;
             }
-            if (FINE && a.causal) mask_causal<16, MODE == DKV>(sr, a.chunk[first + t] * 64 + chalf * 32 + hv * 16, (int)grow);
+            ok = mbar_wait_warp(&bar_s[2], u & 1, fl);
+            if (!ok) break;
+            fence_after();
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-              float ls[4], es[4];
-              if (MODE == DKV) {                            // per-query lse and delta * scale of this chunk
-                const float4 lv = vec[hv * 4 + i / 4], ev = vec[16 + hv * 4 + i / 4];
-                ls[0] = lv.x; ls[1] = lv.y; ls[2] = lv.z; ls[3] = lv.w;
-                es[0] = ev.x; es[1] = ev.y; es[2] = ev.z; es[3] = ev.w;
-                if (KPM || FINE) {
+            for (int hv = 0; hv < 2; ++hv) {
+              uint32_t qr[16], dr[8], ph[8];
+              if (valid) {
+                tmem_ld16(ts + 64 + hv * 16, qr);
+                tmem_ld_wait();
 #pragma unroll
-                  for (int j = 0; j < 4; ++j) ls[j] = ls[j] == kNegInfT ? -kNegInfT : ls[j] - my_b;
+                for (int i = 0; i < 16; i += 4) {
+                  const float4 ev = vec[16 + hv * 4 + i / 4];     // per-query delta of this chunk
+                  const float2 pa = f2(pf[hv * 16 + i], pf[hv * 16 + i + 1]), pb = f2(pf[hv * 16 + i + 2], pf[hv * 16 + i + 3]);
+                  // P (dP - delta); the score scale is applied to dK when it is stored
+                  const float2 d0 = __fmul2_rn(pa, __ffma2_rn(f2(ev.x, ev.y), f2(-1.f, -1.f), u2f(qr[i], qr[i + 1])));
+                  const float2 d1 = __fmul2_rn(pb, __ffma2_rn(f2(ev.z, ev.w), f2(-1.f, -1.f), u2f(qr[i + 2], qr[i + 3])));
+                  dr[i / 2] = pack16<T>(d0.x, d0.y); dr[i / 2 + 1] = pack16<T>(d1.x, d1.y);
+                  ph[i / 2] = pack16<T>(pa.x, pa.y); ph[i / 2 + 1] = pack16<T>(pb.x, pb.y);
                 }
               } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { ls[j] = my_lse; es[j] = my_d; }
-                if constexpr (KPM) {                        // bias of the four keys
-                  const uint2 raw = *reinterpret_cast<const uint2*>(stg + (t % ST) * C::STAGE + 2 * C::CH_BYTES + chalf * 64 + (hv * 16 + i) * 2);
-                  const float2 b01 = unpack16<T>(raw.x), b23 = unpack16<T>(raw.y);
-                  ls[0] -= kpm_term(b01.x, a.kpm_mul); ls[1] -= kpm_term(b01.y, a.kpm_mul);
-                  ls[2] -= kpm_term(b23.x, a.kpm_mul); ls[3] -= kpm_term(b23.y, a.kpm_mul);
-                }
+                for (int i = 0; i < 8; ++i) { dr[i] = 0u; ph[i] = 0u; }
               }
-              if constexpr (XT) {                             // rpe / mask of the four (query, key) pairs
-                const unsigned char* xt = stg + (t % ST) * C::STAGE + C::XT_OFF;
-                const int cc = chalf * 32 + hv * 16 + i;        // column of the chunk: a key (dQ) or a query (dK / dV)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                  ls[j] -= MODE == DKV ? xt_term<T>(xt, a.has_rpe, a.am_mode, half, cc + j, trow & 63)
-                                       : xt_term<T>(xt, a.has_rpe, a.am_mode, half, trow & 63, cc + j);
-              }
-              // two elements per instruction: the negated exponent lse - s c, P = 2^-(that), and
-              // dS = P (dP - delta); the score scale is applied when dQ / dK are written
-              const float2 nsl2 = f2(-a.scale_log2, -a.scale_log2), m1 = f2(-1.f, -1.f);
-              const float2 p0 = exp2_pair<-1>(__ffma2_rn(u2f(sr[i], sr[i + 1]), nsl2, f2(ls[0], ls[1])));
-              const float2 p1 = exp2_pair<-1>(__ffma2_rn(u2f(sr[i + 2], sr[i + 3]), nsl2, f2(ls[2], ls[3])));
-              const float2 d0 = __fmul2_rn(p0, __ffma2_rn(f2(es[0], es[1]), m1, u2f(qr[i], qr[i + 1])));
-              const float2 d1 = __fmul2_rn(p1, __ffma2_rn(f2(es[2], es[3]), m1, u2f(qr[i + 2], qr[i + 3])));
-              pr[i / 2] = pack16<T>(p0.x, p0.y); pr[i / 2 + 1] = pack16<T>(p1.x, p1.y);
-              dr[i / 2] = pack16<T>(d0.x, d0.y); dr[i / 2 + 1] = pack16<T>(d1.x, d1.y);
+              tmem_st8(ts + 64 + hv * 16, ph);
+              tmem_st8(ts + 64 + hv * 16 + 8, dr);
             }
-          } else {
+            tmem_st_wait();
+            fence_before();
+            warp_arrive(&bar_p[0], lane);
+            continue;
+          }
+          // Two passes of 16 columns keep the live registers of a pass at 48.  The packed
+          // 16-bit results of pass hv go to columns [8 hv, 8 hv + 8) of this thread's own
+          // 32-column slice: pass 0 only overwrites columns it has already read.
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { pr[i] = 0u; dr[i] = 0u; }
+          for (int hv = 0; hv < 2; ++hv) {
+            uint32_t sr[16], qr[16], pr[8], dr[8];
+            if (valid) {
+              tmem_ld16(ts + hv * 16, sr);
+              tmem_ld16(ts + 64 + hv * 16, qr);
+              tmem_ld_wait();
+              if (partial && !((pieces >> hv) & 1)) {             // this pass is one group of 16 columns
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sr[i] = kNegInfBits;
+              }
+              if (FINE && a.causal) mask_causal<16, MODE == DKV>(sr, a.chunk[first + t] * 64 + chalf * 32 + hv * 16, (int)grow);
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                float ls[4], es[4];
+                if (MODE == DKV) {                            // per-query lse and delta * scale of this chunk
+                  const float4 lv = vec[hv * 4 + i / 4], ev = vec[16 + hv * 4 + i / 4];
+                  ls[0] = lv.x; ls[1] = lv.y; ls[2] = lv.z; ls[3] = lv.w;
+                  es[0] = ev.x; es[1] = ev.y; es[2] = ev.z; es[3] = ev.w;
+                  if (KPM || FINE) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) ls[j] = ls[j] == kNegInfT ? -kNegInfT : ls[j] - my_b;
+                  }
+                } else {
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) { ls[j] = my_lse; es[j] = my_d; }
+                  if constexpr (KPM) {                        // bias of the four keys
+                    const uint2 raw = *reinterpret_cast<const uint2*>(stg + (u % ST) * C::STAGE + 2 * C::CH_BYTES + chalf * 64 + (hv * 16 + i) * 2);
+                    const float2 b01 = unpack16<T>(raw.x), b23 = unpack16<T>(raw.y);
+                    ls[0] -= kpm_term(b01.x, a.kpm_mul); ls[1] -= kpm_term(b01.y, a.kpm_mul);
+                    ls[2] -= kpm_term(b23.x, a.kpm_mul); ls[3] -= kpm_term(b23.y, a.kpm_mul);
+                  }
+                }
+                if constexpr (XT) {                             // rpe / mask of the four (query, key) pairs
+                  const unsigned char* xt = stg + (u % ST) * C::STAGE + C::XT_OFF;
+                  const int cc = chalf * 32 + hv * 16 + i;        // column of the chunk: a key (dQ) or a query (dK / dV)
+#pragma unroll
+                  for (int j = 0; j < 4; ++j)
+                    ls[j] -= MODE == DKV ? xt_term<T>(xt, a.has_rpe, a.am_mode, half, cc + j, trow & 63)
+                                         : xt_term<T>(xt, a.has_rpe, a.am_mode, half, trow & 63, cc + j);
+                }
+                // two elements per instruction: the negated exponent lse - s c, P = 2^-(that), and
+                // dS = P (dP - delta); the score scale is applied when dQ / dK are written
+                const float2 nsl2 = f2(-a.scale_log2, -a.scale_log2), m1 = f2(-1.f, -1.f);
+                const float2 p0 = exp2_pair<-1>(__ffma2_rn(u2f(sr[i], sr[i + 1]), nsl2, f2(ls[0], ls[1])));
+                const float2 p1 = exp2_pair<-1>(__ffma2_rn(u2f(sr[i + 2], sr[i + 3]), nsl2, f2(ls[2], ls[3])));
+                const float2 d0 = __fmul2_rn(p0, __ffma2_rn(f2(es[0], es[1]), m1, u2f(qr[i], qr[i + 1])));
+                const float2 d1 = __fmul2_rn(p1, __ffma2_rn(f2(es[2], es[3]), m1, u2f(qr[i + 2], qr[i + 3])));
+                pr[i / 2] = pack16<T>(p0.x, p0.y); pr[i / 2 + 1] = pack16<T>(p1.x, p1.y);
+                dr[i / 2] = pack16<T>(d0.x, d0.y); dr[i / 2 + 1] = pack16<T>(d1.x, d1.y);
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) { pr[i] = 0u; dr[i] = 0u; }
+            }
+            if (MODE == DKV) tmem_st8(ts + hv * 8, pr);
+            tmem_st8(ts + 64 + hv * 8, dr);
           }
-          if (MODE == DKV) tmem_st8(ts + hv * 8, pr);
-          tmem_st8(ts + 64 + hv * 8, dr);
+          tmem_st_wait();
+          fence_before();
+          warp_arrive(&bar_p[u % NBUF], lane);
         }
-        tmem_st_wait();
+        if (ok) ok = mbar_wait_warp(&bar_done, done & 1, fl);
+        if (ok) {
+          fence_after();
+          if (mychunk >= 0 && part * 32 < D) {                  // uniform per warp
+            // the threads of a row split the D output columns, 32 or more each
+            constexpr int NCOL = D / (NC / 4) < 32 ? 32 : D / (NC / 4);
+            const uint32_t ta = tmem + C::ACC_BASE + lane_base;
+            const int64_t at = z * a.o_sz + h * a.o_sh + grow * a.o_sr;
+            T* o0 = reinterpret_cast<T*>(a.out0) + at;
+            // (dS is formed without the score scale, which is applied here)
+            const float ds_scale = a.scale;
+            if (MODE == DQ) {
+              store_acc<T>(o0, ta, part * NCOL, NCOL, a.d, row_ok, ds_scale);
+            } else {
+              T* o1 = reinterpret_cast<T*>(a.out1) + at;
+              store_acc<T>(o1, ta, part * NCOL, NCOL, a.d, row_ok, 1.f);            // dV: accumulator columns [0, D)
+              store_acc<T>(o0, ta + D, part * NCOL, NCOL, a.d, row_ok, ds_scale);    // dK: accumulator columns [D, 2D)
+            }
+          }
+        }
+      }
+      if (!ok) break;
+      if (C::PERSIST) {                                         // the accumulators are free for the next tile
         fence_before();
-        warp_arrive(&bar_p[t % NBUF], lane);
+        warp_arrive(&bar_epi, lane);
       }
-      if (ok && mbar_wait_warp(&bar_done, 0, fl)) {
-        fence_after();
-        if (mychunk >= 0) {                                   // uniform per warp
-          // the threads of a row split the D output columns
-          constexpr int NCOL = D / (NC / 4);
-          const uint32_t ta = tmem + C::ACC_BASE + lane_base;
-          const int64_t at = z * a.o_sz + h * a.o_sh + grow * a.o_sr;
-          T* o0 = reinterpret_cast<T*>(a.out0) + at;
-          // (dS is formed without the score scale, which is applied here)
-          const float ds_scale = a.scale;
-          if (MODE == DQ) {
-            store_acc<T>(o0, ta, part * NCOL, NCOL, a.d, row_ok, ds_scale);
-          } else {
-            T* o1 = reinterpret_cast<T*>(a.out1) + at;
-            store_acc<T>(o1, ta, part * NCOL, NCOL, a.d, row_ok, 1.f);            // dV: accumulator columns [0, D)
-            store_acc<T>(o0, ta + D, part * NCOL, NCOL, a.d, row_ok, ds_scale);    // dK: accumulator columns [D, 2D)
-          }
-        }
-      }
+      tile_done();
     }
   }
   fence_before();

@@ -117,6 +117,25 @@ BSP_DEVI void prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// ---- work of CTAs not yet started -----------------------------------------------
+// Asks the hardware for the work of a CTA of this grid that has not started; the answer (16 bytes,
+// aligned) arrives on `bar`.  No further request may follow an answer without work.
+BSP_DEVI void clc_ask(void* answer, uint64_t* bar) {
+  mbar_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(saddr(answer)), "r"(saddr(bar)) : "memory");
+}
+// Whether the answer names a CTA, which then never starts, and its blockIdx.x.
+BSP_DEVI bool clc_answer(const void* answer, uint32_t* block) {
+  uint32_t ok, x;
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b128 r;\n\tld.shared.b128 r, [%2];\n\t"
+               "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\tselp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+               "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}"
+               : "=r"(ok), "=r"(x) : "r"(saddr(answer)) : "memory");
+  *block = x;
+  return ok != 0;
+}
+
 // ---- tensor memory ---------------------------------------------------------------
 BSP_DEVI void tmem_alloc(uint32_t* slot, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(slot)), "r"(ncols) : "memory");
