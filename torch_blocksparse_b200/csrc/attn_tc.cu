@@ -237,9 +237,10 @@ template <int D, int MODE, bool KPM = false, int XT = 0> struct Cfg {
   // alternating chunks fill each other's waits.  At 64 the second CTA of the SM does that.
   // Fixed layout, 1 x 16 x 8192 x 128 (us): forward 152 -> 109, dQ 166 -> 125, dK/dV 222 -> 193; BigBird,
   // 4 x 16 x 16384 x 128: 998 -> 862, 1119 -> 969, 1469 -> 1463.
-  // Not with fewer than three stages, of which two are in use at a time (rpe and mask pieces), and not in
-  // the forward with one kind of pieces, which got slower (3 x 12 x 1664, block 16: 74 -> 78 us).
-  static constexpr int G = (D == 128 && (XT == 0 || (XT == 1 && MODE != FWD))) ? 2 : 1;
+  // So do two groups in dK/dV where the rpe / mask pieces in shared memory leave room for one CTA only
+  // at 64 (4 x 16 x 4096 with rpe, padding and causal masks: 308 -> 257 us). Not with fewer than three stages, of which two are in use at a time (both pieces at 128), and
+  // not in the forward with pieces at 128, which got slower (3 x 12 x 1664, block 16: 74 -> 78 us).
+  static constexpr int G = (D == 128 ? XT == 0 || (XT == 1 && MODE != FWD) : MODE == DKV && XT) ? 2 : 1;
   // Forward with two groups: a thread owns all 64 columns of its row of the chunk, and the two O
   // accumulators (running maxima, sums) belong to the groups instead of to the halves of a chunk.
   static constexpr int NH = (MODE == FWD && G == 2) ? 2 : 1;   // pieces of 32 columns per thread
