@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(DsdCfg<T, B, TN, AKC, BKC>::NW * 32) dsd_kerne
   T* cmat = reinterpret_cast<T*>(p.c) + z * p.c_sz + h * p.c_sh + ((int64_t)o * B + m0) * p.c_sm +
             ((int64_t)n0g + n0) * p.c_sn;
   const int n_lim = n_ok - n0;
-  for_each_acc<T, Sh::WM, Sh::WN>(acc, lane, [&](int r, int cidx, float v) {
+  for_each_acc<T, Sh::WM, Sh::WN, AKC, BKC>(acc, lane, [&](int r, int cidx, float v) {
     if (cidx < n_lim) cmat[r * p.c_sm + cidx * p.c_sn] = cvt_out<T>(v);
   });
 }

@@ -35,6 +35,9 @@ template <> struct SddShape<64>  { static constexpr int WM = 32, WN = 32, NW = 4
 template <> struct SddShape<128> { static constexpr int WM = 64, WN = 32, NW = 8, G = 1; };
 
 constexpr int kStages = 3;
+// FP32 operands are read 16 or 8 bytes at a time (tile.cuh), except for blocks of 32 with A K-contiguous
+// and B not: 4 heads of 1024^3, batch 2, density 0.25 took 180 us with single floats, 189-201 with wide reads.
+template <int B, bool AKC, bool BKC> constexpr bool kWide = !(B == 32 && AKC && !BKC);
 
 template <typename T, int B, bool AKC, bool BKC>
 struct SddSmem {
@@ -114,14 +117,27 @@ __global__ void __launch_bounds__(SddShape<B>::NW * 32) sdd_kernel(SddArgs p) {
     if (nx < nchunks) issue(nx, nx % kStages);
     cp_async_commit();
     const T* st = smem + (c % kStages) * S::STAGE + g_w * (S::A_ELEMS + S::B_ELEMS);
-    warp_tile_mma<T, Sh::WM, Sh::WN, TK, AKC, BKC, S::PA, S::PB>(acc, st, st + S::A_ELEMS, m0, n0, lane);
+    warp_tile_mma<T, Sh::WM, Sh::WN, TK, AKC, BKC, S::PA, S::PB, kWide<B, AKC, BKC>>(acc, st, st + S::A_ELEMS, m0, n0, lane);
   }
   cp_async_wait<0>();
 
   const int bid = bid0 + g_w;
   if (bid < p.nnz) {
     T* cb = reinterpret_cast<T*>(p.c) + z * p.c_sz + (int64_t)bid * B * B;
-    for_each_acc<T, Sh::WM, Sh::WN>(acc, lane, [&](int r, int cidx, float v) {
+    if constexpr (!Elem<T>::MMA && !BKC && kWide<B, AKC, BKC>) {
+      // a lane holds runs of four columns here: whole 16-byte pieces instead of every fourth float
+      if ((reinterpret_cast<uintptr_t>(cb) & 15) == 0) {
+        constexpr int RI = Sh::WM / 8, CJ = Sh::WN / 4;
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+#pragma unroll
+          for (int j = 0; j < CJ; j += 4)
+            *reinterpret_cast<float4*>(cb + (m0 + f32_index<AKC, 8, RI, true>(lane >> 2, i)) * B + n0 + f32_index<false, 4, CJ, true>(lane & 3, j)) =
+                make_float4(acc.v[i * CJ + j], acc.v[i * CJ + j + 1], acc.v[i * CJ + j + 2], acc.v[i * CJ + j + 3]);
+        return;
+      }
+    }
+    for_each_acc<T, Sh::WM, Sh::WN, AKC, BKC, kWide<B, AKC, BKC>>(acc, lane, [&](int r, int cidx, float v) {
       cb[(m0 + r) * B + n0 + cidx] = cvt_out<T>(v);
     });
   }

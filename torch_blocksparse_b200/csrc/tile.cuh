@@ -108,9 +108,62 @@ __device__ __forceinline__ void mma16816<__nv_bfloat16>(float (&d)[4], const uin
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// FP32: which of the warp tile's rows (columns) accumulator index i of lane group g holds, of LANES groups
+// with CNT rows each.  A K-contiguous operand is read 16 (8) bytes along K at a time, rows LANES apart
+// (their pitch, an odd multiple of 16 bytes, spreads them over all banks); a K-strided one V = 4 or
+// 2 consecutive rows at a time.  Single floats took one shared-memory instruction per operand value
+// (batch 2, 4 heads, 1024^3, density 0.25, us: sdd block 16 / 32 / 64 / 128 with A transposed 303 -> 199,
+// 160 -> 129, 144 -> 109, 123 -> 109; dsd transposed 179 -> 157, 148 -> 112, 132 -> 109, 150 -> 136).
+// !WIDE: single floats, rows LANES apart, in either orientation (see kWide of sdd_impl.cuh).
+template <bool KC, int LANES, int CNT, bool WIDE>
+__device__ __forceinline__ constexpr int f32_index(int g, int i) {
+  constexpr int V = CNT % 4 == 0 ? 4 : 2;
+  return KC || !WIDE ? g + LANES * i : (i / V) * (LANES * V) + g * V + i % V;
+}
+// The CNT values of an operand at k0 .. k0 + KQ - 1: v[i][kk].
+template <bool KC, int LANES, int CNT, int PITCH, int KQ, bool WIDE>
+__device__ __forceinline__ void f32_load(const float* s, int base, int g, int k0, float (&v)[CNT][KQ]) {
+  if constexpr (KC) {
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) {
+      const float* p = s + (base + g + LANES * i) * PITCH + k0;
+      if constexpr (KQ == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+      } else if constexpr (KQ == 2) {
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        v[i][0] = x.x; v[i][1] = x.y;
+      } else {
+        v[i][0] = *p;
+      }
+    }
+  } else if constexpr (!WIDE) {
+#pragma unroll
+    for (int kk = 0; kk < KQ; ++kk)
+#pragma unroll
+      for (int i = 0; i < CNT; ++i) v[i][kk] = s[(k0 + kk) * PITCH + base + g + LANES * i];
+  } else {
+    constexpr int V = CNT % 4 == 0 ? 4 : 2;
+    static_assert(CNT % V == 0, "rows per lane");
+#pragma unroll
+    for (int kk = 0; kk < KQ; ++kk)
+#pragma unroll
+      for (int i = 0; i < CNT; i += V) {
+        const float* p = s + (k0 + kk) * PITCH + base + f32_index<false, LANES, CNT, true>(g, i);
+        if constexpr (V == 4) {
+          const float4 x = *reinterpret_cast<const float4*>(p);
+          v[i][kk] = x.x; v[i + 1][kk] = x.y; v[i + 2][kk] = x.z; v[i + 3][kk] = x.w;
+        } else {
+          const float2 x = *reinterpret_cast<const float2*>(p);
+          v[i][kk] = x.x; v[i + 1][kk] = x.y;
+        }
+      }
+  }
+}
+
 // One K-chunk (TK elements) of the warp tile at rows [m0, m0+WM), cols [n0, n0+WN).
 // As / Bs point at the CTA tiles of the current stage; PA / PB are their pitches.
-template <typename T, int WM, int WN, int TK, bool AKC, bool BKC, int PA, int PB>
+template <typename T, int WM, int WN, int TK, bool AKC, bool BKC, int PA, int PB, bool WIDE = true>
 __device__ __forceinline__ void warp_tile_mma(Acc<T, WM, WN>& acc, const T* As, const T* Bs,
                                               int m0, int n0, int lane) {
   if constexpr (Elem<T>::MMA) {
@@ -150,33 +203,30 @@ __device__ __forceinline__ void warp_tile_mma(Acc<T, WM, WN>& acc, const T* As, 
       }
     }
   } else {
-    // FP32: lane (ty, tx) = (lane / 4, lane % 4) owns rows ty + 8i and cols tx + 4j.
-    constexpr int RI = WM / 8, CJ = WN / 4;
+    // FP32: lane (ty, tx) = (lane / 4, lane % 4) owns RI rows and CJ columns (f32_index), k ascending.
+    // (with 32 accumulators or more per thread, two values of k at a time leave registers for more warps;
+    // 32 x 32 with only B K-contiguous: one, sdd block 32 takes 192 us with one, 222 with two, 214 with single floats)
+    constexpr int RI = WM / 8, CJ = WN / 4, KQ = !WIDE || (!AKC && BKC && WM == 32 && WN == 32) ? 1 : RI * CJ >= 32 ? 2 : 4;
+    static_assert(TK % 4 == 0 && PA % 4 == 0 && PB % 4 == 0, "16-byte reads");
     const int ty = lane >> 2, tx = lane & 3;
 #pragma unroll
-    for (int k = 0; k < TK; ++k) {
-      float av[RI], bv[CJ];
+    for (int k = 0; k < TK; k += KQ) {
+      float av[RI][KQ], bv[CJ][KQ];
+      f32_load<AKC, 8, RI, PA, KQ, WIDE>(As, m0, ty, k, av);
+      f32_load<BKC, 4, CJ, PB, KQ, WIDE>(Bs, n0, tx, k, bv);
 #pragma unroll
-      for (int i = 0; i < RI; ++i) {
-        const int m = m0 + ty + 8 * i;
-        av[i] = AKC ? As[m * PA + k] : As[k * PA + m];
-      }
+      for (int kk = 0; kk < KQ; ++kk)
 #pragma unroll
-      for (int j = 0; j < CJ; ++j) {
-        const int n = n0 + tx + 4 * j;
-        bv[j] = BKC ? Bs[n * PB + k] : Bs[k * PB + n];
-      }
+        for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int i = 0; i < RI; ++i)
-#pragma unroll
-        for (int j = 0; j < CJ; ++j) acc.v[i * CJ + j] = fmaf(av[i], bv[j], acc.v[i * CJ + j]);
+          for (int j = 0; j < CJ; ++j) acc.v[i * CJ + j] = fmaf(av[i][kk], bv[j][kk], acc.v[i * CJ + j]);
     }
   }
 }
 
 // Calls f(row, col, value) for every accumulator element of the warp tile
 // (row / col relative to the warp tile origin).
-template <typename T, int WM, int WN, typename F>
+template <typename T, int WM, int WN, bool AKC, bool BKC, bool WIDE = true, typename F>
 __device__ __forceinline__ void for_each_acc(const Acc<T, WM, WN>& acc, int lane, F&& f) {
   if constexpr (Elem<T>::MMA) {
     constexpr int MI = WM / 16, NI = WN / 8;
@@ -194,7 +244,7 @@ __device__ __forceinline__ void for_each_acc(const Acc<T, WM, WN>& acc, int lane
 #pragma unroll
     for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int j = 0; j < CJ; ++j) f(ty + 8 * i, tx + 4 * j, acc.v[i * CJ + j]);
+      for (int j = 0; j < CJ; ++j) f(f32_index<AKC, 8, RI, WIDE>(ty, i), f32_index<BKC, 4, CJ, WIDE>(tx, j), acc.v[i * CJ + j]);
   }
 }
 
