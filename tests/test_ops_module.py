@@ -94,3 +94,21 @@ def test_linear_with_any_number_of_rows(block, rows):
     want_dw = (x2.T @ dy2).reshape(3, block, 4, block)[idx[:, 0], :, idx[:, 1]]
     for got, want in ((y, (x2 @ w).view_as(y)), (dx, (dy2 @ w.T).view_as(dx)), (dw, want_dw)):
         torch.testing.assert_close(got.float(), want, rtol=2e-3, atol=2e-3 * float(want.pow(2).mean().sqrt() + 1e-3))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('grad', [False, True])
+def test_forward_mode_tangents_are_refused(grad):
+    """No operation has a forward-mode derivative: a dual tensor is an error, with and without gradients on."""
+    import torch.autograd.forward_ad as fwd
+    from torch_blocksparse_b200 import Linear, MatMul, Softmax, SparseSelfAttention
+    lay = torch.ones((1, 2, 2), dtype=torch.long)
+    make = lambda *s: torch.randn(s, device='cuda', dtype=torch.float16)
+    layer = Linear(64, 64, 32, lay).to('cuda', torch.float16)
+    layer.requires_grad_(grad)
+    with torch.set_grad_enabled(grad), fwd.dual_level():
+        x, q, rows = (fwd.make_dual(make(*s), make(*s)) for s in ((1, 4, 32, 32), (1, 1, 64, 64), (5, 64)))
+        for call in (lambda: MatMul(lay, 32, 'sdd')(q, make(1, 1, 64, 64)), lambda: Softmax(lay, 32)(x), lambda: layer(rows),
+                     lambda: SparseSelfAttention(layout=lay, block=32)(q, make(1, 1, 64, 64), make(1, 1, 64, 64))):
+            with pytest.raises((RuntimeError, NotImplementedError)):
+                call()

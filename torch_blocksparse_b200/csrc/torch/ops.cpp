@@ -56,6 +56,11 @@ void require_cuda(const Tensor& t) {
   TORCH_CHECK(t.is_cuda(), "torch_blocksparse_b200 runs on CUDA tensors only (got a ", t.device(), " tensor)");
 }
 
+// Whether a call on these tensors goes through autograd: one of them needs a gradient, or carries a
+// forward-mode tangent, which the functions below refuse (passing them by would drop it silently).
+template <typename... Ts> bool recorded(const Ts&... t) {
+  return (at::GradMode::is_enabled() && (t.requires_grad() || ...)) || (t._fw_grad(0).defined() || ...);
+}
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 int64_t vec_of(const Tensor& t) { return 16 / static_cast<int64_t>(t.element_size()); }
 bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0; }
@@ -257,7 +262,7 @@ Tensor matmul_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& a0, cons
   TORCH_CHECK_VALUE(a.scalar_type() == b.scalar_type(), "operands must have the same dtype (got ", a.scalar_type(), " and ",
                     b.scalar_type(), ")");
   const c10::cuda::CUDAGuard guard(a.device());
-  if (at::GradMode::is_enabled() && (a.requires_grad() || b.requires_grad())) return MatMulFn::apply(a, b, p, times);
+  if (recorded(a, b)) return MatMulFn::apply(a, b, p, times);
   return product(p->mode[0], p->mode[1], p->mode[2], *p, a, b, p->trans_a, p->trans_b, false, times ? &times->c : nullptr);
 }
 
@@ -300,7 +305,7 @@ Tensor linear_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& x, const
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor w = w0.scalar_type() == x.scalar_type() ? w0 : w0.to(x.scalar_type());
   double* time = times ? &times->c : nullptr;
-  if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad())) return LinearFn::apply(x, w, p, time);
+  if (recorded(x, w)) return LinearFn::apply(x, w, p, time);
   return LinearFn::run(*p, x, w, time);
 }
 
@@ -411,7 +416,7 @@ Tensor softmax_call(const c10::intrusive_ptr<SoftmaxOp>& p, const Tensor& x, dou
   const bool kpm_mul = mode_flag(kpm_mode, "key_padding_mask_mode"), am_mul = mode_flag(am_mode, "attn_mask_mode");
   const c10::cuda::CUDAGuard guard(x.device());
   double* time = times ? &times->c : nullptr;
-  if (at::GradMode::is_enabled() && x.requires_grad())
+  if (recorded(x))
     return SoftmaxFn::apply(x, p, scale, rpe, kpm, am, kpm_mul, am_mul, time);
   {
     const at::AutoDispatchBelowADInplaceOrView below;
@@ -547,7 +552,7 @@ Tensor attention_call(const c10::intrusive_ptr<AttentionOp>& p, const Tensor& q0
   c->kpm_mul = kpm_mul;
   c->am_mul = am_mul;
   c->use_tiles = use_tiles;
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
+  if (recorded(q, k, v))
     return AttentionFn::apply(q, k, v, c, m, rpe, kpm, am, seq_first);
   Tensor lse;
   return AttentionFn::run(*c, q, k, v, m, seq_first, &lse);
