@@ -112,3 +112,75 @@ def test_forward_mode_tangents_are_refused(grad):
                      lambda: SparseSelfAttention(layout=lay, block=32)(q, make(1, 1, 64, 64), make(1, 1, 64, 64))):
             with pytest.raises((RuntimeError, NotImplementedError)):
                 call()
+
+
+def test_recorded_calls_replay_with_gradients():
+    """torch.jit.trace on CPU: an operation whose result the tracer cannot see (raw memory) is replayed on new
+    inputs, with plain and absent arguments, and the trace passes the tracer's own check."""
+    from torch_blocksparse_b200 import tracing
+
+    class Op:
+        def run(self, a, mask, b, factor):
+            class Hidden(torch.autograd.Function):
+                @staticmethod
+                def forward(ctx, a, b):
+                    ctx.save_for_backward(a, b)
+                    out = torch.empty((a.size(0), b.size(1)))
+                    out.numpy()[...] = factor * (a.detach().numpy() @ b.detach().numpy())
+                    return out
+
+                @staticmethod
+                def backward(ctx, g):
+                    a, b = ctx.saved_tensors
+                    return factor * (g @ b.T), factor * (a.T @ g)
+            return Hidden.apply(a, b)
+    op = Op()
+    g = torch.Generator().manual_seed(0)
+    draw = lambda grad: [torch.randn((3, 3), generator=g).requires_grad_(grad) for _ in range(2)]
+    call = lambda a, b: tracing.call(op, 'run', tracing.call(op, 'run', a, None, b, 2.0), None, b, 0.5) + a
+    for grad in (True, False):
+        traced = torch.jit.trace(call, draw(grad))
+        a, b = draw(True)
+        want = (a @ b) @ b + a
+        torch.testing.assert_close(traced(a, b), want)
+        dy = torch.randn((3, 3), generator=g)
+        torch.testing.assert_close(torch.autograd.grad(traced(a, b), (a, b), dy), torch.autograd.grad(want, (a, b), dy))
+    with pytest.raises(RuntimeError, match='torch.jit.trace'):
+        torch.jit.trace(lambda x: Softmax(LAYOUT, 16)(x * 1), torch.zeros(1, 20, 16, 16), check_trace=False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('which', ['matmul', 'linear', 'attention', 'masked'])
+def test_traced_calls_run_their_kernels_again(which):
+    """A trace of the public classes, replayed on inputs it was not recorded with: the same bits as the call itself,
+    and the same gradients."""
+    from torch_blocksparse_b200 import Linear
+    g = torch.Generator('cuda').manual_seed(0)
+    draw = lambda *s: torch.randn(s, generator=g, device='cuda', dtype=torch.float16).requires_grad_()
+    if which == 'matmul':
+        mod, shapes = MatMul(LAYOUT, 16, 'sdd', trans_b=True), [(2, 2, 64, 32)] * 2
+    elif which == 'linear':
+        mod, shapes = Linear(64, 64, 16, LAYOUT[0]).to('cuda', torch.float16), [(5, 64)]
+    else:
+        mod, shapes = SparseSelfAttention(layout=LAYOUT, block=64, key_padding_mask_mode='mul'), [(2, 2, 256, 64)] * 3
+    mask = {}
+    if which == 'masked':
+        mask['key_padding_mask'] = (torch.arange(256, device='cuda') < torch.tensor([[200], [256]], device='cuda')).half()
+
+    class Call(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.mod = mod
+
+        def forward(self, *xs):
+            return self.mod(*xs, **mask) * 1
+    call = Call()
+    traced = torch.jit.trace(call, [draw(*s) for s in shapes])
+    xs = [draw(*s) for s in shapes]
+    want, got = call(*xs), traced(*xs)
+    assert torch.equal(got, want)
+    dy = torch.randn_like(want)
+    for a, b in zip(torch.autograd.grad(got, xs, dy), torch.autograd.grad(want, xs, dy)):
+        assert torch.equal(a, b)
+    with torch.no_grad():
+        assert torch.equal(traced(*xs), want)

@@ -22,7 +22,7 @@ import weakref
 import torch
 import torch.nn as nn
 
-from . import _lib, fused, tables
+from . import _lib, fused, tables, tracing
 from .matmul import MatMul
 from .softmax import Softmax
 
@@ -98,9 +98,8 @@ class DeepSpeedSparseSelfAttention(nn.Module):
             self.tiles[key] = tables.build_attn_tiles(layout, self.block) if self.fused else None
         return self.ops[key]
 
-    def _attn_op(self, query):
+    def _attn_op(self, query, H, L):
         """The fused attention with this module's tables on the device of `query`."""
-        _, H, L, _ = query.shape
         sdd_nt, _, _ = self.get_ops(H, L)
         op = fused.Attention(sdd_nt.meta, self.tiles[(H, L)], self.block, query.device)
         self._attn[(H, L, query.get_device())] = op
@@ -167,7 +166,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         mask_owner = attn_mask
         if attn_mask is not None:
             attn_mask = self.transpose_mask_for_sparse(query.dtype, attn_mask)
-        return self.attend(query, key, value, query.size(3) ** -0.5, rpe, key_padding_mask, attn_mask,
+        return self.attend(query, key, value, float(query.size(3)) ** -0.5, rpe, key_padding_mask, attn_mask,
                            mask_owner=mask_owner)
 
     def attend(self, query, key, value, scaling, rpe=None, key_padding_mask=None, attn_mask=None, mask_owner=None,
@@ -178,6 +177,8 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         fused kernel writes its result in [L, bsz, heads * head_dim] memory order (returned as the
         [bsz, heads, L, head_dim] view of it)."""
         _, num_heads, tgt_len, _ = query.shape
+        if tracing.recording() is not None:           # (sizes are tensors then, each one a key of its own)
+            num_heads, tgt_len = int(num_heads), int(tgt_len)
         if key_padding_mask is not None and key_padding_mask.dtype != query.dtype:
             key_padding_mask = key_padding_mask.to(query.dtype)
         if attn_mask is not None and attn_mask.dtype != query.dtype:
@@ -188,7 +189,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
             am_mode = self.attn_mask_mode
             if attn_mask is not None and am_mode == 'mul' and self._is_causal(attn_mask, mask_owner):
                 am_mode = 'causal'
-            op = self._attn.get((num_heads, tgt_len, query.get_device())) or self._attn_op(query)
+            op = self._attn.get((num_heads, tgt_len, query.get_device())) or self._attn_op(query, num_heads, tgt_len)
             return fused.attention(op, query, key, value, scaling, rpe, key_padding_mask, attn_mask,
                                    self.key_padding_mask_mode, am_mode, seq_first_out)
         sdd_nt, dsd_nn, softmax = self.get_ops(num_heads, tgt_len)

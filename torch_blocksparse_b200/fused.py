@@ -9,7 +9,7 @@ materialises it.  rpe and the masks follow the softmax op's conventions
 """
 import torch
 
-from . import _lib
+from . import _lib, tracing
 from .matmul import _dtype_code, _require_cuda, _stream
 
 
@@ -184,9 +184,12 @@ def attention(op, q, k, v, scale, rpe=None, key_padding_mask=None, attn_mask=Non
         raise ValueError("key_padding_mask_mode must be 'add' or 'mul'")
     if attn_mask_mode not in _AM_FLAG:
         raise ValueError("attn_mask_mode must be 'add' or 'mul'")
+    args = (q, k, v, scale, rpe, key_padding_mask, attn_mask, key_padding_mask_mode == 'mul', _AM_FLAG[attn_mask_mode],
+            PATH == 'tc', seq_first_out)
+    if tracing.recording() is not None:
+        return tracing.call(op.op, '__call__', *args)
     if PROFILE is None:
-        return op.op(q, k, v, scale, rpe, key_padding_mask, attn_mask, key_padding_mask_mode == 'mul',
-                     _AM_FLAG[attn_mask_mode], PATH == 'tc', seq_first_out)
+        return op.op(*args)
     return _profiled_attention.apply(q, k, v, op.meta, op.tiles, op.block, float(scale), rpe, key_padding_mask, attn_mask,
                                      key_padding_mask_mode, attn_mask_mode, seq_first_out)
 

@@ -17,7 +17,7 @@ import math
 
 import torch
 
-from . import _lib, tables
+from . import _lib, tables, tracing
 
 _DTYPES = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 
@@ -109,6 +109,8 @@ class MatMul:
 
     def __call__(self, a, b):
         op = self._ops.get(a.get_device()) or self._op(a.device)
+        if tracing.recording() is not None:
+            return tracing.call(op, '__call__', a, b)
         if not self.bench:
             return op(a, b)
         times = _lib.ops().Times()
@@ -156,6 +158,8 @@ class Linear(torch.nn.Module):
             raise ValueError('Linear: expected %d input features, got %d' % (self.in_features, input.size(-1)))
         mm = self.matmul
         op = mm._ops.get(input.get_device()) or mm._op(input.device)
+        if tracing.recording() is not None:
+            return tracing.call(op, 'linear', input, self.weight, None)
         times = _lib.ops().Times() if mm.bench else None
         y = op.linear(input, self.weight, times)
         if times is not None:

@@ -16,7 +16,7 @@ function and the launches are in csrc/torch/ops.cpp.
 """
 import torch
 
-from . import _lib, tables
+from . import _lib, tables, tracing
 
 
 class _sparse_softmax:
@@ -59,6 +59,8 @@ class Softmax:
 
     def __call__(self, x, scale=1., rpe=None, key_padding_mask=None, attn_mask=None,
                  key_padding_mask_mode='add', attn_mask_mode='add'):
+        if tracing.recording() is not None:
+            raise RuntimeError('Softmax works in place, which torch.jit.trace cannot replay')
         op = self._ops.get(x.get_device()) or self._op(x.device)
         times = _lib.ops().Times() if self.bench else None
         x = op(x, scale, rpe, key_padding_mask, attn_mask, key_padding_mask_mode, attn_mask_mode, times)
