@@ -60,6 +60,11 @@ def test_bad_arguments_are_rejected_with_messages():
     assert rc == _lib.ERR_UNSUPPORTED and b'32768' in L.bsp_last_error()
     rc = L.bsp_softmax_fwd(None, _lib.F16, 1, 256, 16, 1, 1, 16, 1, 1.0, None, 0, 0, 0, None, 0, 0, None, 0, 0, None)
     assert rc == _lib.ERR_INVALID
+    # a tensor written in place must not share memory between batch entries
+    rc = L.bsp_softmax_fwd(16, _lib.F16, 2, 0, 16, 1, 1, 16, 1, 1.0, None, 0, 0, 0, None, 0, 0, None, 0, 0, None)
+    assert rc == _lib.ERR_INVALID and b'share memory' in L.bsp_last_error()
+    rc = L.bsp_softmax_bwd(16, 16, _lib.F16, 2, 256, 0, 16, 1, 1, 16, 1, 1.0, None)
+    assert rc == _lib.ERR_INVALID and b'share memory' in L.bsp_last_error()
     # fused attention: dtype / head-dimension limits
     args = [16] * 4 + [16, _lib.F32, 16, 1, 1, 16, 64] + [8] * 12 + [hdr, fake_dev, None, None, 1.0] + [None, 0, 0, 0, None, 0, 0, None, 0, 0, None]
     assert L.bsp_attn_fwd(*args) == _lib.ERR_UNSUPPORTED

@@ -207,3 +207,23 @@ def test_config3_small_and_full():
     rowsum.index_add_(1, owner, dx.float().sum(-1))
     assert float(rowsum.abs().max()) < 2e-2
     assert_close(dx[z:z + 1, b0:b1], want_dx, 'config3 backward slice')
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float16])
+def test_gradient_shared_by_the_batch(dtype):
+    """The gradient of a sum over the batch is one tensor expanded over it: the backward, which works in
+    place, takes a copy.  A forward operand of that kind is refused."""
+    layout, block, Z = torch.tril(torch.ones((2, 5, 5), dtype=torch.long)), 16, 3
+    g = torch.Generator().manual_seed(0)
+    x = torch.randn((Z, 30, block, block), generator=g).to(dtype)
+    dy = torch.randn((30, block, block), generator=g).to(dtype)
+    want_y, want_dx = dm.softmax_reference(x, layout, block, dy=dy.expand(Z, -1, -1, -1).contiguous(), scale=0.5)
+    xg = x.to(DEV).requires_grad_()
+    y = Softmax(layout, block)(xg * 1, scale=0.5)
+    shared = dy.to(DEV)
+    dx, = torch.autograd.grad(y, xg, shared.expand(Z, -1, -1, -1), retain_graph=True)
+    assert_close(dx, want_dx, 'dx')
+    assert torch.equal(shared.cpu(), dy)
+    y.sum(0).sum().backward()
+    with pytest.raises(RuntimeError, match='same memory'):
+        Softmax(layout, block)(x[:1].to(DEV).expand(Z, -1, -1, -1))

@@ -914,6 +914,7 @@ extern "C" int bsp_softmax_fwd(void* x, int dtype, int Z, int64_t x_sz, int bloc
   if (maxlut == 0) return BSP_OK;
   const int vec = dtype == BSP_F32 ? 4 : 8;
   if (x_sz % vec) return fail(BSP_ERR_INVALID, "batch stride of x must be a multiple of %d elements", vec);
+  if (Z > 1 && x_sz == 0) return fail(BSP_ERR_INVALID, "batch entries of x share memory, which the result would overwrite");
   FwdArgs a;
   a.x = x; a.x_sz = x_sz; a.lut = lut; a.rows = H * Mb * block; a.block_log2 = log2i(block); a.scale = scale;
   a.rpe = rpe; a.rpe_sz = rpe_sz; a.rpe_sh = rpe_sh; a.rpe_sr = rpe_sr;
@@ -946,6 +947,7 @@ extern "C" int bsp_softmax_bwd(const void* y, void* dy, int dtype, int Z, int64_
   if (maxlut == 0) return BSP_OK;
   const int vec = dtype == BSP_F32 ? 4 : 8;
   if (y_sz % vec || dy_sz % vec) return fail(BSP_ERR_INVALID, "batch strides must be multiples of %d elements", vec);
+  if (Z > 1 && dy_sz == 0) return fail(BSP_ERR_INVALID, "batch entries of dy share memory, which the result would overwrite");
   BwdArgs a;
   a.y = y; a.dy = dy; a.y_sz = y_sz; a.dy_sz = dy_sz; a.lut = lut;
   a.rows = H * Mb * block; a.block_log2 = log2i(block); a.scale = scale;

@@ -134,6 +134,11 @@ bool block_format(const Tensor& x, int64_t block) {
          (x.size(0) == 1 || x.stride(0) % vec_of(x) == 0);
 }
 Tensor prep_sparse(const Tensor& x, int64_t block) { return block_format(x, block) ? x : x.contiguous(); }
+// Whether batch entries of a block-format tensor share memory (an expanded tensor, the gradient of a
+// sum over the batch): such a tensor can be read, but not written in place.
+bool shares_batch(const Tensor& x, int64_t block) {
+  return x.size(0) > 1 && x.size(1) > 0 && x.stride(0) < x.size(1) * block * block;
+}
 
 // `any_k`: the reduction size need not be a multiple of 16 (both operands must be k-strided then).
 Tensor sdd(const MatMulOp& p, Tensor a, Tensor b, bool ta, bool tb, bool tc, double* time, bool any_k = false) {
@@ -365,6 +370,8 @@ void softmax_fwd(const SoftmaxOp& p, const Tensor& x, double scale, OptTensor rp
                         x.size(1) * 4 + 2 * p.H * p.Mb == p.lut.numel(),
                     "x of shape ", x.sizes(), " is not a block-format tensor for this layout");
   const int64_t Z = x.size(0), M = p.Mb * p.block, N = p.Nb * p.block;
+  TORCH_CHECK(!block_format(x, p.block) || !shares_batch(x, p.block),
+              "softmax: batch entries of x refer to the same memory, which the result would overwrite; clone() the tensor first");
   const Tensor work = prep_sparse(x, p.block);
   Masks m;
   set_rpe(m, rpe, Z, p.H, M, N);
@@ -393,7 +400,9 @@ struct SoftmaxFn : torch::autograd::Function<SoftmaxFn> {
     const auto p = c10::static_intrusive_pointer_cast<SoftmaxOp>(ctx->saved_data["p"].toCapsule());
     const Tensor y = ctx->get_saved_variables()[0];
     const c10::cuda::CUDAGuard guard(y.device());
-    const Tensor dx = prep_sparse(grads[0], p->block), yy = prep_sparse(y, p->block);
+    Tensor dx = prep_sparse(grads[0], p->block);
+    if (shares_batch(dx, p->block)) dx = dx.clone(at::MemoryFormat::Contiguous);
+    const Tensor yy = prep_sparse(y, p->block);
     check(bsp_softmax_bwd(yy.const_data_ptr(), dx.mutable_data_ptr(), dtype_code(y), y.size(0), yy.stride(0), dx.stride(0), p->block,
                           p->H, p->Mb, p->lut.const_data_ptr<int32_t>(), p->maxlut,
                           static_cast<float>(ctx->saved_data["scale"].toDouble()), stream_of(y)));
