@@ -184,3 +184,49 @@ def test_traced_calls_run_their_kernels_again(which):
         assert torch.equal(a, b)
     with torch.no_grad():
         assert torch.equal(traced(*xs), want)
+
+
+def test_operands_of_another_type_or_device_are_refused():
+    """Before anything is launched: kernels read every operand through a pointer, as the type of the first."""
+    zeros = lambda *s, dtype=torch.float16, device='cpu': torch.zeros(s, dtype=dtype, device=device)
+    from torch_blocksparse_b200 import Linear
+    q = zeros(1, 2, 64, 96)
+    att = SparseSelfAttention(layout=LAYOUT, block=16)
+    for other in (dict(dtype=torch.bfloat16), dict(dtype=torch.float32)):
+        for args in ((q, zeros(1, 2, 64, 96, **other), q), (q, q, zeros(1, 2, 64, 96, **other))):
+            with pytest.raises(ValueError, match='must be Half'):
+                att(*args)
+        with pytest.raises(ValueError, match='same dtype'):
+            MatMul(LAYOUT, 16, 'sdd')(zeros(1, 2, 64, 16), zeros(1, 2, 16, 64, **other))
+    elsewhere = dict(device='meta')
+    for args, kw in (((q, zeros(1, 2, 64, 96, **elsewhere), q), {}), ((q, q, zeros(1, 2, 64, 96, **elsewhere)), {}),
+                     ((q, q, q), dict(rpe=zeros(2, 64, 64, **elsewhere))),
+                     ((q, q, q), dict(key_padding_mask=zeros(2, 64, **elsewhere)))):
+        with pytest.raises(RuntimeError, match='is on meta'):
+            att(*args, **kw)
+    x = zeros(1, 20, 16, 16)
+    for name, shape in (('rpe', (2, 64, 64)), ('key_padding_mask', (1, 64)), ('attn_mask', (64, 64))):
+        with pytest.raises(RuntimeError, match='is on meta'):
+            Softmax(LAYOUT, 16)(x, **{name: zeros(*shape, **elsewhere)})
+    with pytest.raises(ValueError, match=r'\[Z, H, L, D\]'):
+        from torch_blocksparse_b200 import fused
+        op = fused.Attention(MatMul(LAYOUT, 16, 'sdd').meta, None, 16, torch.device('cpu'))
+        fused.attention(op, q, q[..., :64], q, 1.0)
+    with pytest.raises(RuntimeError, match='CUDA tensors only'):
+        Linear(64, 64, 16, LAYOUT[0])(zeros(3, 64))
+
+
+@pytest.mark.gpu
+def test_operands_on_the_host_are_refused_beside_a_device():
+    zeros = lambda *s, device='cuda': torch.zeros(s, dtype=torch.float16, device=device)
+    from torch_blocksparse_b200 import Linear
+    q = zeros(1, 2, 64, 64)
+    lin = Linear(64, 64, 16, LAYOUT[0])
+    for call in (lambda: MatMul(LAYOUT, 16, 'sdd')(q, zeros(1, 2, 64, 64, device='cpu')), lambda: lin(zeros(3, 64)),
+                 lambda: SparseSelfAttention(layout=LAYOUT, block=16)(q, q, zeros(1, 2, 64, 64, device='cpu')),
+                 lambda: SparseSelfAttention(layout=LAYOUT, block=16)(q, q, q, key_padding_mask=zeros(2, 64, device='cpu')),
+                 lambda: Softmax(LAYOUT, 16)(zeros(1, 20, 16, 16), attn_mask=zeros(64, 64, device='cpu'))):
+        with pytest.raises(RuntimeError, match='cpu'):
+            call()
+    with pytest.raises(ValueError, match='graphed step'):
+        SparseSelfAttention(layout=LAYOUT, block=16).graphed(q, q.bfloat16(), q, q)

@@ -56,6 +56,12 @@ void require_cuda(const Tensor& t) {
   TORCH_CHECK(t.is_cuda(), "torch_blocksparse_b200 runs on CUDA tensors only (got a ", t.device(), " tensor)");
 }
 
+// Everything a call reads has to lie on one device, and a pointer has to be of the type it is read as.
+void require_same(const Tensor& t, const Tensor& ref, const char* what) {
+  TORCH_CHECK(t.device() == ref.device(), what, " is on ", t.device(), ", the call runs on ", ref.device());
+  TORCH_CHECK_VALUE(t.scalar_type() == ref.scalar_type(), what, " must be ", ref.scalar_type(), " (got ", t.scalar_type(), ")");
+}
+
 // Whether a call on these tensors goes through autograd: one of them needs a gradient, or carries a
 // forward-mode tangent, which the functions below refuse (passing them by would drop it silently).
 template <typename... Ts> bool recorded(const Ts&... t) {
@@ -262,10 +268,11 @@ Tensor pad_shape(Tensor x, int64_t dims) {
 Tensor matmul_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& a0, const Tensor& b0, const c10::intrusive_ptr<Times>& times) {
   // (the block format has three dimensions in the reference's reading; a batch of one is added)
   const Tensor a = pad_shape(a0, 4), b = pad_shape(b0, 4);
-  require_cuda(a);
-  require_cuda(b);
   TORCH_CHECK_VALUE(a.scalar_type() == b.scalar_type(), "operands must have the same dtype (got ", a.scalar_type(), " and ",
                     b.scalar_type(), ")");
+  require_cuda(a);
+  require_cuda(b);
+  require_same(b, a, "the second operand");
   const c10::cuda::CUDAGuard guard(a.device());
   if (recorded(a, b)) return MatMulFn::apply(a, b, p, times);
   return product(p->mode[0], p->mode[1], p->mode[2], *p, a, b, p->trans_a, p->trans_b, false, times ? &times->c : nullptr);
@@ -309,6 +316,7 @@ Tensor linear_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& x, const
   require_cuda(w0);
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor w = w0.scalar_type() == x.scalar_type() ? w0 : w0.to(x.scalar_type());
+  require_same(w, x, "the weight");
   double* time = times ? &times->c : nullptr;
   if (recorded(x, w)) return LinearFn::apply(x, w, p, time);
   return LinearFn::run(*p, x, w, time);
@@ -351,10 +359,14 @@ void set_am(Masks& m, OptTensor& am, int64_t M, int64_t N) {
   m.am = am->const_data_ptr();
   m.am_sr = am->stride(0);
 }
-void check_mask_dtypes(const OptTensor& rpe, const OptTensor& kpm, const OptTensor& am, at::ScalarType t) {
+void check_masks(const OptTensor& rpe, const OptTensor& kpm, const OptTensor& am, const Tensor& x) {
+  const at::ScalarType t = x.scalar_type();
   TORCH_CHECK_VALUE(!rpe || rpe->scalar_type() == t, "relative position embedding must be ", t);
   TORCH_CHECK_VALUE(!am || am->scalar_type() == t, "Attention mask must be ", t);
   TORCH_CHECK_VALUE(!kpm || kpm->scalar_type() == t, "Key padding mask must be ", t);
+  if (rpe) require_same(*rpe, x, "relative position embedding");
+  if (kpm) require_same(*kpm, x, "key_padding_mask");
+  if (am) require_same(*am, x, "attn_mask");
 }
 
 // ---- Softmax -----------------------------------------------------------------------------------
@@ -420,7 +432,7 @@ bool mode_flag(const std::string& mode, const char* name) {
 Tensor softmax_call(const c10::intrusive_ptr<SoftmaxOp>& p, const Tensor& x, double scale, const OptTensor& rpe,
                     const OptTensor& kpm, const OptTensor& am, const std::string& kpm_mode, const std::string& am_mode,
                     const c10::intrusive_ptr<Times>& times) {
-  check_mask_dtypes(rpe, kpm, am, x.scalar_type());
+  check_masks(rpe, kpm, am, x);
   require_cuda(x);
   const bool kpm_mul = mode_flag(kpm_mode, "key_padding_mask_mode"), am_mul = mode_flag(am_mode, "attn_mask_mode");
   const c10::cuda::CUDAGuard guard(x.device());
@@ -525,13 +537,15 @@ struct AttentionFn : torch::autograd::Function<AttentionFn> {
 
 Tensor attention_call(const c10::intrusive_ptr<AttentionOp>& p, const Tensor& q0, const Tensor& k0, const Tensor& v0, double scale,
                       OptTensor rpe, OptTensor kpm, OptTensor am, bool kpm_mul, int am_mul, bool use_tiles, bool seq_first) {
+  TORCH_CHECK_VALUE(q0.dim() == 4 && k0.sizes() == q0.sizes() && v0.sizes() == q0.sizes(), "query, key and value must be [Z, H, L, D] (got ",
+                    q0.sizes(), ", ", k0.sizes(), ", ", v0.sizes(), ")");
+  require_same(k0, q0, "the key");
+  require_same(v0, q0, "the value");
+  check_masks(rpe, kpm, am, q0);
   require_cuda(q0);
-  require_cuda(k0);
-  require_cuda(v0);
   const int64_t Z = q0.size(0), H = q0.size(1), L = q0.size(2);
   TORCH_CHECK_VALUE(p->H == H && p->nb * p->block == L, "layout [", p->H, ", ", p->nb, ", ", p->nb, "] with block ", p->block,
                     " does not fit operands of shape ", q0.sizes());
-  check_mask_dtypes(rpe, kpm, am, q0.scalar_type());
   const c10::cuda::CUDAGuard guard(q0.device());
   Tensor q = rows(q0), k = rows(k0), v = rows(v0);
   const int64_t D = q0.size(3);
@@ -540,11 +554,11 @@ Tensor attention_call(const c10::intrusive_ptr<AttentionOp>& p, const Tensor& q0
     // cannot describe (a broadcast operand, a mask off the 16-byte grid) is copied
     for (Tensor* t : {&q, &k, &v})
       if ((t->stride(0) == 0 && Z > 1) || (t->stride(1) == 0 && H > 1) || t->stride(2) == 0) *t = t->contiguous();
-    if (rpe && !(aligned16(*rpe) && rpe->stride(-1) == 1 && rpe->stride(-2) % 8 == 0 && rpe->stride(-2) > 0 &&
+    if (rpe && rpe->dim() >= 3 && !(aligned16(*rpe) && rpe->stride(-1) == 1 && rpe->stride(-2) % 8 == 0 && rpe->stride(-2) > 0 &&
                  rpe->stride(-3) % 8 == 0 && rpe->stride(-3) > 0 && (rpe->dim() < 4 || rpe->stride(0) % 8 == 0)))
       rpe = rpe->clone(at::MemoryFormat::Contiguous);
-    if (kpm && !(aligned16(*kpm) && kpm->stride(0) % 8 == 0)) kpm = kpm->clone(at::MemoryFormat::Contiguous);
-    if (am && !(aligned16(*am) && am->stride(0) % 8 == 0 && am->stride(0) > 0)) am = am->clone(at::MemoryFormat::Contiguous);
+    if (kpm && kpm->dim() == 2 && !(aligned16(*kpm) && kpm->stride(0) % 8 == 0)) kpm = kpm->clone(at::MemoryFormat::Contiguous);
+    if (am && am->dim() == 2 && !(aligned16(*am) && am->stride(0) % 8 == 0 && am->stride(0) > 0)) am = am->clone(at::MemoryFormat::Contiguous);
   }
   Masks m;
   set_rpe(m, rpe, Z, H, L, L);

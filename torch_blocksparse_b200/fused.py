@@ -217,6 +217,8 @@ class GraphedStep:
         _require_cuda(q, k, v, do)
         if not fused_supported(q, block):
             raise NotImplementedError('graphed step: FP16 / BF16 operands with a head dimension that is a multiple of 8 up to 128')
+        if any(t.shape != q.shape or t.dtype != q.dtype or t.device != q.device for t in (k, v, do)):
+            raise ValueError('graphed step: q, k, v and do must agree in shape, dtype and device')
         self.q, self.k, self.v, self.do = (_rows(t) for t in (q, k, v, do))
         for a, b in zip((self.q, self.k, self.v, self.do), (q, k, v, do)):
             if a is not b:
