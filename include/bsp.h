@@ -328,7 +328,9 @@ int bsp_attn_tiles_validate(const int32_t* tiles, int64_t len, int* code, int* p
  * aligned bases and strides that are multiples of 8 elements) the tcgen05 +
  * tensor-memory + TMA kernels run; otherwise, or with NULL, the mma.sync
  * kernels do.  Both give the
- * same result within rounding.  A query row whose keys are all masked out gets
+ * same result within rounding for finite operands; on the tcgen05 kernels an
+ * infinity or a NaN in a row of v (of dO or q in the backward) can also reach
+ * rows of the same 128-row tile whose own blocks do not touch it.  A query row whose keys are all masked out gets
  * zeros (the reference's softmax gives NaN there).
  * am_mul = 2: the caller vouches that `am` is the lower-triangular causal mask
  * in 'mul' form (am[i][j] != 0 exactly for j <= i); kernels that can do so
@@ -469,10 +471,9 @@ int bsp_debug_attn_wait(int wait_budget, int skip_chunk);
  * lets the cases the tcgen05 kernels cover (sdd: K a multiple of 64; dsd / dds:
  * dense width a multiple of 128 and at most 1024 blocks on the reduction side;
  * TMA-friendly strides) run on them; zero keeps every product on the mma.sync
- * kernels.  Process-wide.  At block 32 / 64 the tcgen05 dsd / dds kernel fills
- * the places of absent blocks with zeros instead of skipping them, so a
- * non-finite value of the dense operand can turn into NaN in output rows whose
- * own blocks do not touch it.
+ * kernels.  Process-wide.  Both families give the same result within
+ * rounding, non-finite values included: an infinity or a NaN of the dense
+ * operand reaches the results whose own blocks touch it and no others.
  */
 int bsp_matmul_use_tcgen05(int enable);
 

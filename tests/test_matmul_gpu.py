@@ -412,3 +412,42 @@ def test_linear_layer(block, dtype):
     assert_close(lin.weight.grad.to(dtype), want_dw.to(dtype), 'linear dw')
     with pytest.raises(ValueError):
         Linear(fin, fout + 1, block, layout)
+
+
+@pytest.mark.parametrize('block', [16, 32, 64, 128])
+@pytest.mark.parametrize('mode', ['dsd', 'dds'])
+@pytest.mark.parametrize('Z,H,n', [(1, 1, 300), (2, 3, 256), (1, 2, 1064)])
+@pytest.mark.parametrize('trans', [0, 1, 2, 3])
+def test_non_finite_dense_values_stay_out_of_absent_blocks(block, mode, Z, H, n, trans):
+    """An infinity or NaN of the dense operand reaches the results whose own blocks touch it and no others
+    (kernels that multiply absent blocks as zeros would turn those into NaN)."""
+    g = torch.Generator(DEV).manual_seed(block + n)
+    ts, td = trans & 1, trans >> 1                      # sparse / dense operand given transposed
+    out_b, red_b = (7, 9)
+    sl = (torch.rand((H, out_b, red_b), generator=torch.Generator().manual_seed(block)) > 0.6).long()
+    sl[:, 0, 0], sl[:, 3, :] = 1, 0                     # (a block-row without blocks)
+    if mode == 'dds':
+        layout = sl if ts else sl.transpose(1, 2).contiguous()
+    else:
+        layout = sl.transpose(1, 2).contiguous() if ts else sl
+    s = torch.randn((Z, int(layout.sum()), block, block), generator=g, device=DEV).half()
+    x = torch.randn((Z, H, red_b * block, n), generator=g, device=DEV).half()
+    for value, row, col in ((float('inf'), 5, 7), (float('-inf'), 2 * block + 1, 100), (float('nan'), 4 * block, 255),
+                            (float('inf'), 7 * block + 3, 255)):
+        x[:, :, row, col] = value
+    x[Z - 1, H - 1, 6 * block + 2] = float('inf')       # a whole row of the reduction side
+    x[0, 0, :, 33] = float('nan')                       # and a whole column
+    want = torch.zeros((Z, H, out_b * block, n), device=DEV)
+    for i, (h, r, c) in enumerate(layout.nonzero().tolist()):
+        o, k = (c, r) if (mode == 'dds') != bool(ts) else (r, c)
+        blk = s[:, i].float()
+        blk = blk.transpose(1, 2) if (mode == 'dds') != bool(ts) else blk
+        want[:, h, o * block:(o + 1) * block] += blk @ x[:, h, k * block:(k + 1) * block].float()
+    if mode == 'dsd':
+        got = MatMul(layout, block, 'dsd', trans_a=bool(ts), trans_b=bool(td))(s, x.transpose(2, 3).contiguous() if td else x)
+    else:
+        xt = x if td else x.transpose(2, 3).contiguous()
+        got = MatMul(layout, block, 'dds', trans_a=bool(td), trans_b=bool(ts))(xt, s).transpose(2, 3)
+    # FP16 results of FP32 sums: one rounding (2^-11) of values of about sqrt(4 block)
+    torch.testing.assert_close(got.float(), want, rtol=1e-3, atol=2e-3 * (4 * block) ** 0.5, equal_nan=True)
+    assert bool(want.isfinite().any()) and bool((~want.isfinite()).any())

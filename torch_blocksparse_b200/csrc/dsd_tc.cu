@@ -12,9 +12,8 @@
 // for block 64, four for block 32) by TN = 256 columns, or 128 for narrow or few tiles.
 // The block-rows of a tile are walked together, in
 // column order, over the UNION of their column lists; the piece of the A tile whose row has no
-// block in a column is zero (a non-finite value of the dense operand in such a place turns
-// into NaN where the mma.sync kernels, which skip absent blocks, give a finite result).  A
-// "stage" of the operand ring covers K = 64:
+// block in a column is zero (a non-finite value of the dense operand in such a place gives
+// a NaN, which repair_nan puts right).  A "stage" of the operand ring covers K = 64:
 //   block 128  one half of a nonzero block;
 //   block 64   one column of the union;
 //   block 32   two columns of the union (two sub-tiles of K = 32, 64-byte swizzle; the second
@@ -62,7 +61,7 @@ using namespace mmtc;
 constexpr int kThreads = 256;
 constexpr int kStageA = 16384;
 constexpr int kFirst = 1, kLast = 2, kEnd = 4, kHalf = 8;   // stage flags
-constexpr int kNone = 0x7fffffff;
+constexpr int kMarks = 1024;       // tiles of a CTA that can be marked one by one for repair_nan (the last mark stands for all that follow)
 
 // CTAS: CTAs per SM.  Two (blocks 32 and 64) have one accumulator and a short ring each; one
 // (block 128) has two accumulators, so that the write-back of a tile overlaps the products of the
@@ -76,6 +75,8 @@ template <int TN, int CTAS> struct Geo {
 };
 
 struct DsdTcArgs {
+  const void *s, *b;
+  int64_t s_sz, b_sz, b_sh, b_sk, b_sn;
   void* c;
   int64_t c_sz, c_sh, c_sm, c_sn;
   int H, Mb, block, rows_total, nnz_rows;   // rows_total = Mb * block; nnz_rows = nnz * block (first out-of-range row of S)
@@ -132,6 +133,44 @@ BSP_DEVI int warp_exclusive_sum(int v, int lane, int* total) {
   return x - v;
 }
 
+// One element of C from the blocks of its own block-row, in FP32 (see repair_nan).
+template <typename T, bool A_MN>
+BSP_DEVI float dsd_element(const DsdTcArgs& a, const Tile& t, int grow, int n) {
+  const int block = a.block, br = grow / block, r = grow % block;
+  const T* s = reinterpret_cast<const T*>(a.s) + t.z * a.s_sz + (A_MN ? r : r * block);
+  const T* b = reinterpret_cast<const T*>(a.b) + t.z * a.b_sz + t.h * a.b_sh + (int64_t)n * a.b_sn;
+  float acc = 0.f;
+  for (int j = a.row_ptr[t.h * a.Mb + br]; j < a.row_ptr[t.h * a.Mb + br + 1]; ++j) {
+    const T* sp = s + (int64_t)(a.blk_id ? a.blk_id[j] : j) * block * block;
+    const T* bp = b + (int64_t)a.blk_col[j] * block * a.b_sk;
+    for (int k = 0; k < block; ++k)
+      acc = fmaf(static_cast<float>(sp[A_MN ? k * block : k]), static_cast<float>(bp[k * a.b_sk]), acc);
+    if (acc != acc) break;                                     // NaN stays NaN
+  }
+  return acc;
+}
+// A tile multiplies the places of absent blocks as zeros, and zero times an infinity or a NaN of
+// the dense operand is NaN.  A finite or infinite result has met neither there, so it is right as it
+// is; the NaN of the tiles marked in `marks` are formed again from the blocks that exist.  All
+// threads of the CTA do this when its tiles are written, so that nobody waits for them meanwhile.
+// Finite operands pay for the look at the accumulators only (write-back).
+template <typename T, int TN, bool A_MN>
+BSP_DEVI void repair_nan(const DsdTcArgs& a, const uint32_t* marks, int tid) {
+  int local = 0;
+  for (int t = blockIdx.x; t < a.total_tiles; t += gridDim.x, ++local) {
+    const int bit = min(local, kMarks - 1);
+    if (!((marks[bit >> 5] >> (bit & 31)) & 1u)) continue;
+    const Tile tc_ = tile_of(a, t);
+    const int rows = min(128, a.rows_total - tc_.tr * 128), cols = min(TN, a.N - tc_.nt * TN);
+    for (int i = tid; i < rows * cols; i += kThreads) {
+      const int grow = tc_.tr * 128 + i / cols, n = tc_.nt * TN + i % cols;
+      T* p = reinterpret_cast<T*>(a.c) + tc_.z * a.c_sz + tc_.h * a.c_sh + (int64_t)grow * a.c_sm + (int64_t)n * a.c_sn;
+      const float v = static_cast<float>(*p);
+      if (v != v) *p = cvt1<T>(dsd_element<T, A_MN>(a, tc_, grow, n));
+    }
+  }
+}
+
 // B_KMAJOR: the dense operand has k contiguous ([n][k] in memory); else n contiguous ([k][n]).
 // C_ROWS: the result has unit stride along n (a thread writes its row with 16-byte stores);
 // else unit stride along m (the transposed problem of dds: lanes write neighbouring addresses).
@@ -150,6 +189,7 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
   __shared__ volatile int stage_flags[S];
   __shared__ Plan plan[2];
   __shared__ uint64_t bar_plan_full[2], bar_plan_empty[2];
+  __shared__ uint32_t marks[kMarks / 32];        // (CTAS == 2: blocks 32 and 64) tiles with a non-finite accumulator
   __shared__ uint32_t row_mask[4][32];           // planning warp: block-row r has a block in column 32 * word + bit
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
@@ -166,6 +206,7 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
     }
     mbar_init_fence();
   }
+  if (CTAS == 2 && tid < kMarks / 32) marks[tid] = 0;
   if (warp == 1) { tmem_alloc(&tmem_slot, kAcc * TN); tmem_relinquish(); }
   // the A part of every stage starts as zeros (see the loading thread)
   for (int i = tid; i < S * (kStageA / 16); i += kThreads)
@@ -466,9 +507,9 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
   } else if (warp < 4) {
     // ------------------------------------------------------------------ write-back
     const int row = warp * 32 + lane;
-    int tiles = 0;
+    int tiles = 0, local = 0;
     bool ok = true;
-    for (int t = blockIdx.x; ok && t < a.total_tiles; t += gridDim.x) {
+    for (int t = blockIdx.x; ok && t < a.total_tiles; t += gridDim.x, ++local) {
       const Tile tc_ = tile_of(a, t);
       const int br0 = tc_.tr * R;
       const int br1 = min(br0 + R, a.Mb);
@@ -484,12 +525,18 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
         fence_after();
       }
       const uint32_t ta = tmem + buf * TN + ((uint32_t)(warp * 32) << 16);
+      float2 seen = make_float2(0.f, 0.f);                          // becomes NaN with an accumulator that is not finite
 #pragma unroll 1
       for (int c = 0; c < TN; c += 32) {
         uint32_t r[32];
         if (any) {
           tmem_ld32(ta + c, r);
           tmem_ld_wait();
+          if (CTAS == 2) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 2)
+              seen = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), make_float2(0.f, 0.f), seen);
+          }
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = 0u;                   // block-rows without blocks: zeros, as the reference gives
@@ -519,6 +566,10 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
       if (any) {
         fence_before();
         warp_arrive(&bar_acc_empty[buf], lane);
+        if (CTAS == 2 && __any_sync(0xffffffffu, seen.x != 0.f || seen.y != 0.f) && lane == 0) {
+          const int bit = min(local, kMarks - 1);
+          atomicOr(&marks[bit >> 5], 1u << (bit & 31));
+        }
         ++tiles;
       }
     }
@@ -526,6 +577,7 @@ dsd_tc_kernel(const __grid_constant__ CUtensorMap m_s, const __grid_constant__ C
   fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, kAcc * TN);
+  if (CTAS == 2) repair_nan<T, TN, A_MN>(a, marks, tid);
   if (tid == 0 && failed[0]) atomicExch(&g_dsd_status, 4);
 }
 
@@ -625,6 +677,7 @@ int dsd_tc(const void* s, const void* b, void* c, int dtype, int block, int Z, i
     if (int rc = encode(&mb, b, dtype, 4, dims, strides, box, 128)) return rc;
   }
   DsdTcArgs a = {};
+  a.s = s; a.s_sz = s_sz; a.b = b; a.b_sz = b_sz; a.b_sh = b_sh; a.b_sk = b_sk; a.b_sn = b_sn;
   a.c = c; a.c_sz = c_sz; a.c_sh = c_sh; a.c_sm = c_sm; a.c_sn = c_sn;
   a.H = m.H; a.Mb = out_b; a.block = block; a.rows_total = out_b * block; a.nnz_rows = m.nnz * block;
   a.tiles_per_head = (out_b * block + 127) / 128;
