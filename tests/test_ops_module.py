@@ -230,3 +230,46 @@ def test_operands_on_the_host_are_refused_beside_a_device():
             call()
     with pytest.raises(ValueError, match='graphed step'):
         SparseSelfAttention(layout=LAYOUT, block=16).graphed(q, q.bfloat16(), q, q)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.float16, torch.float32])
+@pytest.mark.parametrize('free', [1, 2, 13, 33])
+@pytest.mark.parametrize('block', [16, 64])
+@pytest.mark.parametrize('where', ['whole', 'transposed', 'unaligned', 'odd rows', 'every other', 'expanded'])
+def test_widths_of_views(dtype, free, block, where):
+    """Dense operands of dsd and dds whose width is no multiple of 16 bytes, as views of any orientation, alignment
+    and row distance: what cannot be read where it lies is copied, never refused."""
+    g = torch.Generator('cuda').manual_seed(free)
+    H, nb = 2, 3
+    n = nb * block
+    layout = torch.ones((H, nb, nb), dtype=torch.long)
+    layout[0, 1] = 0
+    idx = layout.nonzero()
+    rand = lambda *s: torch.randn(s, generator=g, device='cuda', dtype=dtype)
+    s = rand(2, len(idx), block, block)
+    d = torch.zeros(2, H, nb, block, nb, block, device='cuda')
+    d[:, idx[:, 0], idx[:, 1], :, idx[:, 2]] = s.float().transpose(0, 1)
+    d = d.reshape(2, H, n, n)
+
+    def view(rows, cols):
+        if where == 'whole':
+            return rand(2, H, rows, cols)
+        if where == 'transposed':
+            return rand(2, H, cols, rows).transpose(2, 3)
+        if where == 'unaligned':
+            return rand(2 * H * cols * rows + 1)[1:].view(2, H, cols, rows).transpose(2, 3)
+        if where == 'odd rows':
+            return rand(2, H, cols, rows + 1)[..., :rows].transpose(2, 3)
+        if where == 'every other':
+            return rand(2, H, 2 * rows, 2 * cols)[:, :, ::2, ::2]
+        return rand(1, H, cols, rows).transpose(2, 3).expand(2, -1, -1, -1)
+    # FP16 results of FP32 sums: one rounding (2^-11) of values of about sqrt(n); FP32 against TF32-free FP32 sums
+    tol = dict(rtol=1e-3, atol=2e-3 * n ** 0.5) if dtype == torch.float16 else dict(rtol=1e-4, atol=1e-4)
+    close = lambda got, want: torch.testing.assert_close(got.float(), want, **tol)
+    x = view(n, free)
+    close(MatMul(layout, block, 'dsd')(s, x), d @ x.float())
+    close(MatMul(layout, block, 'dsd', trans_b=True)(s, x.transpose(2, 3)), d @ x.float())
+    x = view(free, n)
+    close(MatMul(layout, block, 'dds')(x, s), x.float() @ d)
+    close(MatMul(layout, block, 'dds', trans_a=True)(x.transpose(2, 3), s), x.float() @ d)

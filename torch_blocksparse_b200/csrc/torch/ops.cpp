@@ -170,12 +170,19 @@ Tensor sdd(const MatMulOp& p, Tensor a, Tensor b, bool ta, bool tb, bool tc, dou
   return c;
 }
 
-// A dense operand whose free dimension `dim` is contiguous and no multiple of 16 bytes is padded with
-// zeros (its rows would end inside a 16-byte piece); the result is cut back to the caller's size.
-Tensor pad_free(const Tensor& x, int64_t dim, int64_t vec) {
-  const int64_t pad = (vec - x.size(dim) % vec) % vec;
-  if (pad == 0 || (x.stride(5 - dim) == 1 && x.stride(dim) != 1)) return x;
-  return dim == 3 ? at::constant_pad_nd(x, {0, pad}) : at::constant_pad_nd(x, {0, 0, 0, pad});
+// The dense operand of dsd / dds, whose free dimension is `dim`.  A width that is no multiple of 16
+// bytes is read where it lies if the reduction side is contiguous and the rest can be addressed (a
+// width of one has no stride of its own); along the free side rows would end inside a 16-byte piece:
+// those operands are padded with zeros, and the result is cut back to the caller's size.
+Dense prep_free(const Tensor& x, int64_t dim) {
+  const int64_t vec = vec_of(x), red = 5 - dim, pad = (vec - x.size(dim) % vec) % vec;
+  if (pad == 0) return prep_dense(x);
+  if (x.stride(red) == 1) {
+    Dense d{x, {x.size(0) == 1 ? 0 : x.stride(0), x.size(1) == 1 ? 0 : x.stride(1), x.stride(2), x.stride(3)}};
+    if (x.size(dim) == 1) d.s[dim] = x.size(red);
+    if (d.s[dim] != 1 && d.s[dim] % vec == 0 && d.s[0] % vec == 0 && d.s[1] % vec == 0 && aligned16(x)) return d;
+  }
+  return prep_dense(dim == 3 ? at::constant_pad_nd(x, {0, pad}) : at::constant_pad_nd(x, {0, 0, 0, pad}));
 }
 // The result of dsd / dds, [Z, H, rows, cols], for kernels that compute `n` entries of the free
 // dimension of which the caller sees `keep`.  Rows along a free dimension are a multiple of 16 bytes apart.
@@ -191,8 +198,9 @@ Out make_out(const Tensor& like, int64_t Z, int64_t H, int64_t rows, int64_t col
 
 Tensor dsd(const MatMulOp& p, const Tensor& a, const Tensor& b0, bool ta, bool tb, bool tc, double* time) {
   const int64_t vec = vec_of(b0), fd = tb ? 2 : 3;
-  const Tensor s = prep_sparse(a, p.block), b = pad_free(b0, fd, vec);
-  const Dense B = prep_dense(b);
+  const Tensor s = prep_sparse(a, p.block);
+  const Dense B = prep_free(b0, fd);
+  const Tensor& b = B.t;
   const int64_t Z = b.size(0), H = b.size(1), M = p.block * (ta ? p.Nb : p.Mb), N = b.size(fd);
   TORCH_CHECK_VALUE(a.size(0) == Z && a.size(1) == p.nnz && a.size(2) == p.block && a.size(3) == p.block && H == p.H &&
                         b.size(tb ? 3 : 2) == p.block * (ta ? p.Mb : p.Nb),
@@ -210,8 +218,9 @@ Tensor dsd(const MatMulOp& p, const Tensor& a, const Tensor& b0, bool ta, bool t
 
 Tensor dds(const MatMulOp& p, const Tensor& a0, const Tensor& b, bool ta, bool tb, bool tc, double* time) {
   const int64_t vec = vec_of(a0), fd = ta ? 3 : 2;
-  const Tensor a = pad_free(a0, fd, vec), s = prep_sparse(b, p.block);
-  const Dense A = prep_dense(a);
+  const Tensor s = prep_sparse(b, p.block);
+  const Dense A = prep_free(a0, fd);
+  const Tensor& a = A.t;
   const int64_t Z = a.size(0), H = a.size(1), M = a.size(fd), N = p.block * (tb ? p.Mb : p.Nb);
   TORCH_CHECK_VALUE(b.size(0) == Z && b.size(1) == p.nnz && b.size(2) == p.block && b.size(3) == p.block && H == p.H &&
                         a.size(ta ? 2 : 3) == p.block * (tb ? p.Nb : p.Mb),
