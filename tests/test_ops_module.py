@@ -273,3 +273,29 @@ def test_widths_of_views(dtype, free, block, where):
     x = view(free, n)
     close(MatMul(layout, block, 'dds')(x, s), x.float() @ d)
     close(MatMul(layout, block, 'dds', trans_a=True)(x.transpose(2, 3), s), x.float() @ d)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('which', ['rpe', 'key_padding_mask', 'attn_mask'])
+@pytest.mark.parametrize('op', ['softmax', 'attention 64', 'attention 96', 'chain'])
+def test_biases_that_need_gradients_or_carry_tangents(op, which):
+    """With a gradient needed by a bias or a mask alone the result can be differentiated (the bias receives
+    nothing); a tangent on it is an error."""
+    import torch.autograd.forward_ad as fwd
+    make = lambda *s: torch.ones(s, device='cuda', dtype=torch.float16)
+    shape = {'rpe': (2, 64, 64), 'key_padding_mask': (1, 64), 'attn_mask': (64, 64)}[which]
+    if op == 'softmax':
+        call = lambda t: Softmax(LAYOUT, 16)(make(1, 20, 16, 16), **{which: t})
+    else:
+        D = 96 if op == 'attention 96' else 64
+        q = make(1, 2, 64, D)
+        call = lambda t: SparseSelfAttention(layout=LAYOUT, block=16, fused=op != 'chain')(q, q, q, **{which: t})
+    t = make(*shape).requires_grad_()
+    out = call(t)
+    assert out.requires_grad
+    out.sum().backward()
+    assert t.grad is None or not bool(t.grad.any())
+    with torch.no_grad():
+        assert not call(t).requires_grad
+        with fwd.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+            call(fwd.make_dual(make(*shape), make(*shape)))

@@ -62,10 +62,15 @@ void require_same(const Tensor& t, const Tensor& ref, const char* what) {
   TORCH_CHECK_VALUE(t.scalar_type() == ref.scalar_type(), what, " must be ", ref.scalar_type(), " (got ", t.scalar_type(), ")");
 }
 
-// Whether a call on these tensors goes through autograd: one of them needs a gradient, or carries a
+// Whether a call on these tensors goes through autograd: one of them needs a gradient (a bias or a
+// mask too, although it receives none: the result can then be differentiated), or carries a
 // forward-mode tangent, which the functions below refuse (passing them by would drop it silently).
+bool needs_grad(const Tensor& t) { return t.requires_grad(); }
+bool needs_grad(const OptTensor& t) { return t && t->requires_grad(); }
+bool has_tangent(const Tensor& t) { return t._fw_grad(0).defined(); }
+bool has_tangent(const OptTensor& t) { return t && has_tangent(*t); }
 template <typename... Ts> bool recorded(const Ts&... t) {
-  return (at::GradMode::is_enabled() && (t.requires_grad() || ...)) || (t._fw_grad(0).defined() || ...);
+  return (at::GradMode::is_enabled() && (needs_grad(t) || ...)) || (has_tangent(t) || ...);
 }
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 int64_t vec_of(const Tensor& t) { return 16 / static_cast<int64_t>(t.element_size()); }
@@ -446,7 +451,7 @@ Tensor softmax_call(const c10::intrusive_ptr<SoftmaxOp>& p, const Tensor& x, dou
   const bool kpm_mul = mode_flag(kpm_mode, "key_padding_mask_mode"), am_mul = mode_flag(am_mode, "attn_mask_mode");
   const c10::cuda::CUDAGuard guard(x.device());
   double* time = times ? &times->c : nullptr;
-  if (recorded(x))
+  if (recorded(x, rpe, kpm, am))
     return SoftmaxFn::apply(x, p, scale, rpe, kpm, am, kpm_mul, am_mul, time);
   {
     const at::AutoDispatchBelowADInplaceOrView below;
@@ -584,7 +589,7 @@ Tensor attention_call(const c10::intrusive_ptr<AttentionOp>& p, const Tensor& q0
   c->kpm_mul = kpm_mul;
   c->am_mul = am_mul;
   c->use_tiles = use_tiles;
-  if (recorded(q, k, v))
+  if (recorded(q, k, v, rpe, kpm, am))
     return AttentionFn::apply(q, k, v, c, m, rpe, kpm, am, seq_first);
   Tensor lse;
   return AttentionFn::run(*c, q, k, v, m, seq_first, &lse);
