@@ -299,3 +299,47 @@ def test_biases_that_need_gradients_or_carry_tangents(op, which):
         assert not call(t).requires_grad
         with fwd.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
             call(fwd.make_dual(make(*shape), make(*shape)))
+
+
+def test_attributes_changed_between_calls_are_read():
+    """MatMul, Softmax and attention objects keep native operations that copy their attributes."""
+    mm, x = MatMul(LAYOUT, 16, 'sdd'), torch.zeros(1, 2, 64, 16)
+    ops = [mm._op(x)]
+    for name, value in (('trans_a', True), ('trans_b', True), ('mode', 'dsd'), ('block', 32)):
+        setattr(mm, name, value)
+        ops.append(mm._op(x))
+        assert mm._op(x) is ops[-1]
+    assert len(set(map(id, ops))) == 5
+    sm = Softmax(LAYOUT, 16)
+    first = sm._op(x)
+    sm.block = 32
+    assert sm._op(x) is not first
+    q = torch.zeros(1, 2, 64, 64, dtype=torch.float16)
+    att = SparseSelfAttention(layout=LAYOUT, block=16)
+    with pytest.raises(RuntimeError, match='CUDA tensors only'):
+        att(q, q, q)
+    att.block = 32                                       # (its tables are those of block 16)
+    with pytest.raises((RuntimeError, ValueError), match='does not fit|CUDA tensors only'):
+        att(q, q, q)
+    assert len(att._attn) == 2
+
+
+@pytest.mark.gpu
+def test_products_after_an_attribute_changed():
+    from torch_blocksparse_b200 import Linear
+    g = torch.Generator('cuda').manual_seed(0)
+    a = torch.randn((1, 2, 64, 64), generator=g, device='cuda')
+    mm = MatMul(LAYOUT, 16, 'sdd')
+    plain = mm(a, a)
+    mm.trans_b = True
+    assert torch.equal(mm(a, a), MatMul(LAYOUT, 16, 'sdd', trans_b=True)(a, a)) and not torch.equal(mm(a, a), plain)
+    lin = Linear(64, 64, 16, LAYOUT[0]).cuda()
+    x = a[0, 0].requires_grad_()
+    w = lin.weight
+    for trans in (False, True):
+        lin.matmul.trans_b = trans
+        y = lin(x)
+        want = MatMul(LAYOUT[:1], 16, 'dds', trans_b=trans)(x[None, None], w[None])[0, 0]
+        assert torch.equal(y, want)
+        for got, ref in zip(torch.autograd.grad(y, (x, w), a[0, 1]), torch.autograd.grad(want, (x, w), a[0, 1])):
+            torch.testing.assert_close(got, ref)

@@ -104,7 +104,7 @@ def ops():
 
 
 class OpCache(dict):
-    """Native operations of one object, by device.  A copy or a pickle of the owner starts without
+    """Native operations of one object, by device and what else they hold.  A copy or a pickle of the owner starts without
     them (they are rebuilt on first use)."""
 
     def __reduce_ex__(self, protocol):

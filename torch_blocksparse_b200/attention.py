@@ -66,7 +66,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         self.fused = fused
         self.ops = dict()
         self.tiles = dict()
-        self._attn = _lib.OpCache()       # native attention per (heads, length, device index)
+        self._attn = _lib.OpCache()       # native attention per (heads, length, device index, block)
         self._causal_cache = dict()
         self.causal_checks = 0            # comparisons of a mask against the causal one made so far
 
@@ -102,7 +102,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
         """The fused attention with this module's tables on the device of `query`."""
         sdd_nt, _, _ = self.get_ops(H, L)
         op = fused.Attention(sdd_nt.meta, self.tiles[(H, L)], self.block, query.device)
-        self._attn[(H, L, query.get_device())] = op
+        self._attn[(H, L, query.get_device(), self.block)] = op
         return op
 
     def _is_causal(self, attn_mask, owner=None):
@@ -189,7 +189,7 @@ class DeepSpeedSparseSelfAttention(nn.Module):
             am_mode = self.attn_mask_mode
             if attn_mask is not None and am_mode == 'mul' and self._is_causal(attn_mask, mask_owner):
                 am_mode = 'causal'
-            op = self._attn.get((num_heads, tgt_len, query.get_device())) or self._attn_op(query, num_heads, tgt_len)
+            op = self._attn.get((num_heads, tgt_len, query.get_device(), self.block)) or self._attn_op(query, num_heads, tgt_len)
             return fused.attention(op, query, key, value, scaling, rpe, key_padding_mask, attn_mask,
                                    self.key_padding_mask_mode, am_mode, seq_first_out)
         sdd_nt, dsd_nn, softmax = self.get_ops(num_heads, tgt_len)

@@ -298,7 +298,7 @@ Tensor matmul_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& a0, cons
 struct LinearFn : torch::autograd::Function<LinearFn> {
   static Tensor run(const MatMulOp& p, const Tensor& x, const Tensor& w, double* time) {
     std::vector<int64_t> shape = x.sizes().vec();
-    const Tensor y = dds(p, x.reshape({1, 1, -1, x.size(-1)}), w.unsqueeze(0), false, false, false, time);
+    const Tensor y = dds(p, x.reshape({1, 1, -1, x.size(-1)}), w.unsqueeze(0), false, p.trans_b, false, time);
     shape.back() = y.size(3);
     return y.view(shape);
   }
@@ -315,11 +315,11 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     const Tensor x = s[0].reshape({1, 1, -1, s[0].size(-1)}), w = s[1].unsqueeze(0);
     const Tensor dy = grads[0].reshape({1, 1, -1, grads[0].size(-1)});
     variable_list out(4);
-    if (ctx->needs_input_grad(0)) out[0] = dds(*p, dy, w, false, true, false, nullptr).view(s[0].sizes());
+    if (ctx->needs_input_grad(0)) out[0] = dds(*p, dy, w, false, !p->trans_b, false, nullptr).view(s[0].sizes());
     if (ctx->needs_input_grad(1)) {
       // (the kernels read x and dy k-strided here, so any number of rows; other strides are copied)
       const bool strided = x.stride(3) == 1 && dy.stride(3) == 1;
-      out[1] = sdd(*p, strided ? x : x.contiguous(), strided ? dy : dy.contiguous(), true, false, false, nullptr, true).squeeze(0);
+      out[1] = sdd(*p, strided ? x : x.contiguous(), strided ? dy : dy.contiguous(), true, false, p->trans_b, nullptr, true).squeeze(0);
     }
     return out;
   }
@@ -328,6 +328,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
 Tensor linear_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& x, const Tensor& w0, const c10::intrusive_ptr<Times>& times) {
   require_cuda(x);
   require_cuda(w0);
+  TORCH_CHECK_VALUE(p->mode[0] == 'd' && p->mode[1] == 'd' && !p->trans_a, "Linear: its product is x . W, mode 'dds' with x as it is");
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor w = w0.scalar_type() == x.scalar_type() ? w0 : w0.to(x.scalar_type());
   require_same(w, x, "the weight");

@@ -91,7 +91,7 @@ class MatMul:
         self.time_da = None
         self.time_db = None
         self._meta = None
-        self._ops = _lib.OpCache()           # native operation per device index
+        self._ops = _lib.OpCache()           # native operations, see _op
 
     @property
     def meta(self):
@@ -100,15 +100,18 @@ class MatMul:
             self._meta = tables.build_meta(self.layout)
         return self._meta
 
-    def _op(self, device):
-        """The native operation with this object's tables on `device`."""
-        meta = self.meta
-        op = _lib.ops().MatMulOp(meta.hdr, meta.on(device), self.block, self.mode, self.trans_a, self.trans_b)
-        self._ops[-1 if device.index is None else device.index] = op
+    def _op(self, x):
+        """The native operation with this object's tables on the device of `x`.  It holds copies of the
+        attributes below, which may be changed between calls."""
+        key = (x.get_device(), self.block, self.mode, self.trans_a, self.trans_b)
+        op = self._ops.get(key)
+        if op is None:
+            meta = self.meta
+            op = self._ops[key] = _lib.ops().MatMulOp(meta.hdr, meta.on(x.device), *key[1:])
         return op
 
     def __call__(self, a, b):
-        op = self._ops.get(a.get_device()) or self._op(a.device)
+        op = self._op(a)
         if tracing.recording() is not None:
             return tracing.call(op, '__call__', a, b)
         if not self.bench:
@@ -157,7 +160,7 @@ class Linear(torch.nn.Module):
         if input.size(-1) != self.in_features:
             raise ValueError('Linear: expected %d input features, got %d' % (self.in_features, input.size(-1)))
         mm = self.matmul
-        op = mm._ops.get(input.get_device()) or mm._op(input.device)
+        op = mm._op(input)
         if tracing.recording() is not None:
             return tracing.call(op, 'linear', input, self.weight, None)
         times = _lib.ops().Times() if mm.bench else None

@@ -48,20 +48,23 @@ class Softmax:
         self.bench = bench
         self.lut_cache = dict()
         self.time_y = None
-        self._ops = _lib.OpCache()           # native operation per device index
+        self._ops = _lib.OpCache()           # native operations, see _op
 
-    def _op(self, device):
-        """The native operation with this object's table on `device`."""
-        lut, maxlut = self.make_lut(device)
-        op = _lib.ops().SoftmaxOp(lut, maxlut, *self.spdims, self.block)
-        self._ops[-1 if device.index is None else device.index] = op
+    def _op(self, x):
+        """The native operation with this object's table on the device of `x`.  It holds copies of the
+        attributes below, which may be changed between calls."""
+        key = (x.get_device(), self.spdims, self.block)
+        op = self._ops.get(key)
+        if op is None:
+            lut, maxlut = self.make_lut(x.device)
+            op = self._ops[key] = _lib.ops().SoftmaxOp(lut, maxlut, *self.spdims, self.block)
         return op
 
     def __call__(self, x, scale=1., rpe=None, key_padding_mask=None, attn_mask=None,
                  key_padding_mask_mode='add', attn_mask_mode='add'):
         if tracing.recording() is not None:
             raise RuntimeError('Softmax works in place, which torch.jit.trace cannot replay')
-        op = self._ops.get(x.get_device()) or self._op(x.device)
+        op = self._op(x)
         times = _lib.ops().Times() if self.bench else None
         x = op(x, scale, rpe, key_padding_mask, attn_mask, key_padding_mask_mode, attn_mask_mode, times)
         if times is not None:
