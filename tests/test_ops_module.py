@@ -343,3 +343,23 @@ def test_products_after_an_attribute_changed():
         assert torch.equal(y, want)
         for got, ref in zip(torch.autograd.grad(y, (x, w), a[0, 1]), torch.autograd.grad(want, (x, w), a[0, 1])):
             torch.testing.assert_close(got, ref)
+
+
+def test_objects_saved_before_they_had_native_operations():
+    """Whole modules in files of an earlier version have no cache of native operations."""
+    from torch_blocksparse_b200 import Linear, MultiheadAttention
+    x = torch.zeros(1, 2, 64, 64, dtype=torch.float16)
+    att, mha = SparseSelfAttention(layout=LAYOUT, block=16), MultiheadAttention(128, 2, LAYOUT, 16).half()
+    with pytest.raises(RuntimeError, match='CUDA tensors only'):
+        att(x, x, x)
+    for obj, calls in ((MatMul(LAYOUT, 16, 'sdd'), (x, x)), (Softmax(LAYOUT, 16), (torch.zeros(1, 20, 16, 16),)),
+                       (Linear(64, 64, 16, LAYOUT[0]), (torch.zeros(3, 64),)), (att, (x, x, x)), (mha, (torch.zeros(64, 1, 128).half(),) * 3)):
+        old = copy.deepcopy(obj)
+        parts = list(old.modules()) if isinstance(old, torch.nn.Module) else [old]
+        parts += [getattr(m, 'matmul') for m in parts if hasattr(m, 'matmul')]
+        parts += [o for m in parts for ops in getattr(m, 'ops', {}).values() for o in ops]
+        for m in parts:
+            m.__dict__.pop('_ops', None)
+            m.__dict__.pop('_attn', None)
+        with pytest.raises(RuntimeError, match='CUDA tensors only'):
+            pickle.loads(pickle.dumps(old))(*calls)

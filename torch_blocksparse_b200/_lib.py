@@ -103,6 +103,21 @@ def ops():
     return _ops
 
 
+class WithOps:
+    """An owner of native operations.  Objects saved before they had any (whole modules, in files) get
+    an empty cache when they are loaded."""
+
+    _op_cache = '_ops'                   # the attribute's name
+
+    def __setstate__(self, state):
+        base = super()
+        if hasattr(base, '__setstate__'):
+            base.__setstate__(state)
+        else:
+            self.__dict__.update(state)
+        self.__dict__.setdefault(self._op_cache, OpCache())
+
+
 class OpCache(dict):
     """Native operations of one object, by device and what else they hold.  A copy or a pickle of the owner starts without
     them (they are rebuilt on first use)."""

@@ -43,7 +43,9 @@ class SparsityConfig:
         self.vertsize = vertsize
 
 
-class DeepSpeedSparseSelfAttention(nn.Module):
+class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
+
+    _op_cache = '_attn'
 
     @staticmethod
     def _make_layout(num_heads, num_blocks, mode, block_stride, attention, numverts, vertsize):

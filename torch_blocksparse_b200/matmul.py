@@ -54,7 +54,7 @@ class _sparse_matmul:
         return tables.make_dxx_lut(layout, block, step, trans, device)
 
 
-class MatMul:
+class MatMul(_lib.WithOps):
 
     def make_lut(self, dtype, device):
         """The reference-format tables for c, da and db (matmul.py:611-641), cached

@@ -30,7 +30,7 @@ class _sparse_softmax:
         return tables.make_softmax_lut(layout, device)
 
 
-class Softmax:
+class Softmax(_lib.WithOps):
 
     def make_lut(self, device):
         """Table cache per device (softmax.py:332-336)."""
