@@ -92,3 +92,23 @@ def test_tiles_of_few_chunks(D, which):
     q, k, v, do = rand_qkv(Z, H, nb * 64, D, torch.float16, seed=D)
     kw, km, am = masks_of(which, Z, H, nb * 64, torch.float16, seed=5)
     check(layout, 64, q, k, v, do, True, km, am, **kw)
+
+
+@pytest.mark.parametrize('D', [32, 64, 96])
+def test_profiled_calls_take_the_same_operands(D, monkeypatch):
+    """With an event pair around every kernel a call gives the same bits, on operands that have to be copied too."""
+    from torch_blocksparse_b200 import fused
+    Z, H, L, block = 2, 2, 256, 32
+    q, k, v, do = rand_qkv(1, H, L, D, torch.float16, seed=1)
+    mod = SparseSelfAttention(layout=layout_of(H, L // block, 3), block=block, key_padding_mask_mode='mul')
+    pad = torch.ones(Z, L + 1, dtype=torch.float16, device='cuda')[:, 1:]
+    rpe = 0.1 * torch.randn(H, L, L + 1, device='cuda').half()[..., 1:]
+    xs = [t.cuda().expand(Z, -1, -1, -1).requires_grad_() for t in (q, k, v)]
+    results = []
+    for profile in (None, []):
+        monkeypatch.setattr(fused, 'PROFILE', profile)
+        o = mod(*xs, rpe=rpe, key_padding_mask=pad)
+        results.append((o, *torch.autograd.grad(o, xs, do.cuda().expand(Z, -1, -1, -1))))
+    assert len(fused.PROFILE) == 4
+    for a, b in zip(*results):
+        assert torch.equal(a, b)

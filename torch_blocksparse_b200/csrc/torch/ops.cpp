@@ -241,9 +241,9 @@ Tensor dds(const MatMulOp& p, const Tensor& a0, const Tensor& b, bool ta, bool t
   return o.cut();
 }
 
-Tensor product(char c, char a, char b, const MatMulOp& p, const Tensor& x, const Tensor& y, bool tx, bool ty, bool tc, double* time) {
+// The product of mode c a b ('s' one of them) of the operands in this order; the third letter follows from the first two.
+Tensor product(char c, char a, const MatMulOp& p, const Tensor& x, const Tensor& y, bool tx, bool ty, bool tc, double* time) {
   if (c == 's') return sdd(p, x, y, tx, ty, tc, time);
-  (void)b;
   return a == 's' ? dsd(p, x, y, tx, ty, tc, time) : dds(p, x, y, tx, ty, tc, time);
 }
 
@@ -253,7 +253,7 @@ struct MatMulFn : torch::autograd::Function<MatMulFn> {
     ctx->save_for_backward({a, b});
     ctx->saved_data["p"] = c10::IValue::make_capsule(p);
     if (times) ctx->saved_data["t"] = c10::IValue::make_capsule(times);
-    return product(p->mode[0], p->mode[1], p->mode[2], *p, a, b, p->trans_a, p->trans_b, false, times ? &times->c : nullptr);
+    return product(p->mode[0], p->mode[1], *p, a, b, p->trans_a, p->trans_b, false, times ? &times->c : nullptr);
   }
   // da through mode[1] mode[0] mode[2], db through mode[2] mode[1] mode[0] (matmul.py:587-606)
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
@@ -266,9 +266,9 @@ struct MatMulFn : torch::autograd::Function<MatMulFn> {
     const char* m = p->mode;
     variable_list out(4);
     if (ctx->needs_input_grad(0))
-      out[0] = product(m[1], m[0], m[2], *p, dc, b, false, !p->trans_b, p->trans_a, times ? &times->da : nullptr);
+      out[0] = product(m[1], m[0], *p, dc, b, false, !p->trans_b, p->trans_a, times ? &times->da : nullptr);
     if (ctx->needs_input_grad(1))
-      out[1] = product(m[2], m[1], m[0], *p, a, dc, !p->trans_a, false, p->trans_b, times ? &times->db : nullptr);
+      out[1] = product(m[2], m[1], *p, a, dc, !p->trans_a, false, p->trans_b, times ? &times->db : nullptr);
     return out;
   }
 };
@@ -289,7 +289,7 @@ Tensor matmul_call(const c10::intrusive_ptr<MatMulOp>& p, const Tensor& a0, cons
   require_same(b, a, "the second operand");
   const c10::cuda::CUDAGuard guard(a.device());
   if (recorded(a, b)) return MatMulFn::apply(a, b, p, times);
-  return product(p->mode[0], p->mode[1], p->mode[2], *p, a, b, p->trans_a, p->trans_b, false, times ? &times->c : nullptr);
+  return product(p->mode[0], p->mode[1], *p, a, b, p->trans_a, p->trans_b, false, times ? &times->c : nullptr);
 }
 
 // y = x . W for x [..., in_features] and the nonzero blocks of W ([in, out], one head): the dds
@@ -483,6 +483,39 @@ Tensor rows(const Tensor& x) {
   return ok ? x : x.contiguous();
 }
 
+// Head dimensions other than 64 and 128 are taken only by the kernels that read through tensor maps:
+// whatever such a map cannot describe (a broadcast operand, a mask off the 16-byte grid) is copied.
+Tensor rows_for(const Tensor& x) {
+  const Tensor r = rows(x);
+  const int64_t D = r.size(3);
+  if (D == 64 || D == 128) return r;
+  const bool broadcast = (r.stride(0) == 0 && r.size(0) > 1) || (r.stride(1) == 0 && r.size(1) > 1) || r.stride(2) == 0;
+  return broadcast ? r.contiguous() : r;
+}
+
+// Checks the operands of an attention call and brings them into a form the kernels can address.
+struct AttentionOperands {
+  Tensor q, k, v;
+  OptTensor rpe, kpm, am;
+};
+AttentionOperands attention_operands(const Tensor& q, const Tensor& k, const Tensor& v, OptTensor rpe, OptTensor kpm, OptTensor am) {
+  TORCH_CHECK_VALUE(q.dim() == 4 && k.sizes() == q.sizes() && v.sizes() == q.sizes(), "query, key and value must be [Z, H, L, D] (got ",
+                    q.sizes(), ", ", k.sizes(), ", ", v.sizes(), ")");
+  require_same(k, q, "the key");
+  require_same(v, q, "the value");
+  check_masks(rpe, kpm, am, q);
+  require_cuda(q);
+  const int64_t D = q.size(3);
+  if (D != 64 && D != 128) {
+    if (rpe && rpe->dim() >= 3 && !(aligned16(*rpe) && rpe->stride(-1) == 1 && rpe->stride(-2) % 8 == 0 && rpe->stride(-2) > 0 &&
+                 rpe->stride(-3) % 8 == 0 && rpe->stride(-3) > 0 && (rpe->dim() < 4 || rpe->stride(0) % 8 == 0)))
+      rpe = rpe->clone(at::MemoryFormat::Contiguous);
+    if (kpm && kpm->dim() == 2 && !(aligned16(*kpm) && kpm->stride(0) % 8 == 0)) kpm = kpm->clone(at::MemoryFormat::Contiguous);
+    if (am && am->dim() == 2 && !(aligned16(*am) && am->stride(0) % 8 == 0 && am->stride(0) > 0)) am = am->clone(at::MemoryFormat::Contiguous);
+  }
+  return {rows_for(q), rows_for(k), rows_for(v), rpe, kpm, am};
+}
+
 struct AttentionFn : torch::autograd::Function<AttentionFn> {
   static Tensor run(const AttentionCall& c, const Tensor& q, const Tensor& k, const Tensor& v, Masks& m, bool seq_first, Tensor* lse) {
     const int64_t Z = q.size(0), H = q.size(1), L = q.size(2), D = q.size(3);
@@ -527,9 +560,7 @@ struct AttentionFn : torch::autograd::Function<AttentionFn> {
     if (c->has_am) set_am(m, am = s[at++], L, L);
     m.kpm_mul = c->kpm_mul;
     m.am_mul = c->am_mul;
-    Tensor dout = rows(grads[0]);
-    if (D != 64 && D != 128 && ((dout.stride(0) == 0 && Z > 1) || (dout.stride(1) == 0 && H > 1) || dout.stride(2) == 0))
-      dout = dout.contiguous();
+    const Tensor dout = rows_for(grads[0]);
     const Tensor dq = at::empty({Z, H, L, D}, q.options()), dk = at::empty({Z, H, L, D}, q.options()),
                  dv = at::empty({Z, H, L, D}, q.options()), delta = at::empty({Z, H, L}, lse.options());
     const AttentionOp& p = *c->p;
@@ -551,30 +582,13 @@ struct AttentionFn : torch::autograd::Function<AttentionFn> {
 };
 
 Tensor attention_call(const c10::intrusive_ptr<AttentionOp>& p, const Tensor& q0, const Tensor& k0, const Tensor& v0, double scale,
-                      OptTensor rpe, OptTensor kpm, OptTensor am, bool kpm_mul, int am_mul, bool use_tiles, bool seq_first) {
-  TORCH_CHECK_VALUE(q0.dim() == 4 && k0.sizes() == q0.sizes() && v0.sizes() == q0.sizes(), "query, key and value must be [Z, H, L, D] (got ",
-                    q0.sizes(), ", ", k0.sizes(), ", ", v0.sizes(), ")");
-  require_same(k0, q0, "the key");
-  require_same(v0, q0, "the value");
-  check_masks(rpe, kpm, am, q0);
-  require_cuda(q0);
-  const int64_t Z = q0.size(0), H = q0.size(1), L = q0.size(2);
+                      const OptTensor& rpe0, const OptTensor& kpm0, const OptTensor& am0, bool kpm_mul, int am_mul, bool use_tiles,
+                      bool seq_first) {
+  auto [q, k, v, rpe, kpm, am] = attention_operands(q0, k0, v0, rpe0, kpm0, am0);
+  const int64_t Z = q.size(0), H = q.size(1), L = q.size(2);
   TORCH_CHECK_VALUE(p->H == H && p->nb * p->block == L, "layout [", p->H, ", ", p->nb, ", ", p->nb, "] with block ", p->block,
-                    " does not fit operands of shape ", q0.sizes());
-  const c10::cuda::CUDAGuard guard(q0.device());
-  Tensor q = rows(q0), k = rows(k0), v = rows(v0);
-  const int64_t D = q0.size(3);
-  if (D != 64 && D != 128) {
-    // only the kernels that read through tensor maps take these head dimensions: whatever such a map
-    // cannot describe (a broadcast operand, a mask off the 16-byte grid) is copied
-    for (Tensor* t : {&q, &k, &v})
-      if ((t->stride(0) == 0 && Z > 1) || (t->stride(1) == 0 && H > 1) || t->stride(2) == 0) *t = t->contiguous();
-    if (rpe && rpe->dim() >= 3 && !(aligned16(*rpe) && rpe->stride(-1) == 1 && rpe->stride(-2) % 8 == 0 && rpe->stride(-2) > 0 &&
-                 rpe->stride(-3) % 8 == 0 && rpe->stride(-3) > 0 && (rpe->dim() < 4 || rpe->stride(0) % 8 == 0)))
-      rpe = rpe->clone(at::MemoryFormat::Contiguous);
-    if (kpm && kpm->dim() == 2 && !(aligned16(*kpm) && kpm->stride(0) % 8 == 0)) kpm = kpm->clone(at::MemoryFormat::Contiguous);
-    if (am && am->dim() == 2 && !(aligned16(*am) && am->stride(0) % 8 == 0 && am->stride(0) > 0)) am = am->clone(at::MemoryFormat::Contiguous);
-  }
+                    " does not fit operands of shape ", q.sizes());
+  const c10::cuda::CUDAGuard guard(q.device());
   Masks m;
   set_rpe(m, rpe, Z, H, L, L);
   set_kpm(m, kpm, Z, L);
@@ -644,4 +658,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       }))
       .def("__call__", &attention_call, py::call_guard<py::gil_scoped_release>());
   m.def("attention_key", &attention_key);
+  m.def("attention_operands", [](const Tensor& q, const Tensor& k, const Tensor& v, OptTensor rpe, OptTensor kpm, OptTensor am) {
+    AttentionOperands o = attention_operands(q, k, v, rpe, kpm, am);
+    return std::make_tuple(o.q, o.k, o.v, o.rpe, o.kpm, o.am);
+  });
+  m.def("attention_gradient", &rows_for);
 }

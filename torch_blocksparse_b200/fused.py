@@ -100,13 +100,12 @@ def _mask_args(Z, H, L, dtype, rpe, kpm, am, kp_mode, am_mode):
 
 
 class _profiled_attention(torch.autograd.Function):
-    """What the native operation launches, with an event pair around every kernel (PROFILE)."""
+    """What the native operation launches, with an event pair around every kernel (PROFILE), on operands
+    prepared as it prepares them."""
 
     @staticmethod
     def forward(ctx, q, k, v, meta, tiles, block, scale, rpe, kpm, am, kp_mode, am_mode, seq_first_out=False):
-        _require_cuda(q, k, v)
         Z, H, L, D = q.shape
-        q, k, v = _rows(q), _rows(k), _rows(v)
         margs, keep = _mask_args(Z, H, L, q.dtype, rpe, kpm, am, kp_mode, am_mode)
         if seq_first_out:
             # the result in [L, Z, H * D] memory order (what a sequence-first caller reshapes it to
@@ -135,7 +134,7 @@ class _profiled_attention(torch.autograd.Function):
         kpm = rest.pop(0) if has_kpm else None
         am = rest.pop(0) if has_am else None
         Z, H, L, D = q.shape
-        do = _rows(do)
+        do = _lib.ops().attention_gradient(do)
         margs, _ = _mask_args(Z, H, L, q.dtype, rpe, kpm, am, kp_mode, am_mode)
         dq, dk, dv = (torch.empty((Z, H, L, D), dtype=q.dtype, device=q.device) for _ in range(3))   # the kernels write these densely
         delta = torch.empty((Z, H, L), dtype=torch.float32, device=q.device)
@@ -190,6 +189,7 @@ def attention(op, q, k, v, scale, rpe=None, key_padding_mask=None, attn_mask=Non
         return tracing.call(op.op, '__call__', *args)
     if PROFILE is None:
         return op.op(*args)
+    q, k, v, rpe, key_padding_mask, attn_mask = _lib.ops().attention_operands(q, k, v, rpe, key_padding_mask, attn_mask)
     return _profiled_attention.apply(q, k, v, op.meta, op.tiles, op.block, float(scale), rpe, key_padding_mask, attn_mask,
                                      key_padding_mask_mode, attn_mask_mode, seq_first_out)
 
