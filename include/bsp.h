@@ -467,15 +467,22 @@ int bsp_debug_attn_wait(int wait_budget, int skip_chunk);
 
 /*
  * Kernel family of bsp_sdd / bsp_dsd / bsp_dds for block 32 / 64 / 128 with
- * FP16 / BF16 operands (no counterpart in the reference): non-zero (the default)
- * lets the cases the tcgen05 kernels cover (sdd: K a multiple of 64; dsd / dds:
- * dense width a multiple of 128 and at most 1024 blocks on the reduction side;
- * TMA-friendly strides) run on them; zero keeps every product on the mma.sync
- * kernels.  Process-wide.  Both families give the same result within
+ * FP16 / BF16 operands (no counterpart in the reference): 1 (the default) runs
+ * what the tcgen05 kernels cover (TMA-friendly addresses and strides; dsd /
+ * dds: at most 1024 blocks on the reduction side) on them where they are the
+ * faster ones for its size, 2 runs all of it on them, 0 keeps every product on
+ * the mma.sync kernels.  Process-wide.  Both families give the same result within
  * rounding, non-finite values included: an infinity or a NaN of the dense
  * operand reaches the results whose own blocks touch it and no others.
  */
 int bsp_matmul_use_tcgen05(int enable);
+
+/*
+ * Which of the two the size alone speaks for (*prefers = 1: tcgen05), from the
+ * counts in the metadata's header.  op: 0 sdd, 1 dsd, 2 dds; free_size: K of
+ * sdd, the dense width (dsd) or height (dds).
+ */
+int bsp_matmul_prefers_tcgen05(int op, int block, int Z, int free_size, int trans_s, const int32_t* meta_hdr, int* prefers);
 
 #ifdef __cplusplus
 }

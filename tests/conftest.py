@@ -20,3 +20,12 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if 'gpu' in item.keywords:
             item.add_marker(skip)
+
+
+@pytest.fixture(params=[1, 2], ids=['by size', 'tcgen05'])
+def product_family(request):
+    """MatMul on the kernels its size speaks for, and on tcgen05 wherever they cover it."""
+    from torch_blocksparse_b200 import _lib
+    _lib.check(_lib.lib().bsp_matmul_use_tcgen05(request.param))
+    yield request.param
+    _lib.check(_lib.lib().bsp_matmul_use_tcgen05(1))

@@ -260,6 +260,7 @@ def test_dsd_dds_tcgen05_kernel(mode, ta, tb, block, dtype, width):
     op = MatMul(layout, block, mode, trans_a=ta, trans_b=tb)
     L = _lib.lib()
     try:
+        _lib.check(L.bsp_matmul_use_tcgen05(2))
         c_tc = op(a.to(DEV), b.to(DEV))
         _lib.check(L.bsp_matmul_use_tcgen05(0))
         c_mma = op(a.to(DEV), b.to(DEV))
@@ -306,6 +307,7 @@ def test_tcgen05_kernels_against_mma_sync_on_random_shapes():
         b = dm.dense_to_sparse(w, layout, block) if mode == 'dds' else w
         op = MatMul(layout, block, mode, trans_a=ta, trans_b=tb)
         try:
+            _lib.check(L.bsp_matmul_use_tcgen05(2))
             c_tc = op(a.to(DEV), b.to(DEV))
             _lib.check(L.bsp_matmul_use_tcgen05(0))
             c_mma = op(a.to(DEV), b.to(DEV))
@@ -317,7 +319,7 @@ def test_tcgen05_kernels_against_mma_sync_on_random_shapes():
 
 @pytest.mark.parametrize('mode,ta,tb', [('dsd', False, False), ('dsd', True, False), ('dds', False, True)])
 @pytest.mark.parametrize('block,nred', [(32, 200), (64, 160), (128, 140), (32, 1024), (32, 1056)])
-def test_dsd_dds_long_reduction_side(mode, ta, tb, block, nred):
+def test_dsd_dds_long_reduction_side(product_family, mode, ta, tb, block, nred):
     """Many blocks on the reduction side: a tile whose plan does not fit one buffer of the
     tcgen05 kernel (more than 64 entries: it is handed over in several pieces), the 1024 blocks
     that kernel plans for at most, and 1056 (the mma.sync kernel takes the call).  Rows that are
@@ -374,6 +376,7 @@ def test_sdd_tcgen05_kernel(ta, tb, block, dtype):
     op = MatMul(layout, block, 'sdd', trans_a=ta, trans_b=tb)
     L = _lib.lib()
     try:
+        _lib.check(L.bsp_matmul_use_tcgen05(2))
         c_tc = op(x.to(DEV), w.to(DEV))
         _lib.check(L.bsp_matmul_use_tcgen05(0))
         c_mma = op(x.to(DEV), w.to(DEV))
@@ -418,7 +421,7 @@ def test_linear_layer(block, dtype):
 @pytest.mark.parametrize('mode', ['dsd', 'dds'])
 @pytest.mark.parametrize('Z,H,n', [(1, 1, 300), (2, 3, 256), (1, 2, 1064)])
 @pytest.mark.parametrize('trans', [0, 1, 2, 3])
-def test_non_finite_dense_values_stay_out_of_absent_blocks(block, mode, Z, H, n, trans):
+def test_non_finite_dense_values_stay_out_of_absent_blocks(product_family, block, mode, Z, H, n, trans):
     """An infinity or NaN of the dense operand reaches the results whose own blocks touch it and no others
     (kernels that multiply absent blocks as zeros would turn those into NaN)."""
     g = torch.Generator(DEV).manual_seed(block + n)

@@ -42,7 +42,7 @@ def test_timed_calls_and_versions(dtype):
 @pytest.mark.parametrize('heads', [1, 2])
 @pytest.mark.parametrize('free', [8, 72, 120, 136, 250, 264, 520])
 @pytest.mark.parametrize('trans', [False, True])
-def test_products_with_ragged_free_dimensions(block, heads, free, trans):
+def test_products_with_ragged_free_dimensions(product_family, block, heads, free, trans):
     """dsd, dds and sdd at widths around the tiles of 128 and 256 columns and the 64 of a K stage, with
     batch and heads of one (whose strides carry no meaning), against an FP32 dense product."""
     g = torch.Generator().manual_seed(block + free)
@@ -75,7 +75,7 @@ def test_products_with_ragged_free_dimensions(block, heads, free, trans):
 @pytest.mark.gpu
 @pytest.mark.parametrize('block', [16, 32, 128])
 @pytest.mark.parametrize('rows', [1, 7, 129, 1000])
-def test_linear_with_any_number_of_rows(block, rows):
+def test_linear_with_any_number_of_rows(product_family, block, rows):
     """Forward and both gradients of Linear against the dense layer."""
     from torch_blocksparse_b200 import Linear
     g = torch.Generator().manual_seed(rows)
@@ -237,7 +237,7 @@ def test_operands_on_the_host_are_refused_beside_a_device():
 @pytest.mark.parametrize('free', [1, 2, 13, 33])
 @pytest.mark.parametrize('block', [16, 64])
 @pytest.mark.parametrize('where', ['whole', 'transposed', 'unaligned', 'odd rows', 'every other', 'expanded'])
-def test_widths_of_views(dtype, free, block, where):
+def test_widths_of_views(product_family, dtype, free, block, where):
     """Dense operands of dsd and dds whose width is no multiple of 16 bytes, as views of any orientation, alignment
     and row distance: what cannot be read where it lies is copied, never refused."""
     g = torch.Generator('cuda').manual_seed(free)
@@ -363,3 +363,34 @@ def test_objects_saved_before_they_had_native_operations():
             m.__dict__.pop('_attn', None)
         with pytest.raises(RuntimeError, match='CUDA tensors only'):
             pickle.loads(pickle.dumps(old))(*calls)
+
+
+@pytest.mark.parametrize('op,block,Z,heads,nb,density,free,trans,want', [
+    # sdd: padded or few tiles, the set-up and the union cost more than the products
+    ('sdd', 32, 1, 1, 32, 0.25, 64, 0, 0), ('sdd', 32, 4, 8, 128, 0.25, 32, 0, 0), ('sdd', 64, 1, 1, 16, 0.25, 48, 0, 0),
+    ('sdd', 32, 4, 8, 32, 0.5, 320, 0, 1), ('sdd', 32, 4, 8, 32, 0.5, 336, 0, 1), ('sdd', 64, 4, 8, 64, 0.5, 80, 0, 1),
+    # whole tiles of several entries and heads, and block 128
+    ('sdd', 32, 2, 2, 8, 0.1, 64, 0, 1), ('sdd', 128, 1, 1, 8, 0.1, 16, 0, 1), ('dsd', 32, 2, 2, 8, 0.1, 128, 0, 1),
+    # dsd and dds, narrow and wide
+    ('dsd', 32, 1, 12, 32, 0.25, 64, 0, 0), ('dsd', 32, 1, 12, 32, 0.25, 320, 1, 1), ('dds', 64, 1, 1, 16, 0.25, 64, 1, 0),
+    ('dds', 32, 1, 1, 128, 0.25, 4093, 0, 1), ('dds', 64, 1, 1, 64, 0.5, 2000, 1, 1), ('dsd', 16, 2, 2, 8, 0.5, 128, 0, 0)])
+def test_kernel_family_by_size(op, block, Z, heads, nb, density, free, trans, want):
+    """The family measured as the faster one at sizes well away from where the two are level."""
+    import ctypes
+    from torch_blocksparse_b200 import _lib, tables
+    g = torch.Generator().manual_seed(0)
+    meta = tables.build_meta((torch.rand((heads, nb, nb), generator=g) < density).long())
+    got = ctypes.c_int(-1)
+    _lib.check(_lib.lib().bsp_matmul_prefers_tcgen05(('sdd', 'dsd', 'dds').index(op), block, Z, free, trans, meta.hdr.data_ptr(),
+                                                     ctypes.byref(got)))
+    assert got.value == want
+
+
+def test_kernel_family_arguments():
+    import ctypes
+    from torch_blocksparse_b200 import _lib, tables
+    meta, out, L = tables.build_meta(LAYOUT), ctypes.c_int(-1), _lib.lib()
+    for args in ((3, 32, 1, 64, 0, meta.hdr.data_ptr()), (0, 48, 1, 64, 0, meta.hdr.data_ptr()), (0, 32, 1, 0, 0, meta.hdr.data_ptr()),
+                 (0, 32, 0, 64, 0, meta.hdr.data_ptr()), (0, 32, 1, 64, 0, None)):
+        assert L.bsp_matmul_prefers_tcgen05(*args, ctypes.byref(out)) == _lib.ERR_INVALID
+    assert L.bsp_matmul_use_tcgen05(3) == _lib.ERR_INVALID

@@ -41,6 +41,7 @@ _SIGNATURES = {
     'bsp_device_status': (c_int, [_IP]),
     'bsp_debug_attn_wait': (c_int, [c_int, c_int]),
     'bsp_matmul_use_tcgen05': (c_int, [c_int]),
+    'bsp_matmul_prefers_tcgen05': (c_int, [c_int] * 5 + [c_void_p, POINTER(c_int)]),
     'bsp_attn_tiles_build': (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int64, _I64P]),
     'bsp_meta_build': (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int64, _I64P]),
     'bsp_attn_tiles_device_capacity': (c_int64, [c_int, c_int, c_int]),

@@ -640,16 +640,20 @@ bool dsd_tc_eligible(const void* s, const void* b, const void* c, int dtype, int
   return true;
 }
 
+// Tiles of 256 columns, unless they would leave SMs without a tile (two persistent CTAs per SM)
+// or be mostly padding: a stage of a 128-column tile costs nearly as much as one of 256.
+int dsd_tc_tile_width(int N, int64_t row_tiles, int sms) {
+  return N <= 128 || row_tiles * ((N + 255) / 256) <= sms || (N % 256 != 0 && N % 256 <= 128 && N < 512) ? 128 : 256;
+}
+
 int dsd_tc(const void* s, const void* b, void* c, int dtype, int block, int Z, int N, int64_t s_sz, int trans_s,
            int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn,
            int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn, const Meta& m, cudaStream_t st) {
   const bool bk = b_sk == 1, cr = c_sn == 1;
-  // Tiles of 256 columns, unless they would leave SMs without a tile (two persistent CTAs per SM)
-  // or be mostly padding: a stage of a 128-column tile costs nearly as much as one of 256.
   const int sms = sm_count();
   if (sms <= 0) return fail(BSP_ERR_CUDA, "dsd (tcgen05): cannot query the device");
   const int64_t rows_t = (int64_t)Z * m.H * (((trans_s ? m.Nb : m.Mb) * block + 127) / 128);
-  const int TN = N <= 128 || rows_t * ((N + 255) / 256) <= sms || (N % 256 != 0 && N % 256 <= 128 && N < 512) ? 128 : 256;
+  const int TN = dsd_tc_tile_width(N, rows_t, sms);
   // op(S) has the layout's rows (and walks its CSR) or, transposed, its columns (CSC)
   const int out_b = trans_s ? m.Nb : m.Mb, red_b = trans_s ? m.Mb : m.Nb;
   const int64_t ktot = (int64_t)red_b * block;

@@ -3,7 +3,9 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include "common.h"
 
 namespace bsp {
@@ -20,6 +22,7 @@ int dsd_mma_t(const void* s, const void* b, void* c, int block, int Z, int N,
               int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn,
               const Meta& m, cudaStream_t st);
 
+int dsd_tc_tile_width(int N, int64_t row_tiles, int sms);
 bool dsd_tc_eligible(const void* s, const void* b, const void* c, int dtype, int block, int Z, int H, int N, int64_t s_sz,
                      int64_t b_sz, int64_t b_sh, int64_t b_sk, int64_t b_sn,
                      int64_t c_sz, int64_t c_sh, int64_t c_sm, int64_t c_sn);
@@ -76,8 +79,60 @@ int check_sparse(const char* op, const char* name, const void* p, int dtype, int
   return BSP_OK;
 }
 
-// Switch of the tcgen05 kernels for MatMul (on by default); see bsp_matmul_use_tcgen05.
+// Which forms run on the tcgen05 kernels (0 none, 1 by size, 2 all that they cover); see bsp_matmul_use_tcgen05.
 std::atomic<int> g_matmul_tc{1};
+
+// Whether a product is left to the tcgen05 kernels, by its size.  Whole tiles of several batch entries
+// and heads always are.  Where tiles are padded (a reduction of sdd that is no multiple of 64, a width of
+// dsd / dds that is no multiple of 128) or few (one batch entry, one head) the mma.sync kernels can be
+// faster: they walk the blocks that exist in steps that fit them, while a tcgen05 tile of 128 rows pays
+// its set-up, the union of its block-rows' columns and the padding (FP16, us, tcgen05 / mma.sync: sdd
+// block 32, 4 x 8 heads of 4096 x 32 x 4096, fixed layout 362 / 145; dsd block 32, 12 heads of 1024 x 1024,
+// density 0.25, width 64: 15 / 8, width 320: 19 / 29).
+// The device time of both is estimated from the layout's counts, with coefficients fitted to 10 284 forms
+// (blocks 32 to 128, densities 0.1 to 0.5 and structured layouts, 128 to 4096 rows, free sizes 16 to 4096,
+// 1 to 32 heads in all; mean error 6 to 18 %); the number of columns in a tile's union is taken as if the
+// blocks lay at random, which overrates it for structured layouts.  mma.sync keeps what it would do
+// nearly as fast.  Of the 9 671 padded or few forms 2 % then take over 5 % longer than on mma.sync (with
+// all of them on tcgen05 48 % did, up to 4.4 times as long), and their mean is 1.7 % above the faster kernel's.
+struct Cost { double tc, mma; };
+double ceil_div(double a, double b) { return std::ceil(a / b); }
+
+Cost sdd_cost(int block, int Z, int K, const Meta& m) {
+  const double tc[2][4] = {{1.55, 0.173, 6.26, 0.291}, {1.67, 0.118, 6.01, 0.293}};
+  const double mma[2][4] = {{2.83, 0.0106, 0.0170, 0.0123}, {2.99, 0.0077, 0.0217, 0.0056}};
+  const double *t = tc[block == 64], *q = mma[block == 64];
+  const int R = 128 / block;
+  const double density = m.nnz / ((double)m.H * m.Mb * m.Nb), cols = m.Nb * (1 - std::pow(1 - density, R));
+  const double tiles = (double)Z * m.H * ceil_div(m.Mb, R) * std::max(1.0, cols / (2 * R));   // groups of 2 R columns
+  const double waves = std::max(1.0, tiles / 148), stages = ceil_div(K, 64), area = (double)Z * m.nnz * block * block;
+  return {t[0] + t[1] * stages + t[2] * waves + t[3] * waves * stages, q[0] + q[1] * K + q[2] * area / 1e4 + q[3] * area * K / 1e6};
+}
+Cost dsd_cost(int block, int Z, int N, int trans_s, const Meta& m) {
+  const double tc[3][4] = {{3.76, 0.960, 8.58, 0.049}, {2.14, 1.051, 9.40, 0.0}, {6.15, 0.609, 4.21, 0.041}};
+  const double mma[3][4] = {{3.75, 0.313, 0.0090, 0.187}, {4.65, 0.413, 0.0065, 0.177}, {7.00, 0.526, 0.0054, 0.173}};
+  const double *t = tc[block == 32 ? 0 : block == 64 ? 1 : 2], *q = mma[block == 32 ? 0 : block == 64 ? 1 : 2];
+  const int R = 128 / block, out_b = trans_s ? m.Nb : m.Mb, red_b = trans_s ? m.Mb : m.Nb;
+  const double density = m.nnz / ((double)m.H * m.Mb * m.Nb), cols = red_b * (1 - std::pow(1 - density, R));
+  const double rows_t = (double)Z * m.H * ceil_div(out_b, R);
+  const bool narrow = dsd_tc_tile_width(N, (int64_t)rows_t, 148) == 128;
+  const double waves = std::max(1.0, rows_t * ceil_div(N, narrow ? 128 : 256) / (block == 128 ? 148 : 296)) * (narrow ? 0.6 : 1.0);
+  const double stages = cols * (block == 32 ? 0.5 : block == 64 ? 1 : 2);
+  const double width = N <= 64 ? 64 : 128 * ceil_div(N, 128);              // what the mma.sync kernel computes
+  return {t[0] + t[1] * stages * waves + t[2] * waves + t[3] * stages,
+          q[0] + q[1] * (m.nnz / ((double)m.H * out_b)) * block / 32 + q[2] * Z * (double)m.nnz * block * block * width / 1e6 +
+              q[3] * Z * (double)m.H * out_b * block * N / 1e5};
+}
+bool sdd_prefers_tc(int block, int Z, int K, const Meta& m) {
+  if (block == 128 || (K % 64 == 0 && Z > 1 && m.H > 1)) return true;      // (block 128: at most 1.1 x mma.sync's time, 0.64 in the mean)
+  const Cost c = sdd_cost(block, Z, K, m);
+  return 1.2 * c.tc < c.mma;
+}
+bool dsd_prefers_tc(int block, int Z, int N, int trans_s, const Meta& m) {
+  if (N % 128 == 0 && Z > 1 && m.H > 1) return true;
+  const Cost c = dsd_cost(block, Z, N, trans_s, m);
+  return 1.1 * c.tc < c.mma;
+}
 
 int run_dsd(const void* s, const void* b, void* c, int dtype, int block, int Z, int N,
             int64_t s_sz, int trans_s,
@@ -87,8 +142,10 @@ int run_dsd(const void* s, const void* b, void* c, int dtype, int block, int Z, 
   // (a layout without any block has no sparse tensor to describe to the tensor-map encoder: the
   // mma.sync kernel writes the zeros)
   // (the tcgen05 kernel plans a tile with one bit per block of the reduction side, 1024 at most)
-  if (g_matmul_tc.load() && m.nnz > 0 && (trans_s ? m.Mb : m.Nb) <= 1024 &&
-      dsd_tc_eligible(s, b, c, dtype, block, Z, m.H, N, s_sz, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn))
+  const int tc = g_matmul_tc.load();
+  if (tc && m.nnz > 0 && (trans_s ? m.Mb : m.Nb) <= 1024 &&
+      dsd_tc_eligible(s, b, c, dtype, block, Z, m.H, N, s_sz, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn) &&
+      (tc == 2 || dsd_prefers_tc(block, Z, N, trans_s, m)))
     return dsd_tc(s, b, c, dtype, block, Z, N, s_sz, trans_s, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn, m, st);
   if (dtype == BSP_F32)
     return dsd_mma_t<float>(s, b, c, block, Z, N, s_sz, trans_s, b_sz, b_sh, b_sk, b_sn, c_sz, c_sh, c_sm, c_sn, m, st);
@@ -118,8 +175,10 @@ extern "C" int bsp_sdd(const void* a, const void* b, void* c, int dtype, int blo
   if (m.nnz == 0) return BSP_OK;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // (the tcgen05 kernel's grid: groups of 128 rows per head in y, the batch in z)
-  if (g_matmul_tc.load() && Z <= 65535 && (int64_t)m.H * ((m.Mb * block + 127) / 128) <= 65535 &&
-      sdd_tc_eligible(a, b, c, dtype, block, Z, m.H, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz))
+  const int tc = g_matmul_tc.load();
+  if (tc && Z <= 65535 && (int64_t)m.H * ((m.Mb * block + 127) / 128) <= 65535 &&
+      sdd_tc_eligible(a, b, c, dtype, block, Z, m.H, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz) &&
+      (tc == 2 || sdd_prefers_tc(block, Z, K, m)))
     return sdd_tc(a, b, c, dtype, block, Z, K, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz, m, st);
   if (dtype == BSP_F32)
     return sdd_mma_t<float>(a, b, c, block, Z, K, a_sz, a_sh, a_sm, a_sk, b_sz, b_sh, b_sk, b_sn, c_sz, m, st);
@@ -170,10 +229,20 @@ extern "C" int bsp_dds(const void* a, const void* s, void* c, int dtype, int blo
                  reinterpret_cast<cudaStream_t>(stream));
 }
 
-// Chooses the kernel family of MatMul for block 64 / 128 with FP16 / BF16 operands: non-zero
-// (default) lets the eligible cases run on the tcgen05 kernels, zero keeps everything on the
-// mma.sync kernels.  Process-wide; meant for comparisons and tests.
+// Chooses the kernel family of MatMul for blocks 32, 64 and 128 with FP16 / BF16 operands.
 extern "C" int bsp_matmul_use_tcgen05(int enable) {
-  g_matmul_tc.store(enable ? 1 : 0);
+  if (enable < 0 || enable > 2) return fail(BSP_ERR_INVALID, "bsp_matmul_use_tcgen05: 0, 1 or 2 (got %d)", enable);
+  g_matmul_tc.store(enable);
+  return BSP_OK;
+}
+
+extern "C" int bsp_matmul_prefers_tcgen05(int op, int block, int Z, int free_size, int trans_s, const int32_t* meta_hdr, int* prefers) {
+  Meta m;
+  if (op < 0 || op > 2 || !prefers) return fail(BSP_ERR_INVALID, "bsp_matmul_prefers_tcgen05: op must be 0 (sdd), 1 (dsd) or 2 (dds)");
+  if (int rc = decode_meta(meta_hdr, meta_hdr, m)) return rc;              // (only the counts of the header are read)
+  if (int rc = check_basic("matmul", BSP_F16, block, Z, m.H, m)) return rc;
+  if (free_size <= 0) return fail(BSP_ERR_INVALID, "bsp_matmul_prefers_tcgen05: the free size must be positive");
+  *prefers = block == 16 || m.nnz == 0 ? 0 : op == 0 ? sdd_prefers_tc(block, Z, free_size, m)
+                                                     : dsd_prefers_tc(block, Z, free_size, op == 1 ? trans_s : !trans_s, m);
   return BSP_OK;
 }
