@@ -303,25 +303,35 @@ def test_biases_that_need_gradients_or_carry_tangents(op, which):
 
 def test_attributes_changed_between_calls_are_read():
     """MatMul, Softmax and attention objects keep native operations that copy their attributes."""
+    def used(obj, *args):
+        """The operation `obj` calls (on CPU tensors, which it refuses)."""
+        with pytest.raises((RuntimeError, ValueError), match='CUDA tensors only'):
+            obj(*args)
+        op, = obj._ops.values()
+        return op
     mm, x = MatMul(LAYOUT, 16, 'sdd'), torch.zeros(1, 2, 64, 16)
-    ops = [mm._op(x)]
+    ops = [used(mm, x, x)]
+    assert used(mm, x, x) is ops[0]
+    mm.bench = False
+    assert used(mm, x, x) is ops[0]                     # (nothing that the operation holds)
     for name, value in (('trans_a', True), ('trans_b', True), ('mode', 'dsd'), ('block', 32)):
         setattr(mm, name, value)
-        ops.append(mm._op(x))
-        assert mm._op(x) is ops[-1]
+        ops.append(used(mm, x, x))
     assert len(set(map(id, ops))) == 5
-    sm = Softmax(LAYOUT, 16)
-    first = sm._op(x)
+    sm, y = Softmax(LAYOUT, 16), torch.zeros(1, 20, 16, 16)
+    first = used(sm, y)
     sm.block = 32
-    assert sm._op(x) is not first
+    assert used(sm, y) is not first
     q = torch.zeros(1, 2, 64, 64, dtype=torch.float16)
     att = SparseSelfAttention(layout=LAYOUT, block=16)
     with pytest.raises(RuntimeError, match='CUDA tensors only'):
         att(q, q, q)
+    first, = att._attn.values()
     att.block = 32                                       # (its tables are those of block 16)
     with pytest.raises((RuntimeError, ValueError), match='does not fit|CUDA tensors only'):
         att(q, q, q)
-    assert len(att._attn) == 2
+    second, = att._attn.values()
+    assert second is not first and second.block == 32
 
 
 @pytest.mark.gpu

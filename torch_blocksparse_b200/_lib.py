@@ -105,10 +105,17 @@ def ops():
 
 
 class WithOps:
-    """An owner of native operations.  Objects saved before they had any (whole modules, in files) get
-    an empty cache when they are loaded."""
+    """An owner of native operations, which hold copies of some of its attributes.  Setting one of those
+    starts a new cache (a call that is building an operation meanwhile leaves it in the old one).
+    Objects saved before they had any operations (whole modules, in files) get a cache when loaded."""
 
-    _op_cache = '_ops'                   # the attribute's name
+    _op_cache = '_ops'                   # the cache's name
+    _op_attributes = frozenset()         # attributes that operations copy
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name in self._op_attributes and self._op_cache in self.__dict__:
+            self.__dict__[self._op_cache] = OpCache()
 
     def __setstate__(self, state):
         base = super()
@@ -120,7 +127,7 @@ class WithOps:
 
 
 class OpCache(dict):
-    """Native operations of one object, by device and what else they hold.  A copy or a pickle of the owner starts without
+    """Native operations of one object, by device.  A copy or a pickle of the owner starts without
     them (they are rebuilt on first use)."""
 
     def __reduce_ex__(self, protocol):

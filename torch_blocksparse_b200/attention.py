@@ -22,7 +22,7 @@ import weakref
 import torch
 import torch.nn as nn
 
-from . import _lib, fused, tables, tracing
+from . import _lib, fused, tables
 from .matmul import MatMul
 from .softmax import Softmax
 
@@ -46,6 +46,7 @@ class SparsityConfig:
 class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
 
     _op_cache = '_attn'
+    _op_attributes = frozenset(('block',))
 
     @staticmethod
     def _make_layout(num_heads, num_blocks, mode, block_stride, attention, numverts, vertsize):
@@ -68,7 +69,7 @@ class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
         self.fused = fused
         self.ops = dict()
         self.tiles = dict()
-        self._attn = _lib.OpCache()       # native attention per (heads, length, device index, block)
+        self._attn = _lib.OpCache()       # native attention per (heads, length, device index)
         self._causal_cache = dict()
         self.causal_checks = 0            # comparisons of a mask against the causal one made so far
 
@@ -102,9 +103,10 @@ class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
 
     def _attn_op(self, query, H, L):
         """The fused attention with this module's tables on the device of `query`."""
+        ops = self._attn
         sdd_nt, _, _ = self.get_ops(H, L)
         op = fused.Attention(sdd_nt.meta, self.tiles[(H, L)], self.block, query.device)
-        self._attn[(H, L, query.get_device(), self.block)] = op
+        ops[(H, L, query.get_device())] = op
         return op
 
     def _is_causal(self, attn_mask, owner=None):
@@ -168,7 +170,7 @@ class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
         mask_owner = attn_mask
         if attn_mask is not None:
             attn_mask = self.transpose_mask_for_sparse(query.dtype, attn_mask)
-        return self.attend(query, key, value, float(query.size(3)) ** -0.5, rpe, key_padding_mask, attn_mask,
+        return self.attend(query, key, value, int(query.size(3)) ** -0.5, rpe, key_padding_mask, attn_mask,
                            mask_owner=mask_owner)
 
     def attend(self, query, key, value, scaling, rpe=None, key_padding_mask=None, attn_mask=None, mask_owner=None,
@@ -179,7 +181,7 @@ class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
         fused kernel writes its result in [L, bsz, heads * head_dim] memory order (returned as the
         [bsz, heads, L, head_dim] view of it)."""
         _, num_heads, tgt_len, _ = query.shape
-        if tracing.recording() is not None:           # (sizes are tensors then, each one a key of its own)
+        if type(tgt_len) is not int:                  # (torch.jit.trace: sizes are tensors, each one a key of its own)
             num_heads, tgt_len = int(num_heads), int(tgt_len)
         if key_padding_mask is not None and key_padding_mask.dtype != query.dtype:
             key_padding_mask = key_padding_mask.to(query.dtype)
@@ -191,7 +193,7 @@ class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
             am_mode = self.attn_mask_mode
             if attn_mask is not None and am_mode == 'mul' and self._is_causal(attn_mask, mask_owner):
                 am_mode = 'causal'
-            op = self._attn.get((num_heads, tgt_len, query.get_device(), self.block)) or self._attn_op(query, num_heads, tgt_len)
+            op = self._attn.get((num_heads, tgt_len, query.get_device())) or self._attn_op(query, num_heads, tgt_len)
             return fused.attention(op, query, key, value, scaling, rpe, key_padding_mask, attn_mask,
                                    self.key_padding_mask_mode, am_mode, seq_first_out)
         sdd_nt, dsd_nn, softmax = self.get_ops(num_heads, tgt_len)

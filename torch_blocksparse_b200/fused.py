@@ -11,6 +11,7 @@ import torch
 
 from . import _lib, tracing
 from .matmul import _dtype_code, _require_cuda, _stream
+from .tracing import recording
 
 
 # When set to a list, every forward / backward appends (name, start_event,
@@ -185,7 +186,7 @@ def attention(op, q, k, v, scale, rpe=None, key_padding_mask=None, attn_mask=Non
         raise ValueError("attn_mask_mode must be 'add' or 'mul'")
     args = (q, k, v, scale, rpe, key_padding_mask, attn_mask, key_padding_mask_mode == 'mul', _AM_FLAG[attn_mask_mode],
             PATH == 'tc', seq_first_out)
-    if tracing.recording() is not None:
+    if recording() is not None:
         return tracing.call(op.op, '__call__', *args)
     if PROFILE is None:
         return op.op(*args)

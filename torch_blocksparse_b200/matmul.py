@@ -18,6 +18,7 @@ import math
 import torch
 
 from . import _lib, tables, tracing
+from .tracing import recording
 
 _DTYPES = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 
@@ -56,6 +57,8 @@ class _sparse_matmul:
 
 class MatMul(_lib.WithOps):
 
+    _op_attributes = frozenset(('block', 'mode', 'trans_a', 'trans_b'))
+
     def make_lut(self, dtype, device):
         """The reference-format tables for c, da and db (matmul.py:611-641), cached
         per (dtype, device):
@@ -91,7 +94,7 @@ class MatMul(_lib.WithOps):
         self.time_da = None
         self.time_db = None
         self._meta = None
-        self._ops = _lib.OpCache()           # native operations, see _op
+        self._ops = _lib.OpCache()           # native operation per device index
 
     @property
     def meta(self):
@@ -100,19 +103,16 @@ class MatMul(_lib.WithOps):
             self._meta = tables.build_meta(self.layout)
         return self._meta
 
-    def _op(self, x):
-        """The native operation with this object's tables on the device of `x`.  It holds copies of the
-        attributes below, which may be changed between calls."""
-        key = (x.get_device(), self.block, self.mode, self.trans_a, self.trans_b)
-        op = self._ops.get(key)
-        if op is None:
-            meta = self.meta
-            op = self._ops[key] = _lib.ops().MatMulOp(meta.hdr, meta.on(x.device), *key[1:])
+    def _op(self, device):
+        """The native operation with this object's tables on `device`."""
+        ops, meta = self._ops, self.meta
+        op = _lib.ops().MatMulOp(meta.hdr, meta.on(device), self.block, self.mode, self.trans_a, self.trans_b)
+        ops[-1 if device.index is None else device.index] = op
         return op
 
     def __call__(self, a, b):
-        op = self._op(a)
-        if tracing.recording() is not None:
+        op = self._ops.get(a.get_device()) or self._op(a.device)
+        if recording() is not None:
             return tracing.call(op, '__call__', a, b)
         if not self.bench:
             return op(a, b)
@@ -160,8 +160,8 @@ class Linear(torch.nn.Module):
         if input.size(-1) != self.in_features:
             raise ValueError('Linear: expected %d input features, got %d' % (self.in_features, input.size(-1)))
         mm = self.matmul
-        op = mm._op(input)
-        if tracing.recording() is not None:
+        op = mm._ops.get(input.get_device()) or mm._op(input.device)
+        if recording() is not None:
             return tracing.call(op, 'linear', input, self.weight, None)
         times = _lib.ops().Times() if mm.bench else None
         y = op.linear(input, self.weight, times)

@@ -16,7 +16,8 @@ function and the launches are in csrc/torch/ops.cpp.
 """
 import torch
 
-from . import _lib, tables, tracing
+from . import _lib, tables
+from .tracing import recording
 
 
 class _sparse_softmax:
@@ -31,6 +32,8 @@ class _sparse_softmax:
 
 
 class Softmax(_lib.WithOps):
+
+    _op_attributes = frozenset(('block', 'spdims'))
 
     def make_lut(self, device):
         """Table cache per device (softmax.py:332-336)."""
@@ -48,23 +51,21 @@ class Softmax(_lib.WithOps):
         self.bench = bench
         self.lut_cache = dict()
         self.time_y = None
-        self._ops = _lib.OpCache()           # native operations, see _op
+        self._ops = _lib.OpCache()           # native operation per device index
 
-    def _op(self, x):
-        """The native operation with this object's table on the device of `x`.  It holds copies of the
-        attributes below, which may be changed between calls."""
-        key = (x.get_device(), self.spdims, self.block)
-        op = self._ops.get(key)
-        if op is None:
-            lut, maxlut = self.make_lut(x.device)
-            op = self._ops[key] = _lib.ops().SoftmaxOp(lut, maxlut, *self.spdims, self.block)
+    def _op(self, device):
+        """The native operation with this object's table on `device`."""
+        ops = self._ops
+        lut, maxlut = self.make_lut(device)
+        op = _lib.ops().SoftmaxOp(lut, maxlut, *self.spdims, self.block)
+        ops[-1 if device.index is None else device.index] = op
         return op
 
     def __call__(self, x, scale=1., rpe=None, key_padding_mask=None, attn_mask=None,
                  key_padding_mask_mode='add', attn_mask_mode='add'):
-        if tracing.recording() is not None:
+        if recording() is not None:
             raise RuntimeError('Softmax works in place, which torch.jit.trace cannot replay')
-        op = self._op(x)
+        op = self._ops.get(x.get_device()) or self._op(x.device)
         times = _lib.ops().Times() if self.bench else None
         x = op(x, scale, rpe, key_padding_mask, attn_mask, key_padding_mask_mode, attn_mask_mode, times)
         if times is not None:
