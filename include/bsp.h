@@ -229,7 +229,8 @@ int bsp_attn_tiles_build_device(const void* layout, int elem_bytes, int H, int n
  * *_mul  0: the mask is added; 1: 'mul' mode, mask == 0 -> -inf, else 0
  *        (softmax.py:104-110).
  * Rows longer than 32767 elements are rejected with BSP_ERR_UNSUPPORTED
- * (softmax.py:225-227).
+ * (softmax.py:225-227); so is, with BSP_ERR_INVALID, a batch stride of 0 with
+ * Z > 1 (of x here, of dy in the backward: they are overwritten).
  */
 int bsp_softmax_fwd(void* x, int dtype, int Z, int64_t x_sz, int block,
                     int H, int Mb, const int32_t* lut, int maxlut, float scale,
@@ -259,7 +260,8 @@ int bsp_softmax_bwd(const void* y, void* dy, int dtype, int Z, int64_t y_sz, int
  * how trans_a / trans_b / trans_c of the reference are expressed (one of the
  * two inner strides of each operand must be 1).  C is written in block format
  * (z-stride c_sz), every block completely.  K must be a multiple of 16
- * (matmul.py:318-319), else BSP_ERR_INVALID.
+ * (matmul.py:318-319), else BSP_ERR_INVALID, unless neither operand has unit
+ * stride along K.
  */
 int bsp_sdd(const void* a, const void* b, void* c, int dtype, int block,
             int Z, int H, int K,
@@ -273,7 +275,8 @@ int bsp_sdd(const void* a, const void* b, void* c, int dtype, int block,
  * s_sz); trans_s != 0 uses S transposed.  B is the logical [Z, H, K, N] operand,
  * C the logical [Z, H, M, N] result, both through element strides (trans_b and
  * trans_c of the reference).  Every element of C is written, zeros where a
- * block-row of op(S) is empty.
+ * block-row of op(S) is empty.  N must be a multiple of 16 bytes where B has
+ * unit stride along it; with unit stride along K it may be any.
  */
 int bsp_dsd(const void* s, const void* b, void* c, int dtype, int block,
             int Z, int H, int N, int64_t s_sz, int trans_s,

@@ -581,7 +581,7 @@ int attn_fwd_t(const AttnArgs& p, int block, int D, int Z, cudaStream_t st) {
   BSP_ATTN_CASE(16, 64) BSP_ATTN_CASE(32, 64) BSP_ATTN_CASE(64, 64) BSP_ATTN_CASE(128, 64)
   BSP_ATTN_CASE(16, 128) BSP_ATTN_CASE(32, 128) BSP_ATTN_CASE(64, 128) BSP_ATTN_CASE(128, 128)
 #undef BSP_ATTN_CASE
-  return fail(BSP_ERR_UNSUPPORTED, "without tile lists the fused attention supports head dimensions 64 and 128 (got %d)", D);
+  return fail(BSP_ERR_UNSUPPORTED, "the mma.sync attention kernels (no tile lists, or operands that tensor maps cannot describe) take head dimensions 64 and 128 (got %d)", D);
 }
 
 template <typename T>
@@ -590,7 +590,7 @@ int attn_bwd_t(const AttnArgs& p, int block, int D, int Z, int parts, cudaStream
   BSP_ATTN_CASE(16, 64) BSP_ATTN_CASE(32, 64) BSP_ATTN_CASE(64, 64) BSP_ATTN_CASE(128, 64)
   BSP_ATTN_CASE(16, 128) BSP_ATTN_CASE(32, 128) BSP_ATTN_CASE(64, 128) BSP_ATTN_CASE(128, 128)
 #undef BSP_ATTN_CASE
-  return fail(BSP_ERR_UNSUPPORTED, "without tile lists the fused attention supports head dimensions 64 and 128 (got %d)", D);
+  return fail(BSP_ERR_UNSUPPORTED, "the mma.sync attention kernels (no tile lists, or operands that tensor maps cannot describe) take head dimensions 64 and 128 (got %d)", D);
 }
 
 }  // namespace bsp

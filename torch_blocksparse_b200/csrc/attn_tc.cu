@@ -1023,7 +1023,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
             warp_arrive(&bar_p[u & 1], lane);
             continue;
           }
-          if constexpr (C::ER2) {
+          if constexpr (C::ER2) {                           // (no rpe / mask here: those variants run with two groups)
             // First all of S^T: read, handed back, exponentials, P^T packed to 16 bits; this runs
             // while dP^T is still being computed.  Then dP^T in two passes of 16 columns; pass
             // hv leaves its part of the packed P^T in columns [16 hv, 16 hv + 8) and its packed
@@ -1046,13 +1046,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
                 if (KPM || FINE) {                              // own bias; a query row without any key counts as +inf
                   lv.x = lv.x == kNegInfT ? -kNegInfT : lv.x - my_b; lv.y = lv.y == kNegInfT ? -kNegInfT : lv.y - my_b;
                   lv.z = lv.z == kNegInfT ? -kNegInfT : lv.z - my_b; lv.w = lv.w == kNegInfT ? -kNegInfT : lv.w - my_b;
-                }
-                if constexpr (XT) {                             // rpe / mask of (query chalf * 32 + i .. + 3, this key)
-                  const unsigned char* xt = stg + (u % ST) * C::STAGE + C::XT_OFF;
-                  lv.x -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i, trow & 63);
-                  lv.y -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 1, trow & 63);
-                  lv.z -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 2, trow & 63);
-                  lv.w -= xt_term<T>(xt, a.has_rpe, a.am_mode, half, chalf * 32 + i + 3, trow & 63);
                 }
                 // the negated exponent lse - s c: the lse comes from shared memory as it is
                 const float2 z0 = __ffma2_rn(u2f(sr[i], sr[i + 1]), nsl2, f2(lv.x, lv.y));

@@ -19,8 +19,8 @@
 // blocks past the end of the union are neither loaded nor computed (N = 128) or computed on
 // whatever the ring holds and not stored.
 //
-// Warps: 0-3 write the blocks back, 4 issues the TMA loads (one lane per box), 5 the MMAs
-// (one thread).  Two CTAs per SM, two stages each.  mbarriers only; every wait is bounded
+// Warps: 0-3 write the blocks back, 4 issues the TMA loads, 5 the MMAs (one elected lane of
+// each acts).  Two CTAs per SM, two stages each.  mbarriers only; every wait is bounded
 // and a wait that expires sets a device status word.
 #include <algorithm>
 #include "mm_tc.cuh"

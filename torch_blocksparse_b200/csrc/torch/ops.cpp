@@ -2,7 +2,7 @@
 // the C-ABI library (include/bsp.h), as one native module (torch_blocksparse_b200/_ops).
 //
 // Why native: at small sizes a call is bound by the host, not by the kernel.  With the autograd
-// functions in Python and 40-argument ctypes calls a forward took 46 us and a forward + backward
+// functions in Python and 40-argument ctypes calls a forward took 44 us and a forward + backward
 // 150-190 us of host time around 9 and 33 us of kernels (one sequence of 1024 tokens, 12 heads).
 // Each operation object below holds what does not change between calls (the layout's tables on one
 // device, block, mode), so that a call from Python passes little more than the tensors.
