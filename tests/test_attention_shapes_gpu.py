@@ -112,3 +112,24 @@ def test_profiled_calls_take_the_same_operands(D, monkeypatch):
     assert len(fused.PROFILE) == 4
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('which', ['none', 'padding'])
+@pytest.mark.parametrize('D,block', [(128, 64), (96, 32), (128, 128), (64, 64)])
+def test_results_do_not_depend_on_the_order_of_tiles(D, block, which):
+    """More tiles than SMs, taken over by running CTAs in any order: the bits of every batch entry are those it has
+    alone, where each CTA runs one tile, call after call."""
+    Z, H, L = 6, 4, 2560
+    q, k, v, do = (t.cuda() for t in rand_qkv(Z, H, L, D, torch.float16, seed=D))
+    kw, km, am = masks_of(which, Z, H, L, torch.float16, seed=2)
+    kw = {n: t.cuda() for n, t in kw.items()}
+    mod = SparseSelfAttention(layout=layout_of(H, L // block, 7), block=block, key_padding_mask_mode=km, attn_mask_mode=am)
+
+    def results(z):
+        xs = [t[z].clone().requires_grad_() for t in (q, k, v)]
+        o = mod(*xs, **{n: t[z] for n, t in kw.items()})
+        return (o, *torch.autograd.grad(o, xs, do[z]))
+    alone = [results(slice(z, z + 1)) for z in range(Z)]
+    for _ in range(3):
+        for i, got in enumerate(results(slice(0, Z))):
+            assert torch.equal(got, torch.cat([one[i] for one in alone]))

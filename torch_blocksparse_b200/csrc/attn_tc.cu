@@ -910,26 +910,26 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap m_res0, const __grid_constant
         if (ok) {
           fence_after();
           if (mychunk >= 0) {                                   // uniform per warp: a warp lies inside one chunk
-            const float ma = xch[0][0][trow], mb = xch[1][0][trow], la = xch[0][1][trow], lb = xch[1][1][trow];
+            // a: the first half of the chunks' columns or, with two groups, the even chunks of the tile.  Which group has
+            // those depends on the tiles this CTA ran before; the sums below must not (products and sums are contracted,
+            // so that exchanging a and b changes the last bit).
+            const int ia = G == 1 ? 0 : base & 1, ib = ia ^ 1;
+            const float ma = xch[ia][0][trow], mb = xch[ib][0][trow], la = xch[ia][1][trow], lb = xch[ib][1][trow];
             const float m = fmaxf(ma, mb);
             const float wa = ma == kNegInfT ? 0.f : fast_exp2(ma - m), wb = mb == kNegInfT ? 0.f : fast_exp2(mb - m);
             const float lsum = la * wa + lb * wb;
             const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
             T* orow = reinterpret_cast<T*>(a.out0) + z * a.o_sz + h * a.o_sh + grow * a.o_sr;
             const uint32_t ta = tmem + C::ACC_BASE + lane_base;
-            // (a tile of one chunk leaves the other group's accumulator as it was)
-            const bool use_a = G == 1 || ntiles > 1 || !(base & 1), use_b = G == 1 || ntiles > 1 || (base & 1);
+            const bool use_b = G == 1 || ntiles > 1;               // (a tile of one chunk leaves the other group's accumulator as it was)
             for (int c = part * (D / 2); c < (part + 1) * (D / 2); c += 32) {
               uint32_t ra[32], rb[32];
-              tmem_ld32(ta + c, ra);
-              tmem_ld32(ta + D + c, rb);
+              tmem_ld32(ta + ia * D + c, ra);
+              tmem_ld32(ta + ib * D + c, rb);
               tmem_ld_wait();
-              if (!use_a || !use_b) {
+              if (!use_b) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                  if (!use_a) ra[i] = 0u;
-                  if (!use_b) rb[i] = 0u;
-                }
+                for (int i = 0; i < 32; ++i) rb[i] = 0u;
               }
 #pragma unroll
               for (int i = 0; i < 32; i += 8) {
