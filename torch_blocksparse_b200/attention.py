@@ -170,7 +170,10 @@ class DeepSpeedSparseSelfAttention(_lib.WithOps, nn.Module):
         mask_owner = attn_mask
         if attn_mask is not None:
             attn_mask = self.transpose_mask_for_sparse(query.dtype, attn_mask)
-        return self.attend(query, key, value, int(query.size(3)) ** -0.5, rpe, key_padding_mask, attn_mask,
+        head_dim = query.size(3)
+        if type(head_dim) is not int:                 # (torch.jit.trace: sizes are tensors)
+            head_dim = int(head_dim)
+        return self.attend(query, key, value, head_dim ** -0.5, rpe, key_padding_mask, attn_mask,
                            mask_owner=mask_owner)
 
     def attend(self, query, key, value, scaling, rpe=None, key_padding_mask=None, attn_mask=None, mask_owner=None,

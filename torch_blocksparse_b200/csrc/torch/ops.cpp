@@ -486,7 +486,7 @@ Tensor rows(const Tensor& x) {
 // Head dimensions other than 64 and 128 are taken only by the kernels that read through tensor maps:
 // whatever such a map cannot describe (a broadcast operand, a mask off the 16-byte grid) is copied.
 Tensor rows_for(const Tensor& x) {
-  const Tensor r = rows(x);
+  Tensor r = rows(x);
   const int64_t D = r.size(3);
   if (D == 64 || D == 128) return r;
   const bool broadcast = (r.stride(0) == 0 && r.size(0) > 1) || (r.stride(1) == 0 && r.size(1) > 1) || r.stride(2) == 0;
