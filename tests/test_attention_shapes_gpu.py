@@ -47,7 +47,7 @@ def test_head_dimensions(D, block, which):
 
 @pytest.mark.parametrize('which', ['none', 'padding', 'causal', 'all'])
 @pytest.mark.parametrize('block,nb', [(16, 5), (16, 6), (16, 11), (32, 5), (32, 7)])
-@pytest.mark.parametrize('D', [64, 128, 96])
+@pytest.mark.parametrize('D', [64, 128, 96, 32])
 def test_sequences_that_end_inside_a_chunk(block, nb, D, which):
     Z, H = 2, 2
     q, k, v, do = rand_qkv(Z, H, nb * block, D, torch.float16, seed=nb)

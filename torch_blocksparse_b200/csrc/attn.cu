@@ -57,6 +57,17 @@ XtHost xt_of(const void* rpe, int64_t rpe_sz, int64_t rpe_sh, int64_t rpe_sr, co
   return x;
 }
 
+// Whether a forward on a sequence that ends inside a chunk of 64 stays on the mma.sync kernel (both kernels give the same
+// log-sum-exp, so the backward may take the other family): with few keys per row and few tiles that kernel, a CTA per
+// block-row, is done before a tcgen05 CTA has set up and walked its coarsened chunks.  FP16, us, tcgen05 / mma.sync,
+// no mask: block 16, band of 80 keys, D 64: 2 x 1072 8.4 / 5.5, 8 x 1056 8.2 / 6.2, 16 x 2576 14.9 / 12.9, level at 48 x 1120,
+// 48 x 5488 58 / 60; D 128, 16 x 208 9.2 / 6.5, 8 x 1696 10.3 / 9.8; block 32, 160 keys: 8 x 928 8.5 / 6.5, 16 x 800 8.5 / 7.7.  With
+// more keys tcgen05 is the faster one at any size (bigbird, 8 x 912, D 128: 16 / 36), and so are its backward kernels.
+bool brief_forward(int Z, int H, int L, int D, int block, const int32_t* hdr, const void* rpe, const void* am) {
+  return L % 64 != 0 && (D == 64 || D == 128) && !rpe && !am && (int64_t)hdr[4] * block <= 160LL * H * (L / block) &&
+         (int64_t)Z * H * ((L + 127) / 128) <= 336;
+}
+
 // Strides the tensor-map encoder takes: positive (an operand expanded over the batch or the heads
 // has stride 0 and stays on the mma.sync kernels).
 bool tma_strides(int Z, int H, int64_t sz, int64_t sh, int64_t sr) {
@@ -158,6 +169,7 @@ extern "C" int bsp_attn_fwd(const void* q, const void* k, const void* v, void* o
   p.v_sz = v_sz; p.v_sh = v_sh; p.v_sr = v_sr; p.o_sz = o_sz; p.o_sh = o_sh; p.o_sr = o_sr;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (tc_eligible(tiles_hdr, tiles, block, rpe, rpe_sz, rpe_sh, rpe_sr, kpm, kpm_sz, am, am_sr) &&
+      !brief_forward(Z, H, L, D, block, meta_hdr, rpe, am) &&
       tma_strides(Z, H, q_sz, q_sh, q_sr) && tma_strides(Z, H, k_sz, k_sh, k_sr) && tma_strides(Z, H, v_sz, v_sh, v_sr)) {
     const XtHost xt = xt_of(rpe, rpe_sz, rpe_sh, rpe_sr, am, am_sr, am_mul);
     return attn_fwd_tc(q, k, v, o, lse, dtype, Z, H, L, D, q_sz, q_sh, q_sr, k_sz, k_sh, k_sr, v_sz, v_sh, v_sr,
